@@ -59,6 +59,7 @@ struct LaunchItem {
 
 inline int elem_bytes(int dt) { return dt == CAME_DT_F32 ? 4 : 2; }
 inline bool is_nd(const CameTensorDesc& d) { return d.cols != 0 && d.batch > 1; }
+inline int nd_chunk(const CameTensorDesc& d) { return is_nd(d) && !disable_fast() ? nd_small_batch(d.rows, d.cols) : 0; }
 
 // vector-path eligibility of a tensor for each kernel family
 struct VecFlags {
@@ -109,7 +110,8 @@ Geometry geometry(const CameTensorDesc& d) {
     if (is_nd(d)) {      // nbR / nbC: blocks of the flattened row / column vectors; flat_chunks: flat blocks of 256 elements
         g.nbR = (int)cdiv((int64_t)d.batch * g.R, QBLOCK);
         g.nbC = (int)cdiv((int64_t)d.batch * g.C, QBLOCK);
-        g.flat_chunks = cdiv((int64_t)d.batch * g.R * g.C, QBLOCK);
+        const int nm = nd_chunk(d);      // small matrices: flat_chunks counts chunks of them, and nothing else is launched
+        g.flat_chunks = nm ? cdiv((int64_t)d.batch, nm) : cdiv((int64_t)d.batch * g.R * g.C, QBLOCK);
         return g;
     }
     g.nbC = (int)cdiv(g.C, QBLOCK);
@@ -137,6 +139,14 @@ size_t carve(const CameTensorDesc& d, const Geometry& g, float* base, Scratch* o
     } else if (is_nd(d)) {
         const size_t B = d.batch;
         s.nbC = g.nbC;
+        s.tiles_r = (int)g.flat_chunks;      // partials of S
+        s.tiles_c = nd_chunk(d);
+        if (s.tiles_c) {
+            s.scal = take(4);
+            s.spart = take((size_t)g.flat_chunks);
+            if (out) *out = s;
+            return off;
+        }
         s.vr = take(B * (size_t)g.R); s.vc = take(B * (size_t)g.C);
         s.Rr = take(B * (size_t)g.R); s.Rc = take(B * (size_t)g.C);
         s.rowblk = take(B); s.rowblk2 = take(B);      // per matrix: guarded mean of the fresh row vectors
@@ -429,13 +439,15 @@ int came_b200_plan_create(const CameTensorDesc* descs, int n_tensors, void* work
     auto nvec = [&](int i) { return (int64_t)geo[i].nbR + geo[i].nbC; };
     auto nmat = [&](int i) { return (int64_t)D[i].batch; };
     auto nblk = [&](int i) { return geo[i].flat_chunks; };
-    build(KID_ND_SQ, isnd, nokey, nvec);
-    build(KID_ND_MEAN, isnd, nokey, nmat);
-    build(KID_ND_SUMSQ, isnd, nokey, nblk);
+    auto ndlarge = [&](int i) { return isnd(i) && !nd_chunk(D[i]); };
+    auto ndkey = [&](int i) { return nd_chunk(D[i]) ? Key{0, 0, nd_small_key(D[i].rows, D[i].cols), 2} : Key{0, 0, 0, 0}; };
+    build(KID_ND_SQ, ndlarge, nokey, nvec);
+    build(KID_ND_MEAN, ndlarge, nokey, nmat);
+    build(KID_ND_SUMSQ, isnd, ndkey, nblk);
     build(KID_ND_S, isnd, nokey, [&](int) { return (int64_t)1; });
-    build(KID_ND_RES, isnd, nokey, nvec);
-    build(KID_ND_RESMEAN, isnd, nokey, nmat);
-    build(KID_ND_APPLY, isnd, nokey, nblk);
+    build(KID_ND_RES, ndlarge, nokey, nvec);
+    build(KID_ND_RESMEAN, ndlarge, nokey, nmat);
+    build(KID_ND_APPLY, isnd, ndkey, nblk);
     auto fusedA = [&](int i) { return is2d(i) && vf[i].k == 2; };
     auto twopass = [&](int i) { return is2d(i) && vf[i].k != 2; };
     auto fused_code = [&](int i) {      // column groups per thread | row sets << 4 | ring slot KB << 8
@@ -699,7 +711,7 @@ int came_b200_step(came_plan_t* plan, const CameHyper* hypers, int n_groups, cam
         else if (it.kernel == KID_SQ_PARTIALS && it.key.variant == 2)
             e = launch_fused_sq(it.key, a, wbase + it.work_off, it.n, st);
         else if (it.kernel >= KID_ND_SQ && it.kernel <= KID_ND_APPLY)
-            e = launch_nd(it.kernel, a, wbase + it.work_off, it.n, st);
+            e = launch_nd(it.kernel, it.key, a, wbase + it.work_off, it.n, st);
         else if (it.kernel == KID_MOMENT_APPLY)
             e = launch_fused_ma(it.key, a, wbase + it.work_off, it.n, wbase + it.work2_off, it.n2, sync, sync + plan->n_tensors,
                                 sync + 2 * plan->n_tensors + 2 * (fused_launches++ % 6), st);      // two list cursors per launch (at most 6)

@@ -16,40 +16,6 @@ constexpr int CODEC_THREADS = 256;
 constexpr int CODEC_WARPS = CODEC_THREADS / 32;
 
 template <bool SIGNED>
-__device__ __forceinline__ uint32_t codec_code(float x, float a) {
-    return SIGNED ? (uint32_t)quant_i8_div(x, a) & 0xffu : (uint32_t)quant_u8_div(x, a);
-}
-// Four codes.  code = rint(RN(x / a) * qmax) is what the reference computes; a division per element makes the encoders
-// issue-bound (66 us for a 4096 x 11008 matrix, tile layout).  t = x * RN(qmax / a) differs from RN(x / a) * qmax by
-// at most four roundings, 4 * 2^-24 * 255 < 6.1e-5, so both round to the same integer unless t lies within that
-// distance of a half-integer: only then (one element in ten thousand; also NaN, or an absmax outside the range in which
-// qmax / a is safe) are the four divided.  The sum t + 1.5 * 2^23 rounds t to the nearest integer, ties to even, and
-// carries the code in its low byte.
-constexpr float CODEC_SURE = 0.5f - 6.5e-5f;
-template <bool SIGNED>
-__device__ __forceinline__ uint32_t codec_pack4(const float4& v, float a, float scale) {
-    const float magic = 12582912.0f;
-    const float x[4] = {v.x, v.y, v.z, v.w};
-    uint32_t y[4];
-    bool sure = true;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        const float t = __fmul_rn(SIGNED ? x[e] : fmaxf(x[e], 0.0f), scale);
-        const float r = __fadd_rn(t, magic);
-        sure = sure && fabsf(__fsub_rn(t, __fsub_rn(r, magic))) <= CODEC_SURE;
-        y[e] = __float_as_uint(r);
-    }
-    if (!sure)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) y[e] = codec_code<SIGNED>(x[e], a);
-    return __byte_perm(__byte_perm(y[0], y[1], 0x0040u), __byte_perm(y[2], y[3], 0x0040u), 0x5410u);
-}
-// NaN where the multiplication is not safe: every comparison above then fails
-template <bool SIGNED>
-__device__ __forceinline__ float codec_scale(float a) {
-    return recip_safe(a) ? (SIGNED ? QMAX_I8 : QMAX_U8) / a : __int_as_float(0x7fffffff);
-}
-template <bool SIGNED>
 __device__ __forceinline__ float4 codec_unpack4(uint32_t w, float s) {
     if (SIGNED)
         return make_float4((float)(int8_t)(w & 0xffu) * s, (float)(int8_t)((w >> 8) & 0xffu) * s,
@@ -74,9 +40,9 @@ __global__ void __launch_bounds__(CODEC_THREADS) k_quant_flat(const float* __res
         const float4 v0 = __ldcs(s4 + lane), v1 = __ldcs(s4 + 32 + lane);
         const float a = fix_absmax(warp_max(SIGNED ? fmaxf(absmax4(v0), absmax4(v1)) : fmaxf(max4(v0), max4(v1))));
         uint32_t* dst = reinterpret_cast<uint32_t*>(q + base);
-        const float sc = codec_scale<SIGNED>(a);
-        dst[lane] = codec_pack4<SIGNED>(v0, a, sc);
-        dst[32 + lane] = codec_pack4<SIGNED>(v1, a, sc);
+        const float sc = quant_scale<SIGNED>(a);
+        dst[lane] = quant_pack4<SIGNED>(v0, a, sc);
+        dst[32 + lane] = quant_pack4<SIGNED>(v1, a, sc);
         if (lane == 0) absmax[blk] = a;
         return;
     }
@@ -95,7 +61,7 @@ __global__ void __launch_bounds__(CODEC_THREADS) k_quant_flat(const float* __res
 #pragma unroll
     for (int i = 0; i < QBLOCK / 32; ++i) {
         const int64_t idx = base + 32 * i + lane;
-        if (idx < n) q[idx] = (uint8_t)codec_code<SIGNED>(v[i], a);
+        if (idx < n) q[idx] = (uint8_t)quant_code<SIGNED>(v[i], a);
     }
     if (lane == 0) absmax[blk] = a;
 }
@@ -145,10 +111,10 @@ __global__ void __launch_bounds__(CODEC_THREADS) k_quant_tile(const float* __res
         for (int r = 0; r < TILE; ++r) m = fmaxf(m, absmax4(v[r]));
         m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
         m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
-        const float a = fix_absmax(m), sc = codec_scale<true>(a);
+        const float a = fix_absmax(m), sc = quant_scale<true>(a);
 #pragma unroll
         for (int r = 0; r < TILE; ++r)
-            if (in && r < nrows) *reinterpret_cast<uint32_t*>(q + off + (int64_t)r * cols) = codec_pack4<true>(v[r], a, sc);
+            if (in && r < nrows) *reinterpret_cast<uint32_t*>(q + off + (int64_t)r * cols) = quant_pack4<true>(v[r], a, sc);
         if (in && (lane & 3) == 0) absmax[(int64_t)ty * tile_cols + (col >> 4)] = a;
     } else {
         float v[TILE];

@@ -285,8 +285,9 @@ __device__ __forceinline__ float block_vector_sum(const float* x, int n, float* 
 
 // ------------------------------------------------------------------------------------------
 // codec arithmetic.  Quantisation is rint((x / absmax) * qmax) with an IEEE quotient, as
-// blockwise_quantization.py:73-80 computes it.  div_by() forms the correctly rounded quotient from
-// a precomputed reciprocal with one residual correction (cheaper than a division per element).
+// blockwise_quantization.py:73-80 computes it.  div_by() forms the quotient from a precomputed reciprocal with one
+// residual correction (P. Markstein, IBM J. Res. Dev. 34, 1990: correctly rounded when the reciprocal is and nothing
+// under- or overflows), which is cheaper than a division per element.
 // ------------------------------------------------------------------------------------------
 __device__ __forceinline__ float fix_absmax(float a) { return a > 0.0f ? a : 1.0f; }
 
@@ -310,6 +311,41 @@ __device__ __forceinline__ int quant_i8_fast(float x, float absmax, float inv) {
 // The reciprocal trick needs 1/absmax and the residual to stay normal; outside this range take the
 // plain division (uniform per block, so no divergence inside a warp's block).
 __device__ __forceinline__ bool recip_safe(float absmax) { return absmax > 1e-30f && absmax < 1e30f; }
+
+template <bool SIGNED>
+__device__ __forceinline__ uint32_t quant_code(float x, float a) {
+    return SIGNED ? (uint32_t)quant_i8_div(x, a) & 0xffu : (uint32_t)quant_u8_div(x, a);
+}
+// Four codes.  code = rint(RN(x / a) * qmax) is what the reference computes; a division per element makes the encoders
+// issue-bound (66 us for a 4096 x 11008 matrix, tile layout).  t = x * RN(qmax / a) differs from RN(x / a) * qmax by
+// at most four roundings, 4 * 2^-24 * 255 < 6.1e-5, so both round to the same integer unless t lies within that
+// distance of a half-integer: only then (one element in ten thousand; also NaN, or an absmax outside the range in which
+// qmax / a is safe) are the four divided.  The sum t + 1.5 * 2^23 rounds t to the nearest integer, ties to even, and
+// carries the code in its low byte.
+constexpr float QUANT_SURE = 0.5f - 6.5e-5f;
+template <bool SIGNED>
+__device__ __forceinline__ uint32_t quant_pack4(const float4& v, float a, float scale) {
+    const float magic = 12582912.0f;
+    const float x[4] = {v.x, v.y, v.z, v.w};
+    uint32_t y[4];
+    bool sure = true;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float t = __fmul_rn(SIGNED ? x[e] : fmaxf(x[e], 0.0f), scale);
+        const float r = __fadd_rn(t, magic);
+        sure = sure && fabsf(__fsub_rn(t, __fsub_rn(r, magic))) <= QUANT_SURE;
+        y[e] = __float_as_uint(r);
+    }
+    if (!sure)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[e] = quant_code<SIGNED>(x[e], a);
+    return __byte_perm(__byte_perm(y[0], y[1], 0x0040u), __byte_perm(y[2], y[3], 0x0040u), 0x5410u);
+}
+// NaN where the multiplication is not safe: every comparison above then fails
+template <bool SIGNED>
+__device__ __forceinline__ float quant_scale(float a) {
+    return recip_safe(a) ? (SIGNED ? QMAX_I8 : QMAX_U8) / a : __int_as_float(0x7fffffff);
+}
 
 // ------------------------------------------------------------------------------------------
 // exponential moving average of a row / column statistic, with every rounding pinned (no contraction into
@@ -340,6 +376,15 @@ __device__ __forceinline__ float row_factor(float v, float mean, bool clamp) {
 __device__ __forceinline__ float col_factor(float v, bool clamp) {
     if (clamp) v = fmaxf(v, 1e-30f);
     return 1.0f / sqrtf(v);
+}
+
+// 1 / sqrt(x) by one Newton step y (3 - x y^2) / 2 from the hardware's approximation: within one unit in the last place, like
+// a rounded division of a rounded square root, in a fifth of the instructions.  Outside the range in which no term
+// under- or overflows: those two.
+__device__ __forceinline__ float inv_sqrt(float x) {
+    if (!(x > 1e-30f && x < 1e30f)) return 1.0f / sqrtf(x);
+    const float y = rsqrtf(x);
+    return fmaf(0.5f * y, fmaf(-x * y, y, 1.0f), y);
 }
 
 // ------------------------------------------------------------------------------------------

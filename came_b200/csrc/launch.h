@@ -78,7 +78,10 @@ bool fused_sq_eligible(int64_t cols, int elem_bytes);
 cudaError_t launch_nonfactored(int kernel, const KernelKey& key, const StepArgs& a, const Work* work, int n,
                                cudaStream_t st);
 
-cudaError_t launch_nd(int kernel, const StepArgs& a, const Work* work, int n, cudaStream_t st);
+cudaError_t launch_nd(int kernel, const KernelKey& key, const StepArgs& a, const Work* work, int n, cudaStream_t st);
+// tensors of more than two dimensions made of small matrices: matrices of a chunk (0: other kernels), launch key
+int nd_small_batch(int64_t rows, int64_t cols);
+int nd_small_key(int64_t rows, int64_t cols);
 cudaError_t launch_selftest_bounded_wait(int* status, int* observed, cudaStream_t st);
 
 cudaError_t launch_quantize_blockwise(const float* src, void* q, float* absmax, int64_t n, bool is_signed,
