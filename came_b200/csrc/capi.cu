@@ -53,60 +53,85 @@ struct LaunchItem {
     KernelKey key;
     size_t work_off;   // in Work units from the start of the work region
     int n;
-    size_t work2_off;  // fused momentum / apply kernel: its F items
+    size_t work2_off;  // fused momentum / apply kernel: its F items; whole-step kernel: vector blocks
     int n2;
+    size_t work3_off, work4_off;      // whole-step kernel: flat blocks, 1-D blocks
+    int n3, n4, bar;
 };
 
 inline int elem_bytes(int dt) { return dt == CAME_DT_F32 ? 4 : 2; }
 inline bool is_nd(const CameTensorDesc& d) { return d.cols != 0 && d.batch > 1; }
 inline int nd_chunk(const CameTensorDesc& d) { return is_nd(d) && !disable_fast() ? nd_small_batch(d.rows, d.cols) : 0; }
 
-// vector-path eligibility of a tensor for each kernel family
+// Which kernels take the passes of a matrix.
 struct VecFlags {
-    int k;      // gradient reductions: 1 = runs of 8
-    int p2;     // momentum pass: 1 = runs of 16 over g and m, 2 = staged fast path (tile / fp32 layout: cols % 64 == 0)
-    int p3;     // apply pass: same over m and p
-    int flat;   // flat apply: 1 = runs of 8 over g, m, p
-    bool operator==(const VecFlags& o) const { return k == o.k && p2 == o.p2 && p3 == o.p3 && flat == o.flat; }
+    int k;      // gradient sums of the staged path: 2 = one pass (fused_sq.cu), 1 = two passes (rows too wide for it)
+    int wide;   // staged momentum / apply passes
+    int v;      // elements per access of the whole-step kernel (generic.cu): 8, or 1 for any shape and alignment
+    bool operator==(const VecFlags& o) const { return k == o.k && wide == o.wide && v == o.v; }
 };
 
 VecFlags vec_flags(const CameTensorDesc& d) {
-    VecFlags v{0, 0, 0, 0};
-    if (d.cols == 0 || is_nd(d)) return v;      // 1-D and N-D tensors have kernels of their own
-    const bool c8 = d.cols % 8 == 0, c16 = d.cols % 16 == 0;
-    // staged fast path of the momentum / apply passes: both or neither, as they share the tile geometry
-    const bool all_aligned = aligned16(d.g) && aligned16(d.m) && aligned16(d.p);
-    const bool fast = !disable_fast() && all_aligned &&
-                      ((d.mode == CAME_MODE_TILE8 && d.cols % 64 == 0) ||
-                       (d.mode == CAME_MODE_FP32 && d.cols % 64 == 0) ||
-                       (d.mode == CAME_MODE_FLAT8 && d.cols % 256 == 0 && d.g_dtype == d.p_dtype));
-    v.k = c8 && aligned16(d.g);
+    VecFlags f{0, 0, 0};
+    if (d.cols == 0 || is_nd(d)) return f;      // 1-D and N-D tensors have kernels of their own
+    const bool aligned = aligned16(d.g) && aligned16(d.m) && aligned16(d.p);
+    f.v = aligned && d.cols % 8 == 0 ? 8 : 1;
+    f.wide = !disable_fast() && aligned &&
+             ((d.mode != CAME_MODE_FLAT8 && d.cols % 64 == 0) ||
+              (d.mode == CAME_MODE_FLAT8 && d.cols % 256 == 0 && d.g_dtype == d.p_dtype));
     // (tensors with the 1e-30 clamps take the fused first pass too: its closed form for the clip sum holds whenever no
     // clamp binds, which the finalize checks; if one does, the two-pass sum runs for that tensor)
-    if (v.k && !disable_fast() && fused_sq_eligible(d.cols, elem_bytes(d.g_dtype))) v.k = 2;
-    v.p2 = (c16 && aligned16(d.g) && aligned16(d.m)) ? (fast ? 2 : 1) : 0;
-    v.p3 = (c16 && aligned16(d.p) && aligned16(d.m)) ? (fast ? 2 : 1) : 0;
-    v.flat = c8 && aligned16(d.g) && aligned16(d.p) && (reinterpret_cast<uintptr_t>(d.m) & 7u) == 0;
-    if (fast && d.mode == CAME_MODE_FLAT8) v.flat = 2;
-    return v;
+    if (f.wide) f.k = fused_sq_eligible(d.cols, elem_bytes(d.g_dtype)) ? 2 : 1;
+    return f;
+}
+
+// Small sets: every matrix of a set with fewer elements than this on the staged path takes the whole-step kernel.
+// CAME_B200_SMALL_SET_ELEMS overrides the line (0: none; read whenever a plan is sized or created).
+constexpr long long SMALL_SET_ELEMS = 16 << 20;
+
+// What a plan decides about the set as a whole.
+struct Context {
+    bool small;      // the whole-step kernel takes every matrix
+    int bands;       // its bands of 16 rows per warp
+    bool generic(const CameTensorDesc& d) const { return d.cols != 0 && !is_nd(d) && (small || !vec_flags(d).wide); }
+};
+
+int64_t generic_tiles(const CameTensorDesc& d, int bands) {
+    return cdiv(d.rows, (int64_t)bands * 16) * cdiv(d.cols, generic_tile_cols());
+}
+// partials, groups of them and counters of a reduction over n items (leave_partial in generic.cu)
+size_t partial_floats(int64_t n) { return (size_t)(n + cdiv(n, PARTIAL_GROUP) + 1); }
+size_t partial_counters(int64_t n) { return (size_t)(1 + cdiv(n, PARTIAL_GROUP)); }
+
+Context context(const CameTensorDesc* descs, int n) {
+    const char* e = getenv("CAME_B200_SMALL_SET_ELEMS");
+    const double line = e ? atof(e) : (double)SMALL_SET_ELEMS;
+    double staged = 0.0;
+    for (int i = 0; i < n; ++i)
+        if (vec_flags(descs[i]).wide) staged += (double)descs[i].rows * (double)descs[i].cols;
+    Context c{staged < line, 4};
+    // as few bands per item as it takes to give every resident warp of the GPU (24 per SM) two items
+    for (; c.bands > 1; c.bands /= 2) {
+        int64_t tiles = 0;
+        for (int i = 0; i < n; ++i)
+            if (c.generic(descs[i])) tiles += generic_tiles(descs[i], c.bands);
+        if (tiles >= 2 * 24 * 148) break;
+    }
+    return c;
 }
 
 struct Geometry {
     int64_t R, C;
     int tiles_r, tiles_c, ptiles_r, ptiles_c, nbR, nbC;
     int64_t flat_chunks;
-    size_t floats;   // scratch floats of this tensor
 };
 
-Geometry geometry(const CameTensorDesc& d) {
+Geometry geometry(const CameTensorDesc& d, const Context& ctx) {
     Geometry g{};
     g.R = d.rows;
     g.C = d.cols;
     g.nbR = (int)cdiv(g.R, QBLOCK);
-    if (d.cols == 0) {
-        g.floats = align_up((size_t)g.nbR + 1, 4);
-        return g;
-    }
+    if (d.cols == 0) return g;
     if (is_nd(d)) {      // nbR / nbC: blocks of the flattened row / column vectors; flat_chunks: flat blocks of 256 elements
         g.nbR = (int)cdiv((int64_t)d.batch * g.R, QBLOCK);
         g.nbC = (int)cdiv((int64_t)d.batch * g.C, QBLOCK);
@@ -115,17 +140,21 @@ Geometry geometry(const CameTensorDesc& d) {
         return g;
     }
     g.nbC = (int)cdiv(g.C, QBLOCK);
+    if (ctx.generic(d)) {
+        g.tiles_r = (int)cdiv(g.R, (int64_t)ctx.bands * 16);
+        g.tiles_c = (int)cdiv(g.C, generic_tile_cols());
+        if (d.mode == CAME_MODE_FLAT8) g.flat_chunks = cdiv(g.R * g.C, QBLOCK);
+        return g;
+    }
     g.tiles_r = (int)cdiv(g.R, K_TR);
     g.tiles_c = (int)cdiv(g.C, K_TC);
-    const bool wide = vec_flags(d).p2 == 2;
-    g.ptiles_r = (int)cdiv(g.R, wide ? W_TR : P_TR);
-    g.ptiles_c = (int)cdiv(g.C, wide ? W_TC : P_TC);
-    g.flat_chunks = cdiv(cdiv(g.R * g.C, QBLOCK), FLAT_BLOCKS_PER_CTA);
+    g.ptiles_r = (int)cdiv(g.R, W_TR);
+    g.ptiles_c = (int)cdiv(g.C, W_TC);
     return g;
 }
 
 // carve the per-tensor float scratch; base == nullptr computes sizes only
-size_t carve(const CameTensorDesc& d, const Geometry& g, float* base, Scratch* out) {
+size_t carve(const CameTensorDesc& d, const Geometry& g, const Context& ctx, float* base, Scratch* out) {
     size_t off = 0;
     auto take = [&](size_t n) -> float* {
         float* p = base ? base + off : nullptr;
@@ -135,7 +164,9 @@ size_t carve(const CameTensorDesc& d, const Geometry& g, float* base, Scratch* o
     Scratch s{};
     s.nbR = g.nbR;
     if (d.cols == 0) {
-        s.spart = take((size_t)g.nbR + 1);      // block partials of sum u^2, then their sum
+        s.spart = take((size_t)g.nbR);      // block partials of sum u^2
+        s.scal = take(4);
+        s.counters = reinterpret_cast<int32_t*>(take(4));
     } else if (is_nd(d)) {
         const size_t B = d.batch;
         s.nbC = g.nbC;
@@ -152,6 +183,21 @@ size_t carve(const CameTensorDesc& d, const Geometry& g, float* base, Scratch* o
         s.rowblk = take(B); s.rowblk2 = take(B);      // per matrix: guarded mean of the fresh row vectors
         s.scal = take(4);
         s.spart = take((size_t)g.flat_chunks);
+    } else if (ctx.generic(d)) {
+        s.nbC = g.nbC;
+        s.tiles_r = g.tiles_r; s.tiles_c = g.tiles_c;
+        s.g_v = vec_flags(d).v;
+        s.g_nb = ctx.bands;
+        s.vr = take((size_t)g.R); s.vc = take((size_t)g.C);      // v_row, column factors c_j
+        s.Rr = take((size_t)g.R); s.Rc = take((size_t)g.C);      // residual row vector, C'_j
+        s.rowblk = take((size_t)g.nbR); s.rowblk2 = take((size_t)g.nbR);
+        s.scal = take(4);
+        s.rowpart = take((size_t)g.tiles_c * (size_t)g.R);
+        s.colpart = take((size_t)g.tiles_r * (size_t)g.C);
+        const int64_t items = (int64_t)g.tiles_r * g.tiles_c;
+        s.spart = take(partial_floats(items));
+        s.fac = d.mode == CAME_MODE_FLAT8 ? take((size_t)g.R) : nullptr;
+        s.counters = reinterpret_cast<int32_t*>(take(partial_counters(items)));
     } else {
         s.nbC = g.nbC;
         s.tiles_r = g.tiles_r; s.tiles_c = g.tiles_c;
@@ -169,13 +215,10 @@ size_t carve(const CameTensorDesc& d, const Geometry& g, float* base, Scratch* o
         }
         s.colpart = take((size_t)std::max(s.sq_col_parts, g.ptiles_r) * (size_t)g.C);
         s.spart = take(std::max((size_t)g.tiles_r * (size_t)g.tiles_c, (size_t)g.nbC));
-        s.fac = (d.mode == CAME_MODE_FLAT8 && vec_flags(d).flat != 2) ? take(2 * (size_t)(g.R + g.C)) : nullptr;
-        if (vec_flags(d).p2 == 2) {
-            s.res_eps_deferred = 1;
-            s.mfac = take((size_t)g.R);
-            s.mfac_c = take((size_t)g.C);
-            s.mfac_c2 = d.mode == CAME_MODE_FLAT8 ? take((size_t)g.C) : nullptr;
-        }
+        s.res_eps_deferred = 1;
+        s.mfac = take((size_t)g.R);
+        s.mfac_c = take((size_t)g.C);
+        s.mfac_c2 = d.mode == CAME_MODE_FLAT8 ? take((size_t)g.C) : nullptr;
         if (vec_flags(d).k == 2) {
             s.fused_a = 1;
             s.fa_rb = fa_rb;
@@ -213,16 +256,20 @@ int validate(const CameTensorDesc& d, int i) {
 }
 
 struct Layout {
-    size_t off_descs, off_scr, off_hyp, off_status, off_sync, off_work, off_float, total;
+    size_t off_descs, off_scr, off_hyp, off_status, off_bar, off_sync, off_work, off_float, total;
     size_t n_work;
 };
 
-size_t count_work(const CameTensorDesc* descs, int n) {
+size_t count_work(const CameTensorDesc* descs, int n, const Context& ctx) {
     size_t w = 0;
     for (int i = 0; i < n; ++i) {
-        const Geometry g = geometry(descs[i]);
+        const Geometry g = geometry(descs[i], ctx);
         if (descs[i].cols == 0) {
-            w += 2 * (size_t)g.nbR + 1;      // partial, apply; one reduce CTA
+            w += (size_t)g.nbR;
+            continue;
+        }
+        if (ctx.generic(descs[i])) {
+            w += (size_t)g.tiles_r * g.tiles_c + (size_t)(g.nbR + g.nbC) + (size_t)g.flat_chunks;
             continue;
         }
         if (is_nd(descs[i])) {      // two vector passes, two mean passes (one item per matrix), S, two element passes
@@ -231,17 +278,15 @@ size_t count_work(const CameTensorDesc* descs, int n) {
         }
         w += 2 * (size_t)g.tiles_r * g.tiles_c;      // sq_partials, sumsq
         w += 2 * (size_t)(g.nbR + g.nbC);            // two vector finalizes
-        // clip finalize: one CTA per S_FIN_CHUNK entries of the factor vectors on the staged momentum path
-        w += vec_flags(descs[i]).p2 == 2 ? (size_t)std::max<int64_t>(1, cdiv(g.R + g.C, S_FIN_CHUNK)) : (size_t)1;
-        w += (size_t)g.ptiles_r * g.ptiles_c;        // moment
-        if (descs[i].mode == CAME_MODE_FLAT8)
-            w += (size_t)(g.nbR + g.nbC) + std::max((size_t)g.flat_chunks, (size_t)g.ptiles_r * g.ptiles_c);
-        else w += (size_t)g.ptiles_r * g.ptiles_c;   // apply
+        w += (size_t)std::max<int64_t>(1, cdiv(g.R + g.C, S_FIN_CHUNK));      // clip finalize
+        w += 2 * (size_t)g.ptiles_r * g.ptiles_c;    // moment, apply
     }
     return w;
 }
 
-Layout layout(const CameTensorDesc* descs, int n) {
+constexpr int MAX_GENERIC_LAUNCHES = 32;      // (gradient type, parameter type, layout) combinations: 27
+
+Layout layout(const CameTensorDesc* descs, int n, const Context& ctx) {
     Layout L{};
     size_t off = 0;
     L.off_descs = off; off = align_up(off + (size_t)n * sizeof(CameTensorDesc));
@@ -249,11 +294,12 @@ Layout layout(const CameTensorDesc* descs, int n) {
     L.off_hyp = off;   off = align_up(off + (size_t)MAX_GROUPS * sizeof(CameHyper));
     L.off_status = off; off = align_up(off + sizeof(int));
     L.off_sync = off;  off = align_up(off + (2 * (size_t)n + 12) * sizeof(int));   // fused kernel: per-tensor item counters, list cursors
-    L.n_work = count_work(descs, n);
+    L.off_bar = off;   off = align_up(off + 2 * MAX_GENERIC_LAUNCHES * sizeof(int));      // grid barriers of the whole-step kernel
+    L.n_work = count_work(descs, n, ctx);
     L.off_work = off;  off = align_up(off + L.n_work * sizeof(Work));
     L.off_float = off;
     size_t fl = 0;
-    for (int i = 0; i < n; ++i) fl += align_up(carve(descs[i], geometry(descs[i]), nullptr, nullptr), 64);
+    for (int i = 0; i < n; ++i) fl += align_up(carve(descs[i], geometry(descs[i], ctx), ctx, nullptr, nullptr), 64);
     off = align_up(off + fl * sizeof(float));
     L.total = off;
     return L;
@@ -291,6 +337,8 @@ struct came_plan {
     int last_launches = 0;
     bool has_fused_ma = false;
     std::vector<char> fused;       // per tensor: stepped by the fused momentum / apply kernel
+    std::vector<char> pushable;    // ... or by the whole-step kernel, which serves the push mode too
+    bool needs_hyp = false;        // some kernel reads the hyper-parameters from the workspace
     int n_push = 0;                // push mode: peers that receive every parameter the fused kernel updates
     long long push_delta[MAX_PUSH_PEERS] = {};
     uintptr_t push_lo = 0, push_hi = 0;      // the local buffer the pushed parameters must lie in
@@ -366,7 +414,7 @@ size_t came_b200_workspace_bytes(const CameTensorDesc* descs, int n_tensors) {
     if (!descs || n_tensors <= 0) return 0;
     for (int i = 0; i < n_tensors; ++i)
         if (validate(descs[i], i) != CAME_OK) return 0;
-    return layout(descs, n_tensors).total;
+    return layout(descs, n_tensors, context(descs, n_tensors)).total;
 }
 
 int came_b200_plan_create(const CameTensorDesc* descs, int n_tensors, void* workspace, size_t workspace_bytes,
@@ -378,7 +426,8 @@ int came_b200_plan_create(const CameTensorDesc* descs, int n_tensors, void* work
         const int rc = validate(descs[i], i);
         if (rc != CAME_OK) return rc;
     }
-    const Layout L = layout(descs, n_tensors);
+    const Context ctx = context(descs, n_tensors);
+    const Layout L = layout(descs, n_tensors, ctx);
     if (!workspace || (reinterpret_cast<uintptr_t>(workspace) % ALIGN) != 0)
         return fail(CAME_E_WORKSPACE, "plan_create: workspace must be non-null and %zu-byte aligned", ALIGN);
     if (workspace_bytes < L.total)
@@ -397,9 +446,9 @@ int came_b200_plan_create(const CameTensorDesc* descs, int n_tensors, void* work
     float* fbase = reinterpret_cast<float*>(plan->ws + L.off_float);
     size_t foff = 0;
     for (int i = 0; i < n_tensors; ++i) {
-        geo[i] = geometry(descs[i]);
+        geo[i] = geometry(descs[i], ctx);
         plan->vflags[i] = vec_flags(descs[i]);
-        foff += align_up(carve(descs[i], geo[i], fbase + foff, &scr[i]), 64);
+        foff += align_up(carve(descs[i], geo[i], ctx, fbase + foff, &scr[i]), 64);
     }
 
     // work lists, one per (kernel, template key), in execution order
@@ -425,16 +474,45 @@ int came_b200_plan_create(const CameTensorDesc* descs, int n_tensors, void* work
     };
     const CameTensorDesc* D = descs;
     auto is1d = [&](int i) { return D[i].cols == 0; };
-    auto is2d = [&](int i) { return D[i].cols != 0 && !is_nd(D[i]); };
+    auto isgen = [&](int i) { return ctx.generic(D[i]); };
+    auto is2d = [&](int i) { return D[i].cols != 0 && !is_nd(D[i]) && !isgen(i); };      // staged
     auto isnd = [&](int i) { return is_nd(D[i]); };
-    auto isflat = [&](int i) { return is2d(i) && D[i].mode == CAME_MODE_FLAT8; };
-    auto notflat = [&](int i) { return is2d(i) && D[i].mode != CAME_MODE_FLAT8; };
     auto nokey = [&](int) { return Key{0, 0, 0, 0}; };
     const auto& vf = plan->vflags;
 
-    build(KID_NF_PARTIAL, is1d, [&](int i) { return Key{D[i].g_dtype, 0, 0, 0}; }, [&](int i) { return (int64_t)geo[i].nbR; });
-    build(KID_NF_REDUCE, is1d, nokey, [&](int) { return (int64_t)1; });
-    build(KID_NF_APPLY, is1d, [&](int i) { return Key{D[i].g_dtype, D[i].p_dtype, 0, 0}; }, [&](int i) { return (int64_t)geo[i].nbR; });
+    // Whole-step kernel: one launch per (gradient type, parameter type, layout) of its matrices; the vectors of the
+    // same types ride along with the first of them, or get a launch of their own.
+    {
+        using GKey = std::tuple<int, int, int>;
+        std::map<GKey, std::pair<std::vector<int>, std::vector<int>>> groups;      // matrices, vectors
+        for (int i = 0; i < n_tensors; ++i)
+            if (isgen(i)) groups[GKey{D[i].g_dtype, D[i].p_dtype, D[i].mode}].first.push_back(i);
+        for (int i = 0; i < n_tensors; ++i)
+            if (is1d(i)) {
+                auto it = groups.lower_bound(GKey{D[i].g_dtype, D[i].p_dtype, 0});
+                if (it == groups.end() || std::get<0>(it->first) != D[i].g_dtype || std::get<1>(it->first) != D[i].p_dtype)
+                    it = groups.emplace(GKey{D[i].g_dtype, D[i].p_dtype, CAME_MODE_FP32}, std::pair<std::vector<int>, std::vector<int>>{}).first;
+                it->second.second.push_back(i);
+            }
+        for (auto& kv : groups) {
+            LaunchItem it{};
+            it.kernel = KID_GENERIC;
+            it.key = KernelKey{std::get<0>(kv.first), std::get<1>(kv.first), std::get<2>(kv.first), 1};
+            it.bar = (int)plan->launches.size();
+            auto list = [&](const std::vector<int>& ids, auto count) {
+                const size_t off = work.size();
+                for (int i : ids)
+                    for (int64_t t = 0, c = count(i); t < c; ++t) work.push_back(Work{i, (int32_t)t});
+                return std::pair<size_t, int>{off, (int)(work.size() - off)};
+            };
+            const auto& mats = kv.second.first;
+            std::tie(it.work_off, it.n) = list(mats, [&](int i) { return (int64_t)geo[i].tiles_r * geo[i].tiles_c; });
+            std::tie(it.work2_off, it.n2) = list(mats, [&](int i) { return (int64_t)geo[i].nbR + geo[i].nbC; });
+            std::tie(it.work3_off, it.n3) = list(mats, [&](int i) { return geo[i].flat_chunks; });
+            std::tie(it.work4_off, it.n4) = list(kv.second.second, [&](int i) { return (int64_t)geo[i].nbR; });
+            plan->launches.push_back(it);
+        }
+    }
     // tensors of more than two dimensions
     auto nvec = [&](int i) { return (int64_t)geo[i].nbR + geo[i].nbC; };
     auto nmat = [&](int i) { return (int64_t)D[i].batch; };
@@ -457,26 +535,21 @@ int came_b200_plan_create(const CameTensorDesc* descs, int n_tensors, void* work
     };
     build(KID_SQ_PARTIALS, fusedA, [&](int i) { return Key{D[i].g_dtype, 0, fused_code(i), 2}; },
           [&](int i) { return (int64_t)geo[i].tiles_r; });
-    build(KID_SQ_PARTIALS, twopass, [&](int i) { return Key{D[i].g_dtype, 0, 0, vf[i].k}; },
+    build(KID_SQ_PARTIALS, twopass, [&](int i) { return Key{D[i].g_dtype, 0, 0, 1}; },
           [&](int i) { return (int64_t)geo[i].tiles_r * geo[i].tiles_c; });
     build(KID_SQ_FINALIZE, is2d, nokey, [&](int i) { return (int64_t)geo[i].nbR + geo[i].nbC; });
     // (also for fused-first-pass tensors that carry the clamps: those CTAs return at once unless a clamp binds)
     auto needs_sumsq = [&](int i) { return twopass(i) || (fusedA(i) && (D[i].flags & CAME_F_SQ_CLAMP)); };
-    build(KID_SUMSQ, needs_sumsq, [&](int i) { return Key{D[i].g_dtype, 0, 0, vf[i].k >= 1 ? 1 : 0}; },
+    build(KID_SUMSQ, needs_sumsq, [&](int i) { return Key{D[i].g_dtype, 0, 0, 1}; },
           [&](int i) { return (int64_t)geo[i].tiles_r * geo[i].tiles_c; });
-    // one CTA per tensor for the clip scalar; tensors of the staged momentum pass get one CTA per 2048 entries of
-    // their factor vectors (each CTA repeats the cheap scalar part)
-    build(KID_S_FINALIZE, is2d, nokey, [&](int i) {
-        return vf[i].p2 == 2 ? std::max<int64_t>(1, cdiv(D[i].rows + D[i].cols, S_FIN_CHUNK)) : (int64_t)1;
-    });
+    // one CTA per S_FIN_CHUNK entries of a tensor's factor vectors (each CTA repeats the cheap scalar part)
+    build(KID_S_FINALIZE, is2d, nokey, [&](int i) { return std::max<int64_t>(1, cdiv(D[i].rows + D[i].cols, S_FIN_CHUNK)); });
     // Tensors of the tile layout on the staged path (same element type for g and p) take the fused kernel: their M, F
     // and A items form one list, a tensor's F and A items delayed by `lag` momentum items of later tensors.
     std::vector<char> fused(n_tensors, 0);
     if (!disable_fast() && fused_ma_enabled()) {
         for (int i = 0; i < n_tensors; ++i)
-            fused[i] = is2d(i) && D[i].g_dtype == D[i].p_dtype &&
-                       ((D[i].mode == CAME_MODE_TILE8 && vf[i].p2 == 2 && vf[i].p3 == 2) ||
-                        (D[i].mode == CAME_MODE_FLAT8 && vf[i].p2 == 2 && vf[i].flat == 2));
+            fused[i] = is2d(i) && D[i].g_dtype == D[i].p_dtype && D[i].mode != CAME_MODE_FP32;
     }
     {
         const int grid = persistent_grid_limit();
@@ -534,6 +607,8 @@ int came_b200_plan_create(const CameTensorDesc* descs, int n_tensors, void* work
         }
     }
     plan->fused = fused;
+    plan->pushable = fused;
+    for (int i = 0; i < n_tensors; ++i) plan->pushable[i] = fused[i] || isgen(i);
     // The momentum pass, the residual finalize and the apply pass run wave by wave: a wave is a run of consecutive
     // tensors whose momentum state together stays below `wave_bytes`, so that the codes the momentum pass writes are
     // still in L2 when the apply pass reads them back (0: one wave, every pass covers all tensors).
@@ -553,19 +628,13 @@ int came_b200_plan_create(const CameTensorDesc* descs, int n_tensors, void* work
     }
     for (int w = 0; w < n_waves; ++w) {
         auto in2d = [&](int i) { return is2d(i) && wave[i] == w && !fused[i]; };
-        auto in_notflat = [&](int i) { return notflat(i) && wave[i] == w && !fused[i]; };
-        build(KID_MOMENT, in2d, [&](int i) { return Key{D[i].g_dtype, 0, D[i].mode, vf[i].p2}; },
-              [&](int i) { return (int64_t)geo[i].ptiles_r * geo[i].ptiles_c; });
+        auto in_notflat = [&](int i) { return in2d(i) && D[i].mode != CAME_MODE_FLAT8; };
+        auto in_flat = [&](int i) { return in2d(i) && D[i].mode == CAME_MODE_FLAT8; };
+        auto tiles = [&](int i) { return (int64_t)geo[i].ptiles_r * geo[i].ptiles_c; };
+        build(KID_MOMENT, in2d, [&](int i) { return Key{D[i].g_dtype, 0, D[i].mode, 2}; }, tiles);
         build(KID_RES_FINALIZE, in2d, nokey, [&](int i) { return (int64_t)geo[i].nbR + geo[i].nbC; });
-        build(KID_APPLY, in_notflat, [&](int i) { return Key{0, D[i].p_dtype, D[i].mode, vf[i].p3}; },
-              [&](int i) { return (int64_t)geo[i].ptiles_r * geo[i].ptiles_c; });
-        auto flat_generic = [&](int i) { return isflat(i) && vf[i].flat != 2 && wave[i] == w; };
-        auto flat_staged = [&](int i) { return isflat(i) && vf[i].flat == 2 && wave[i] == w && !fused[i]; };
-        build(KID_FACTORS, flat_generic, nokey, [&](int i) { return (int64_t)geo[i].nbR + geo[i].nbC; });
-        build(KID_APPLY_FLAT, flat_generic, [&](int i) { return Key{D[i].g_dtype, D[i].p_dtype, 0, vf[i].flat}; },
-              [&](int i) { return geo[i].flat_chunks; });
-        build(KID_APPLY_FLAT, flat_staged, [&](int i) { return Key{D[i].g_dtype, D[i].p_dtype, 0, 2}; },
-              [&](int i) { return (int64_t)geo[i].ptiles_r * geo[i].ptiles_c; });
+        build(KID_APPLY, in_notflat, [&](int i) { return Key{0, D[i].p_dtype, D[i].mode, 2}; }, tiles);
+        build(KID_APPLY_FLAT, in_flat, [&](int i) { return Key{D[i].g_dtype, D[i].p_dtype, 0, 2}; }, tiles);
     }
 
     if (work.size() > L.n_work) {
@@ -578,7 +647,7 @@ int came_b200_plan_create(const CameTensorDesc* descs, int n_tensors, void* work
                                     cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(plan->ws + L.off_scr, scr.data(), (size_t)n_tensors * sizeof(Scratch), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(plan->ws + L.off_status, 0, sizeof(int), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(plan->ws + L.off_status, 0, L.off_work - L.off_status, st);      // status word, barriers, counters
     // the scratch starts at zero once (flags in it are reset by the kernels that use them)
     if (e == cudaSuccess) e = cudaMemsetAsync(plan->ws + L.off_float, 0, L.total - L.off_float, st);
     if (e == cudaSuccess && !work.empty())
@@ -591,6 +660,7 @@ int came_b200_plan_create(const CameTensorDesc* descs, int n_tensors, void* work
         delete plan;
         return fail(CAME_E_CUDA, "plan_create: %s", cudaGetErrorString(e));
     }
+    for (const LaunchItem& it : plan->launches) plan->needs_hyp = plan->needs_hyp || it.kernel != KID_GENERIC;
     *out = plan;
     return CAME_OK;
 }
@@ -616,7 +686,7 @@ int came_b200_plan_set_push(came_plan_t* plan, const void* local_base, size_t lo
     const uintptr_t buf_lo = reinterpret_cast<uintptr_t>(local_base), buf_hi = buf_lo + local_bytes;
     if (buf_lo % 16 != 0) return fail(CAME_E_INVALID, "plan_set_push: the local buffer is not 16-byte aligned");
     for (int i = 0; i < plan->n_tensors; ++i)
-        if (plan->fused[i] && !param_in_range(buf_lo, buf_hi, plan->descs[i]))
+        if (plan->pushable[i] && !param_in_range(buf_lo, buf_hi, plan->descs[i]))
             return fail(CAME_E_INVALID, "plan_set_push: tensor %d does not lie inside the local buffer", i);
     long long delta[MAX_PUSH_PEERS];
     for (int k = 0; k < n_peers; ++k) {
@@ -634,7 +704,7 @@ int came_b200_plan_set_push(came_plan_t* plan, const void* local_base, size_t lo
 int came_b200_plan_pushed(const came_plan_t* plan, int* flags, int n_tensors) {
     if (!plan || !flags) return fail(CAME_E_INVALID, "plan_pushed: null argument");
     if (n_tensors != plan->n_tensors) return fail(CAME_E_INVALID, "plan_pushed: %d tensors given, plan has %d", n_tensors, plan->n_tensors);
-    for (int i = 0; i < n_tensors; ++i) flags[i] = plan->fused[i] ? 1 : 0;
+    for (int i = 0; i < n_tensors; ++i) flags[i] = plan->pushable[i] ? 1 : 0;
     return CAME_OK;
 }
 
@@ -649,7 +719,7 @@ int came_b200_plan_set_pointers(came_plan_t* plan, const void* const* g, void* c
         if (!next[i].g || !next[i].p) return fail(CAME_E_INVALID, "set_pointers: tensor %d: null pointer", i);
         if (!(vec_flags(next[i]) == plan->vflags[i]))
             return fail(CAME_E_INVALID, "set_pointers: tensor %d changes 16-byte alignment class; create a new plan", i);
-        if (plan->n_push > 0 && plan->fused[i] && !pushed_param_in_range(*plan, next[i]))
+        if (plan->n_push > 0 && plan->pushable[i] && !pushed_param_in_range(*plan, next[i]))
             return fail(CAME_E_INVALID, "set_pointers: tensor %d leaves the buffer the push mode was set up for", i);
     }
     plan->descs.swap(next);
@@ -675,17 +745,23 @@ int came_b200_step(came_plan_t* plan, const CameHyper* hypers, int n_groups, cam
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) { cap = cudaStreamCaptureStatusNone; cudaGetLastError(); }
     const bool capturing = cap == cudaStreamCaptureStatusActive;
-    std::vector<CameHyper> norm(hypers, hypers + n_groups);      // pageable source: read before the copy call returns
-    normalise_hypers(norm.data(), n_groups);
-    const CameHyper* src = norm.data();
+    CameHyper norm[MAX_GROUPS];      // pageable source: read before the copy call returns
+    std::memcpy(norm, hypers, (size_t)n_groups * sizeof(CameHyper));
+    normalise_hypers(norm, n_groups);
+    const CameHyper* src = norm;
     if (capturing) {
         rc = stage_graph_hypers("step", plan, hypers, n_groups);
         if (rc != CAME_OK) return rc;
         src = plan->graph_hyp;
     }
-    cudaError_t e = cudaMemcpyAsync(plan->ws + plan->L.off_hyp, src, (size_t)n_groups * sizeof(CameHyper),
-                                    cudaMemcpyHostToDevice, st);
-    if (e != cudaSuccess) return fail(CAME_E_CUDA, "step: hyper-parameter upload: %s", cudaGetErrorString(e));
+    // The whole-step kernel takes a few records as kernel arguments; a captured step reads them from memory, so that a
+    // replay sees new values.
+    const bool by_value = !capturing && n_groups <= GENERIC_MAX_HYP;
+    cudaError_t e = cudaSuccess;
+    if (plan->needs_hyp || !by_value) {
+        e = cudaMemcpyAsync(plan->ws + plan->L.off_hyp, src, (size_t)n_groups * sizeof(CameHyper), cudaMemcpyHostToDevice, st);
+        if (e != cudaSuccess) return fail(CAME_E_CUDA, "step: hyper-parameter upload: %s", cudaGetErrorString(e));
+    }
     const bool timing = plan->timing && !capturing;      // events are not recorded into a graph
     StepArgs a{reinterpret_cast<const CameTensorDesc*>(plan->ws + plan->L.off_descs),
                reinterpret_cast<const Scratch*>(plan->ws + plan->L.off_scr),
@@ -706,8 +782,11 @@ int came_b200_step(came_plan_t* plan, const CameHyper* hypers, int n_groups, cam
                 return fail(CAME_E_CUDA, "step: cudaEventCreate failed");
             cudaEventRecord(tm.t0, st);
         }
-        if (it.kernel == KID_NF_PARTIAL || it.kernel == KID_NF_APPLY || it.kernel == KID_NF_REDUCE)
-            e = launch_nonfactored(it.kernel, it.key, a, wbase + it.work_off, it.n, st);
+        if (it.kernel == KID_GENERIC) {
+            const GenericLists l{wbase + it.work_off, wbase + it.work2_off, wbase + it.work3_off, wbase + it.work4_off,
+                                 it.n, it.n2, it.n3, it.n4, reinterpret_cast<int*>(plan->ws + plan->L.off_bar) + 2 * it.bar};
+            e = launch_generic(it.key, a, by_value ? norm : nullptr, n_groups, l, st);
+        }
         else if (it.kernel == KID_SQ_PARTIALS && it.key.variant == 2)
             e = launch_fused_sq(it.key, a, wbase + it.work_off, it.n, st);
         else if (it.kernel >= KID_ND_SQ && it.kernel <= KID_ND_APPLY)
@@ -825,7 +904,7 @@ const char* came_b200_kernel_name(int kernel) {
     static const char* names[CAME_KERNEL_COUNT] = {
         "sq_partials", "sq_finalize", "sumsq", "s_finalize", "moment", "res_finalize",
         "apply", "factors", "apply_flat", "nf_partial", "nf_apply", "nf_reduce", "nd_sq", "nd_mean", "nd_sumsq", "nd_s", "nd_res",
-        "nd_resmean", "nd_apply", "moment_apply"};
+        "nd_resmean", "nd_apply", "moment_apply", "generic"};
     return (kernel >= 0 && kernel < CAME_KERNEL_COUNT) ? names[kernel] : "?";
 }
 

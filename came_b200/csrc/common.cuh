@@ -18,16 +18,11 @@ constexpr float QMAX_U8 = 255.0f;
 // reduction tile of the gradient passes (rows x cols handled by one CTA)
 constexpr int K_TR = 128;
 constexpr int K_TC = 512;
-// tile of the momentum / apply passes
-constexpr int P_TR = 128;
-constexpr int P_TC = 256;
 constexpr int THREADS = 256;
 // tile of the shared-memory staged (tile-layout) momentum / apply passes
 constexpr int W_TR = 128;
 constexpr int W_TC = 1024;
 constexpr int W_THREADS = 512;
-// flat blocks (of 256 elements) handled by one CTA of the flat-layout apply pass
-constexpr int FLAT_BLOCKS_PER_CTA = 64;
 
 // Per-tensor scratch, laid out in the caller's workspace by the plan.  All pointers are device
 // pointers to fp32.
@@ -42,16 +37,18 @@ struct Scratch {
     float* rowpart;   // [max(tiles_c, ptiles_c) * rows]  per-CTA row partial sums
     float* colpart;   // [tiles_r * cols]                 per-CTA column partial sums
     float* spart;     // [tiles_r * tiles_c] partials of S; 1-D tensors: [nbR] block partials of sum u^2
-    float* fac;       // flat layout only: r[rows], c[cols], R'[rows], C'[cols] factors, else nullptr
+    float* fac;       // flat layout on generic.cu: row factors r_i [rows], else nullptr
     float* tpart;     // fused first pass only: [tiles_r * cols] per-strip column sums of g^2 / v_row
     int32_t tiles_r, tiles_c;     // K_TR x K_TC grid
-    int32_t ptiles_r, ptiles_c;   // P_TR x P_TC grid (W_TR x W_TC when the staged fast path runs)
+    int32_t ptiles_r, ptiles_c;   // W_TR x W_TC grid of the staged passes
     int32_t nbR, nbC;             // ceil(rows/256), ceil(cols/256)
     int32_t fused_a;              // 1: the fused first pass runs (complete row sums, v_row and tpart come from it)
     int32_t fa_rb;                // fused first pass: rows per staged batch
     float* mfac;                  // staged momentum pass: row factors r_i / clip [R]
     float* mfac_c;                // staged passes: column factors [C], 16-byte aligned (c_j; after the residual finalize C'_j)
     float* mfac_c2;               // flat layout on the staged path: C'_j (c_j stays in mfac_c for the apply items), else nullptr
+    int32_t g_v, g_nb;            // generic.cu: elements per access (8 or 1), bands of 16 rows per item
+    int32_t* counters;            // generic.cu: items through with a phase (zero between launches)
     int32_t sq_col_parts;         // column partial sets the first pass leaves (strips, or strips x 2 warp groups)
     int32_t res_eps_deferred;     // 1: the residual partials hold sums of (u-m)^2 only; eps1 is added per row / column
                                   //    by the finalize kernel (cols * eps1, rows * eps1)
@@ -136,50 +133,6 @@ __device__ __forceinline__ void load_run(const __half* p, int64_t off, int col, 
     } else {
 #pragma unroll
         for (int e = 0; e < N; ++e) v[e] = (col + e < ncols) ? __half2float(p[off + e]) : 0.0f;
-    }
-}
-
-// N contiguous int8 codes -> fp32 (N = 8 or 16)
-template <int N, bool VEC>
-__device__ __forceinline__ void load_codes(const int8_t* p, int64_t off, int col, int ncols, float* v) {
-    if (VEC) {
-        uint32_t w[N / 4];
-        if (N == 16) {
-            const uint4 r = *reinterpret_cast<const uint4*>(p + off);
-            w[0] = r.x; w[1] = r.y; w[2] = r.z; w[3] = r.w;
-        } else {
-            const uint2 r = *reinterpret_cast<const uint2*>(p + off);
-            w[0] = r.x; w[1] = r.y;
-        }
-#pragma unroll
-        for (int i = 0; i < N / 4; ++i) {
-#pragma unroll
-            for (int b = 0; b < 4; ++b) v[4 * i + b] = (float)(int)(int8_t)((w[i] >> (8 * b)) & 0xffu);
-        }
-    } else {
-#pragma unroll
-        for (int e = 0; e < N; ++e) v[e] = (col + e < ncols) ? (float)p[off + e] : 0.0f;
-    }
-}
-
-template <int N, bool VEC>
-__device__ __forceinline__ void store_codes(int8_t* p, int64_t off, int col, int ncols, const int* q) {
-    if (VEC) {
-        uint32_t w[N / 4];
-#pragma unroll
-        for (int i = 0; i < N / 4; ++i) {
-            w[i] = ((uint32_t)q[4 * i] & 0xffu) | (((uint32_t)q[4 * i + 1] & 0xffu) << 8) |
-                   (((uint32_t)q[4 * i + 2] & 0xffu) << 16) | (((uint32_t)q[4 * i + 3] & 0xffu) << 24);
-        }
-        if (N == 16) {
-            *reinterpret_cast<uint4*>(p + off) = make_uint4(w[0], w[1], w[2], w[3]);
-        } else {
-            *reinterpret_cast<uint2*>(p + off) = make_uint2(w[0], w[1]);
-        }
-    } else {
-#pragma unroll
-        for (int e = 0; e < N; ++e)
-            if (col + e < ncols) p[off + e] = (int8_t)q[e];
     }
 }
 
@@ -304,10 +257,6 @@ __device__ __forceinline__ int quant_u8_div(float x, float absmax) {
     const float q = rintf((x / absmax) * QMAX_U8);
     return (int)fminf(QMAX_U8, fmaxf(0.0f, q));
 }
-__device__ __forceinline__ int quant_i8_fast(float x, float absmax, float inv) {
-    const float q = rintf(div_by(x, absmax, inv) * QMAX_I8);
-    return (int)fminf(QMAX_I8, fmaxf(-QMAX_I8, q));
-}
 // The reciprocal trick needs 1/absmax and the residual to stay normal; outside this range take the
 // plain division (uniform per block, so no divergence inside a warp's block).
 __device__ __forceinline__ bool recip_safe(float absmax) { return absmax > 1e-30f && absmax < 1e30f; }
@@ -381,27 +330,59 @@ __device__ __forceinline__ float col_factor(float v, bool clamp) {
 // 1 / sqrt(x) by one Newton step y (3 - x y^2) / 2 from the hardware's approximation: within one unit in the last place, like
 // a rounded division of a rounded square root, in a fifth of the instructions.  Outside the range in which no term
 // under- or overflows: those two.
+static __device__ __noinline__ float inv_sqrt_plain(float x) { return 1.0f / sqrtf(x); }      // (out of line: rare, and long)
 __device__ __forceinline__ float inv_sqrt(float x) {
-    if (!(x > 1e-30f && x < 1e30f)) return 1.0f / sqrtf(x);
+    if (!(x > 1e-30f && x < 1e30f)) return inv_sqrt_plain(x);
     const float y = rsqrtf(x);
     return fmaf(0.5f * y, fmaf(-x * y, y, 1.0f), y);
 }
 
 // ------------------------------------------------------------------------------------------
-// weight decay + update of one parameter value, in the three forms the reference uses
+// weight decay + update of one parameter value, in the three forms the reference uses (wd_form: 0 no decay, 1 one
+// rounding, 2 multiply form with a rounding to the parameter's type, 3 subtract form with one); every fused multiply-add
+// is written out, so that all kernels agree bit for bit
 // ------------------------------------------------------------------------------------------
-template <typename TP>
-__device__ __forceinline__ float apply_one(float pv, float upd, const CameHyper& h, uint32_t flags) {
-    if (h.weight_decay != 0.0f) {
-        if (flags & CAME_F_WD_MUL2) {
-            pv = round_to<TP>(pv * h.decay_mul);
-        } else if (flags & CAME_F_WD_ADD2) {
-            pv = round_to<TP>(pv - h.wd_lr * pv);
-        } else {
-            pv = pv - h.wd_lr * pv;
-        }
-    }
-    return pv - h.lr * upd;
+__device__ __forceinline__ int wd_form(const CameHyper& h, uint32_t flags) {
+    return h.weight_decay == 0.0f ? 0 : ((flags & CAME_F_WD_MUL2) ? 2 : ((flags & CAME_F_WD_ADD2) ? 3 : 1));
+}
+// (selects, no branches: wd is uniform, but a branch per element would serialise the elements of a thread)
+template <typename RND>
+__device__ __forceinline__ float apply_step(float pv, float upd, float lr, float wd_lr, float decay_mul, int wd, RND round) {
+    const float x = wd == 2 ? __fmul_rn(pv, decay_mul) : wd == 0 ? pv : fmaf(-wd_lr, pv, pv);
+    return fmaf(-lr, upd, wd >= 2 ? round(x) : x);
+}
+
+// ------------------------------------------------------------------------------------------
+// 1-D tensors: second moment, update before the clip, momentum (came_kernels.cu:1035-1042, 1489-1601)
+// ------------------------------------------------------------------------------------------
+__device__ __forceinline__ float nf_second_moment(float old, float g, const CameHyper& h) {
+    return fmaf(old, h.beta2, __fmul_rn(h.om_beta2, fmaf(g, g, h.eps0)));
+}
+__device__ __forceinline__ float nf_update(float v, float g, uint32_t flags) {
+    return __fmul_rn(inv_sqrt((flags & CAME_F_RSQRT_CLAMP) ? fmaxf(v, 1e-30f) : v), g);
+}
+__device__ __forceinline__ float nf_clip(float S, int64_t n, const CameHyper& h) {
+    return fmaxf(1.0f, sqrtf(S / (float)n) / h.clip_threshold);
+}
+// (clip >= 1: the quotient by div_by is the correctly rounded one unless it is close to underflow)
+__device__ __forceinline__ float nf_momentum(float m_old, float u, float clip, float inv_clip, uint32_t flags, const CameHyper& h) {
+    if (flags & CAME_F_UPDATE_F16) u = __half2float(__float2half_rn(u));
+    return fmaf(m_old, h.beta1, __fmul_rn(h.om_beta1, clip == 1.0f ? u : div_by(u, clip, inv_clip)));
+}
+
+// ------------------------------------------------------------------------------------------
+// sums of per-item partials in a fixed order: groups of 64 consecutive ones, then the groups (one warp each)
+// ------------------------------------------------------------------------------------------
+constexpr int PARTIAL_GROUP = 64;
+__device__ __forceinline__ float partial_group_sum(const float* part, int g, int n, int lane) {
+    const int i = g * PARTIAL_GROUP + lane;
+    const float x = i < n ? __ldcg(part + i) : 0.0f, y = i + 32 < n ? __ldcg(part + i + 32) : 0.0f;
+    return warp_sum(x + y);
+}
+__device__ __forceinline__ float partial_total(const float* groups, int ng, int lane) {
+    float t = 0.0f;
+    for (int i = lane; i < ng; i += 32) t += __ldcg(groups + i);
+    return warp_sum(t);
 }
 
 }  // namespace came

@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(FPM_ALL_THREADS, 1) k_moment_fp32_wide(StepArg
 }
 
 // ------------------------------------------------------------------------------------------------
-// apply pass: p -= lr * m * R'_i * C'_j, with the weight-decay forms of apply_one
+// apply pass: p -= lr * m * R'_i * C'_j, with the weight-decay forms of apply_step
 // ------------------------------------------------------------------------------------------------
 template <typename TP>
 __global__ void __launch_bounds__(W_ALL_THREADS, 1) k_apply_fp32_wide(StepArgs a, const Work* __restrict__ work, int n_items) {

@@ -1,0 +1,1001 @@
+// The whole step of any set of matrices and vectors as ONE cooperative kernel: every shape and alignment, and the sets
+// that are too small for the staged kernels.
+//
+// The staged kernels (fused_sq.cu, fused_ma.cu, fp_wide.cu) move 128 x 1024 tiles through one CTA per SM and need columns
+// in multiples of 64.  Two kinds of work do not fit them.  Small sets: eight such tiles leave 140 SMs idle, and the seven
+// launches of a step, each 2-5 us with its gap, are most of its time.  Odd widths, unaligned buffers and thin matrices:
+// no bulk copies.  Here a step is six phases of one kernel, separated by grid-wide barriers:
+//
+//   S1  g                 -> row / column partial sums of g^2          1-D tensors: partials of sum u^2, their sum
+//   F1  partials          -> v_row, c_j, requantised states, mean      1-D tensors: v, m, p
+//   S2  g                 -> partials of S = sum (g r c)^2; the tensor's last item leaves S and the clip
+//   M   g, m              -> m, row / column partials of (u - m)^2     (flat layout: m is not written yet)
+//   F2  partials          -> residual vectors, C'_j, mean
+//   A   m, p (flat: g too) -> p (flat: m too)
+//
+// What bounds it: latency in small sets (a phase is a chain of dependent loads, and its code is fetched cold), bytes in
+// flight and instruction issue in large ones.  So the unit of work on a matrix is a warp, not a CTA: bands of 16 rows x 64
+// columns, which hold whole 16 x 16 tiles of the momentum; nothing meets at a CTA barrier.  A band and everything it needs
+// (vector slices, absmax) comes to the warp's own shared memory by 16-byte asynchronous copies of the aligned chunks that
+// cover its rows, whatever the rows' alignment, and (16-bit types) the next band is under way while one is computed.  V =
+// 8: rows on 16-byte boundaries, a lane owns 8 consecutive columns of 4 rows; V = 1: any alignment, a lane owns columns
+// lane and lane + 32 of 16 rows.  Items are dealt out across the SMs first.  All reductions have a fixed order: of the items
+// that share a result the last to finish (a counter) adds the partials in index order.
+#include "common.cuh"
+#include "launch.h"
+#include "pipeline.cuh"
+
+#include <algorithm>
+#include <map>
+#include <mutex>
+#include <type_traits>
+#include <utility>
+
+namespace came {
+
+namespace {
+
+constexpr int G_WARPS = THREADS / 32;
+constexpr uint32_t G_POLL_LIMIT = 1u << 22;      // polls of the grid barrier (seconds) before a CTA gives up
+
+// ---- element buffers: one type, or (g and p of different types) a type read at run time --------------------------
+template <typename T> struct Buf {
+    T* p;
+    __device__ __forceinline__ Buf(const void* q, int) : p(reinterpret_cast<T*>(const_cast<void*>(q))) {}
+    __device__ __forceinline__ float get(int64_t i) const { return to_f32(p[i]); }
+    __device__ __forceinline__ void get8(int64_t i, float* v) const { load_run<8, true>(p, i, 0, 8, v); }
+    __device__ __forceinline__ float round(float x) const { return round_to<T>(x); }
+    __device__ __forceinline__ void put(int64_t i, float x, int64_t delta = 0) const {
+        *reinterpret_cast<T*>(reinterpret_cast<char*>(p + i) + delta) = from_f32<T>(x);
+    }
+    __device__ __forceinline__ void put8(int64_t i, const float* v, int64_t delta = 0) const {
+        store_run<8, true>(reinterpret_cast<T*>(reinterpret_cast<char*>(p) + delta), i, 0, 8, v);
+    }
+};
+struct Any {};
+template <> struct Buf<Any> {
+    void* p;
+    int dt;
+    __device__ __forceinline__ Buf(const void* q, int t) : p(const_cast<void*>(q)), dt(t) {}
+    template <typename F> __device__ __forceinline__ void with(F f) const {
+        if (dt == CAME_DT_F32) f(Buf<float>(p, 0));
+        else if (dt == CAME_DT_F16) f(Buf<__half>(p, 0));
+        else f(Buf<__nv_bfloat16>(p, 0));
+    }
+    __device__ __forceinline__ float get(int64_t i) const { float x; with([&](auto b) { x = b.get(i); }); return x; }
+    __device__ __forceinline__ void get8(int64_t i, float* v) const { with([&](auto b) { b.get8(i, v); }); }
+    __device__ __forceinline__ float round(float x) const { float y; with([&](auto b) { y = b.round(x); }); return y; }
+    __device__ __forceinline__ void put(int64_t i, float x, int64_t delta = 0) const { with([&](auto b) { b.put(i, x, delta); }); }
+    __device__ __forceinline__ void put8(int64_t i, const float* v, int64_t delta = 0) const { with([&](auto b) { b.put8(i, v, delta); }); }
+};
+
+struct GShared {
+    float red[33];
+    int last;
+    float col[G_WARPS][QBLOCK];
+};
+
+// (acquire-release instead of __threadfence(), which is sequentially consistent and waits longer)
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+__device__ __forceinline__ int atom_add_acq_rel(int* p, int x) {
+    int old;
+    asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(x) : "memory");
+    return old;
+}
+__device__ __forceinline__ int ld_acquire_gpu(const int* p) {
+    int v;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// Grid-wide barrier of a cooperative launch.  bar[0] counts arrivals and is back at zero afterwards, bar[1] is the
+// generation.  False when the others did not arrive within the limit (the status word is set; the CTA then leaves).
+__device__ __forceinline__ bool grid_barrier(int* bar, int* status) {
+    __shared__ int s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s_ok = 1;
+        fence_gpu();      // (the whole CTA's writes: they happened before the barrier above)
+        const int g = ld_acquire_gpu(bar + 1);
+        if (atom_add_acq_rel(bar, 1) == (int)gridDim.x - 1) {
+            *reinterpret_cast<volatile int*>(bar) = 0;
+            atom_add_acq_rel(bar + 1, 1);
+        } else {
+            uint32_t polls = 0;
+            while (ld_acquire_gpu(bar + 1) == g)
+                if (++polls > G_POLL_LIMIT) { atomicExch(status, STATUS_MBAR_TIMEOUT); s_ok = 0; break; }
+        }
+        fence_gpu();
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
+// True in every thread of the CTA that is the last of `total` to come here (the counter is then back at zero); the
+// other CTAs' writes are visible to it.
+__device__ __forceinline__ bool last_cta(int* counter, int total, GShared& sh) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        fence_gpu();      // (the whole CTA's writes: they happened before the barrier)
+        const int before = atom_add_acq_rel(counter, 1);
+        sh.last = before == total - 1;
+        if (sh.last) *counter = 0;
+        fence_gpu();
+    }
+    __syncthreads();
+    return sh.last;
+}
+__device__ __forceinline__ float block_vector_sum_cg(const float* x, int n, float* red) {
+    float t = 0.0f;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) t += __ldcg(x + i);
+    return block_sum(t, red);
+}
+
+// True (in every lane) when this warp is the last of `total` to come here; the counter is then back at zero and the
+// other warps' writes are visible.
+__device__ __forceinline__ bool last_warp(int* counter, int total, int lane) {
+    __syncwarp();
+    int before = 0;
+    if (lane == 0) {
+        fence_gpu();
+        before = atom_add_acq_rel(counter, 1);
+        if (before == total - 1) *counter = 0;
+        fence_gpu();
+    }
+    return __shfl_sync(0xffffffffu, before, 0) == total - 1;
+}
+// Sum of n partials, one per item, in index order: the last of every 64 items adds their partials (leave_partial); up to
+// 32 such groups the readers add themselves (read_sum: one load per lane, cheaper than one more chain of a fence, an atomic
+// and a load before the grid barrier), more the last group adds.
+// part: n partials, the groups' sums, the total; counters: one for the groups, then one per group.
+__device__ __forceinline__ void leave_partial(float* part, int* counters, int i, int n, float x, int lane) {
+    const int ng = (n + PARTIAL_GROUP - 1) / PARTIAL_GROUP, g = i / PARTIAL_GROUP;
+    if (lane == 0) part[i] = x;
+    if (!last_warp(counters + 1 + g, min(PARTIAL_GROUP, n - g * PARTIAL_GROUP), lane)) return;
+    const float t = partial_group_sum(part, g, n, lane);
+    if (lane == 0) part[n + g] = t;
+    if (ng <= 32 || !last_warp(counters, ng, lane)) return;
+    const float sum = partial_total(part + n, ng, lane);
+    if (lane == 0) part[n + ng] = sum;
+}
+__device__ __forceinline__ float read_sum(const float* part, int n, int lane) {
+    const int ng = (n + PARTIAL_GROUP - 1) / PARTIAL_GROUP;
+    if (ng > 32) return __ldcg(part + n + ng);
+    return warp_sum(lane < ng ? __ldcg(part + n + lane) : 0.0f);
+}
+// mean of a vector from the sums of its blocks of 256 entries, guarded
+__device__ __forceinline__ float read_mean(const float* blk, int nb, int n, bool fix, bool clamp, int lane) {
+    float t = 0.0f;
+    for (int i = lane; i < nb; i += 32) t += __ldcg(blk + i);
+    return guard_mean(warp_sum(t) / (float)n, fix, clamp);
+}
+
+// ---- a warp's item of a matrix ---------------------------------------------------------------------------------
+constexpr int G_CW = 64;      // columns of an item
+
+template <typename T> struct Size { static constexpr int BYTES = sizeof(T); };
+template <> struct Size<Any> { static constexpr int BYTES = 4; };      // the largest
+template <typename T> __device__ __forceinline__ int size_of(int dt) {
+    if constexpr (std::is_same<T, Any>::value) return dt == CAME_DT_F32 ? 4 : 2;
+    else return (int)sizeof(T);
+}
+
+// One band (16 rows x 64 columns) in a warp's shared memory: rows of operand A (g or p) and of the momentum, each from the
+// 16-byte boundary at or before its first byte; the band's 16 row values, 64 column factors, and absmax values.
+template <typename T, int MODE> struct Stage {
+    static constexpr int PA = G_CW * Size<T>::BYTES + 16;
+    static constexpr int PM = G_CW * (MODE == CAME_MODE_FP32 ? 4 : 1) + 16;
+    static constexpr int OFF_M = 16 * PA, OFF_V = OFF_M + 16 * PM, OFF_C = OFF_V + 16 * 4, OFF_X = OFF_C + G_CW * 4, BYTES = OFF_X + 32 * 4;
+    // two stages where a third CTA per SM still fits beside them
+    static constexpr int COUNT = 2 * G_WARPS * BYTES <= 72 * 1024 ? 2 : 1;
+};
+
+__device__ __forceinline__ void cp16(void* dst, const void* src, int bytes) {      // bytes < 16: the rest becomes zero
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp4(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+struct Item {
+    int tensor, tile, R, C, tr, tc, brow, col0, k, nb;      // brow: first row of band k of nb
+    bool v8;
+    __device__ __forceinline__ void decode(const StepArgs& a, const Work& w) {
+        const CameTensorDesc& d = a.descs[w.tensor];
+        const Scratch& s = a.scr[w.tensor];
+        tensor = w.tensor; tile = w.tile;
+        R = (int)d.rows; C = (int)d.cols;
+        tr = w.tile / s.tiles_c; tc = w.tile - tr * s.tiles_c;
+        brow = tr * s.g_nb * 16; col0 = tc * G_CW; k = 0;
+        nb = min(s.g_nb, (R - brow + 15) >> 4);
+        v8 = s.g_v == 8;
+    }
+};
+
+// The band's rows of an array of R x C elements of `esz` bytes.  Rows past the end are zero-filled; the columns past the
+// end of a row are the next row's (the reader masks them).  A chunk may begin before the array or end behind it only
+// inside the same 16 bytes, and of the last one only the array's bytes are read.
+__device__ __forceinline__ void stage_rows(char* dst, int pitch, const void* base, int esz, const Item& it, int lane) {
+    const int nch = G_CW / 16 * esz + 1, rows = min(16, it.R - it.brow), width = min(G_CW, it.C - it.col0) * esz;
+    const uintptr_t b = reinterpret_cast<uintptr_t>(base), end = b + (uintptr_t)((int64_t)it.R * it.C * esz);
+    const uintptr_t first = b + (uintptr_t)(((int64_t)it.brow * it.C + it.col0) * esz);
+    const int pitch_g = it.C * esz;      // (rows of a chunk below 2^31 bytes: C < 2^29)
+    for (int j = lane; j < 16 * nch; j += 32) {
+        const int r = j / nch, ch = j - r * nch;
+        const uintptr_t row = first + (uintptr_t)((int64_t)r * pitch_g), src = (row & ~(uintptr_t)15) + 16 * ch;
+        const bool want = r < rows && src < row + width;
+        cp16(dst + r * pitch + 16 * ch, reinterpret_cast<const void*>(want ? src : b & ~(uintptr_t)15),
+             want ? (int)min((uintptr_t)16, end - src) : 0);
+    }
+}
+// 16 row values from `v`, 64 column values from `c` (arrays of the workspace: 16-byte aligned, padded to 4 values)
+__device__ __forceinline__ void stage_vectors(char* st, int off_v, int off_c, const float* v, const float* c, const Item& it, int lane) {
+    if (lane < 16) {
+        const int col = it.col0 + 4 * lane;
+        cp16(st + off_c + 16 * lane, c + (col < it.C ? col : 0), col < it.C ? 16 : 0);
+    } else if (lane < 20) {
+        const int row = it.brow + 4 * (lane - 16);
+        cp16(st + off_v + 16 * (lane - 16), v + (row < it.R ? row : 0), row < it.R ? 16 : 0);
+    }
+}
+// tile layout: the absmax of the band's four tiles; flat layout: of the two flat blocks a row's columns may lie in
+template <int MODE>
+__device__ __forceinline__ void stage_absmax(char* x, const float* absmax, const Item& it, int lane) {
+    if (MODE == CAME_MODE_TILE8) {
+        const int tile_cols = (it.C + TILE - 1) / TILE, t = (it.col0 >> 4) + lane;
+        if (lane < 4 && t < tile_cols) cp4(x + 4 * lane, absmax + (int64_t)(it.brow >> 4) * tile_cols + t);
+    } else if (MODE == CAME_MODE_FLAT8) {
+        const int row = min(it.brow + (lane >> 1), it.R - 1);
+        const int64_t last = ((int64_t)it.R * it.C - 1) >> 8, blk = (((int64_t)row * it.C + it.col0) >> 8) + (lane & 1);
+        cp4(x + 4 * lane, absmax + min(blk, last));
+    }
+}
+
+// Walks a warp's items band by band: issue(item, stage) starts the copies of a band, proc(item, stage) computes it.
+template <int STAGES, typename ISSUE, typename PROC>
+__device__ __forceinline__ void stream(const StepArgs& a, const Work* list, int n, int first, int stride, ISSUE issue, PROC proc) {
+    if (first >= n) return;
+    Item it;
+    it.decode(a, list[first]);
+    issue(it, 0);
+    cp_commit();
+    Work ahead = list[min(first + stride, n - 1)];
+    int st = 0;
+    for (int i = first;;) {
+        Item nx = it;
+        bool more = true;
+        if (++nx.k < it.nb) {
+            nx.brow += 16;
+        } else {
+            i += stride;
+            more = i < n;
+            if (more) {
+                nx.decode(a, ahead);
+                ahead = list[min(i + stride, n - 1)];
+            }
+        }
+        if (STAGES == 2) {
+            if (more) issue(nx, st ^ 1);
+            cp_commit();
+            cp_wait<1>();
+        } else {
+            cp_wait<0>();
+        }
+        __syncwarp();
+        proc(it, st);
+        __syncwarp();      // the stage is read before it is filled again
+        if (STAGES == 1 && more) { issue(nx, 0); cp_commit(); }
+        if (!more) break;
+        it = nx;
+        if (STAGES == 2) st ^= 1;
+    }
+    cp_wait<0>();
+}
+
+// How a lane reads its part of a band.  V = 8: columns 8 (lane & 7) .. + 7 of rows (lane >> 3) + 4 i; V = 1: columns lane
+// and lane + 32 of row i.
+template <int V> struct Lane {
+    static constexpr int NR = V == 8 ? 4 : 16, E = V == 8 ? 8 : 2;
+    static __device__ __forceinline__ int row(int lane, int i) { return V == 8 ? (lane >> 3) + 4 * i : i; }
+    static __device__ __forceinline__ int col(int lane, int e) { return V == 8 ? 8 * (lane & 7) + e : lane + 32 * e; }
+};
+// Elements of row r of a staged array; `low`: byte offset of the row's first element from a 16-byte boundary
+template <int V, typename T>
+__device__ __forceinline__ void read_row(const char* rows, int pitch, int dt, int low, int r, int lane, float* x) {
+    const Buf<T> b(rows + r * pitch + (V == 8 ? 0 : low), dt);
+    if constexpr (V == 8) b.get8(8 * (lane & 7), x);
+    else { x[0] = b.get(lane); x[1] = b.get(lane + 32); }
+}
+template <int V>
+__device__ __forceinline__ void read_codes(const char* rows, int pitch, int low, int r, int lane, float* x) {
+    if constexpr (V == 8) {
+        const uint2 q = *reinterpret_cast<const uint2*>(rows + r * pitch + low + 8 * (lane & 7));
+        const uint32_t w[2] = {q.x ^ 0x80808080u, q.y ^ 0x80808080u};
+#pragma unroll
+        for (int e = 0; e < 8; e += 2) { const u64 f = codes_to_f2(w[e >> 2], e & 3); x[e] = f.x; x[e + 1] = f.y; }
+    } else {
+        const signed char* p = reinterpret_cast<const signed char*>(rows + r * pitch + low);
+        x[0] = (float)p[lane]; x[1] = (float)p[lane + 32];
+    }
+}
+// offset of row r of a band from a 16-byte boundary (and what it grows by per row), modulo 16
+__device__ __forceinline__ int low_bits(const void* base, const Item& it, int esz) {
+    return (int)((reinterpret_cast<uintptr_t>(base) + (uintptr_t)(((int64_t)it.brow * it.C + it.col0) * esz)) & 15);
+}
+
+// Sums over a row's lanes of the NR row values a lane holds -> the band's row partials.  Halving butterfly: each step
+// exchanges half of the rows.
+template <int V>
+__device__ __forceinline__ void band_row_sums(const Item& it, float* rowpart, float* rs, int lane) {
+    int o = V == 8 ? 4 : 16;
+#pragma unroll
+    for (int h = Lane<V>::NR / 2; h >= 1; h >>= 1, o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int k = 0; k < h; ++k) {
+            const float send = up ? rs[k] : rs[k + h], keep = up ? rs[k + h] : rs[k];
+            rs[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    const float v = rs[0] + __shfl_xor_sync(0xffffffffu, rs[0], 1);
+    const int row = it.brow + (V == 8 ? (lane >> 3) + 4 * ((lane >> 1) & 3) : lane >> 1);
+    if ((lane & 1) == 0 && row < it.R) rowpart[(int64_t)it.tc * it.R + row] = v;
+}
+template <int V>
+__device__ __forceinline__ void tile_col_sums(const Item& it, float* colpart, float* acc, int lane) {
+    float* dst = colpart + (int64_t)it.tr * it.C + it.col0;
+    if constexpr (V == 8) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], 8);
+            acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], 16);
+        }
+        if (lane < 8 && it.col0 + 8 * lane < it.C) store_run<8, true>(dst, 8 * lane, 0, 8, acc);
+    } else {
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+            if (it.col0 + lane + 32 * e < it.C) dst[lane + 32 * e] = acc[e];
+    }
+}
+// Row factors 1 / sqrt(v_i / mean) times `mul` of a band: lane l < 16 has the one of row l (0 past the end).
+__device__ __forceinline__ float band_row_factor(const Item& it, const float* v, float mean, bool clamp, float mul, int lane) {
+    if (it.brow + (lane & 15) >= it.R) return 0.0f;
+    const float x = v[lane & 15];
+    float ratio = mean > 1e-30f && mean < 1e30f ? div_by(x, mean, 1.0f / mean) : x / mean;
+    if (clamp) ratio = fmaxf(ratio, 1e-30f);
+    return inv_sqrt(ratio) * mul;
+}
+// column factors of a lane (0 past the end: those columns then take no part in anything)
+template <int V>
+__device__ __forceinline__ void band_col_factors(const Item& it, const float* c, int lane, float* cf) {
+#pragma unroll
+    for (int e = 0; e < Lane<V>::E; ++e) {
+        const int col = Lane<V>::col(lane, e);
+        cf[e] = it.col0 + col < it.C ? c[col] : 0.0f;
+    }
+}
+
+// ---- S1 -------------------------------------------------------------------------------------------------------
+template <typename TG, int V>
+__device__ __forceinline__ void band_sq(const StepArgs& a, const Item& it, const char* st, int pitch, float* colacc) {
+    constexpr int NR = Lane<V>::NR, E = Lane<V>::E;
+    const CameTensorDesc& d = a.descs[it.tensor];
+    const int lane = threadIdx.x & 31, esz = size_of<TG>(d.g_dtype), dt = d.g_dtype;
+    const int low = low_bits(d.g, it, esz), grow = it.C * esz;
+    float rs[NR];
+    if (it.k == 0)
+#pragma unroll
+        for (int e = 0; e < E; ++e) colacc[e] = 0.0f;
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+        const int r = Lane<V>::row(lane, i);
+        float x[E];
+        read_row<V, TG>(st, pitch, dt, (low + r * grow) & 15, r, lane, x);
+        rs[i] = 0.0f;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const float y = it.col0 + Lane<V>::col(lane, e) < it.C ? x[e] : 0.0f;
+            rs[i] = fmaf(y, y, rs[i]);
+            colacc[e] = fmaf(y, y, colacc[e]);
+        }
+    }
+    const Scratch& s = a.scr[it.tensor];
+    float* colpart = s.colpart;
+    band_row_sums<V>(it, s.rowpart, rs, lane);
+    if (it.k == it.nb - 1) tile_col_sums<V>(it, colpart, colacc, lane);
+}
+
+// ---- S2 -------------------------------------------------------------------------------------------------------
+template <typename TG, typename S, int V>
+__device__ __forceinline__ void band_clip(const StepArgs& a, const Item& it, const char* st, float& acc, float& mean) {
+    constexpr int NR = Lane<V>::NR, E = Lane<V>::E;
+    const CameTensorDesc& d = a.descs[it.tensor];
+    const Scratch& s = a.scr[it.tensor];
+    const int lane = threadIdx.x & 31, esz = size_of<TG>(d.g_dtype), dt = d.g_dtype;
+    const int low = low_bits(d.g, it, esz), grow = it.C * esz;
+    if (it.k == 0) {
+        acc = 0.0f;
+        mean = read_mean(s.rowblk, s.nbR, it.R, d.flags & CAME_F_SQ_FIX, d.flags & CAME_F_SQ_CLAMP, lane);
+    }
+    const float f = band_row_factor(it, reinterpret_cast<const float*>(st + S::OFF_V), mean, d.flags & CAME_F_SQ_CLAMP, 1.0f, lane);
+    float cf[E];
+    band_col_factors<V>(it, reinterpret_cast<const float*>(st + S::OFF_C), lane, cf);
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+        const int r = Lane<V>::row(lane, i);
+        const float rf = __shfl_sync(0xffffffffu, f, r);
+        float x[E];
+        read_row<V, TG>(st, S::PA, dt, (low + r * grow) & 15, r, lane, x);
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const float u = (x[e] * rf) * cf[e];
+            acc = fmaf(u, u, acc);
+        }
+    }
+    if (s.fac && it.tc == 0 && lane < 16 && it.brow + lane < it.R) s.fac[it.brow + lane] = f;      // for the flat apply phase
+    if (it.k == it.nb - 1) leave_partial(s.spart, s.counters, it.tile, s.tiles_r * s.tiles_c, warp_sum(acc), lane);
+}
+// gradient scale / clip divisor, clip = max(1, sqrt(S/n)/clip_threshold) (came_kernels.cu:2619-2620)
+__device__ __forceinline__ float read_inv_clip(const Scratch& s, const CameHyper& h, int64_t n, int lane) {
+    const float gs = h.grad_scale, S = read_sum(s.spart, s.tiles_r * s.tiles_c, lane) * (gs * gs);
+    return gs / fmaxf(1.0f, sqrtf(S / (float)n) / h.clip_threshold);
+}
+
+// ---- M --------------------------------------------------------------------------------------------------------
+// u = g r c / clip, m = beta1 m + (1 - beta1) u, sums of (u - m)^2 (eps1 is added when the partials are finalised).
+// tile layout (came_kernels.cu:2584-2683): m re-quantised per 16 x 16 tile; fp32 (came_kernels.cu:2307-2342): m written;
+// flat layout: nothing written, the apply phase forms m again (came_kernels.cu:2246-2305 keeps it in fp32 scratch)
+template <typename TG, int MODE, int V>
+__device__ __forceinline__ void band_moment(const StepArgs& a, const CameHyper* hyp, const Item& it, const char* st, float* colacc, float& mean,
+                                            float& inv_clip) {
+    using S = Stage<TG, MODE>;
+    constexpr int NR = Lane<V>::NR, E = Lane<V>::E;
+    const CameTensorDesc& d = a.descs[it.tensor];
+    const Scratch& s = a.scr[it.tensor];
+    const int lane = threadIdx.x & 31, esz = size_of<TG>(d.g_dtype), dt = d.g_dtype, msz = MODE == CAME_MODE_FP32 ? 4 : 1;
+    const int low = low_bits(d.g, it, esz), grow = it.C * esz, mlow = low_bits(d.m, it, msz), mgrow = it.C * msz;
+    const float beta1 = hyp[d.group].beta1, om1 = hyp[d.group].om_beta1;
+    if (it.k == 0) {
+        mean = read_mean(s.rowblk, s.nbR, it.R, d.flags & CAME_F_SQ_FIX, d.flags & CAME_F_SQ_CLAMP, lane);
+        inv_clip = read_inv_clip(s, hyp[d.group], (int64_t)it.R * it.C, lane);
+    }
+    const float f = band_row_factor(it, reinterpret_cast<const float*>(st + S::OFF_V), mean, d.flags & CAME_F_SQ_CLAMP, 1.0f, lane);
+    const float* xs = reinterpret_cast<const float*>(st + S::OFF_X);
+    char* const m_base = reinterpret_cast<char*>(d.m);
+    float* const absmax = d.m_absmax;
+    float* const rowpart = s.rowpart;
+    float* const colpart = s.colpart;
+    float cf[E], m[NR][E], rs[NR], amax[V == 8 ? 1 : 2], sc[V == 8 ? 1 : 2];
+    bool in[E];
+    band_col_factors<V>(it, reinterpret_cast<const float*>(st + S::OFF_C), lane, cf);
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        in[e] = it.col0 + Lane<V>::col(lane, e) < it.C;
+        if (it.k == 0) colacc[e] = 0.0f;
+    }
+#pragma unroll
+    for (int q = 0; q < (V == 8 ? 1 : 2); ++q) {
+        amax[q] = 0.0f;
+        if (MODE == CAME_MODE_TILE8) {
+            const float A = in[q] ? xs[V == 8 ? (lane & 7) >> 1 : (lane >> 4) + 2 * q] : 0.0f;
+            sc[q] = A > 0.0f ? A / QMAX_I8 : 0.0f;
+        }
+    }
+    // (past the end of the matrix g is masked by its factors, m by a zero scale: u = m = 0, nothing enters the sums)
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+        const int r = Lane<V>::row(lane, i);
+        const float rf = __shfl_sync(0xffffffffu, f, r);
+        float x[E];
+        read_row<V, TG>(st, S::PA, dt, (low + r * grow) & 15, r, lane, x);
+        if constexpr (MODE == CAME_MODE_FP32) read_row<V, float>(st + S::OFF_M, S::PM, 0, (mlow + r * mgrow) & 15, r, lane, m[i]);
+        else read_codes<V>(st + S::OFF_M, S::PM, (mlow + r * mgrow) & 15, r, lane, m[i]);
+        float fs[2];
+        if (MODE == CAME_MODE_FLAT8) { fs[0] = xs[2 * r] / QMAX_I8; fs[1] = xs[2 * r + 1] / QMAX_I8; }
+        const uint32_t o8 = MODE == CAME_MODE_FLAT8 ? (uint32_t)(((uint32_t)(it.brow + r) * (uint32_t)it.C + (uint32_t)it.col0) & 255u) : 0u;
+        rs[i] = 0.0f;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const float u = ((x[e] * rf) * cf[e]) * inv_clip;
+            float mo = m[i][e];
+            if (MODE == CAME_MODE_TILE8) mo *= sc[V == 8 ? 0 : e & 1];
+            else if (MODE == CAME_MODE_FLAT8) mo *= !in[e] ? 0.0f : o8 + Lane<V>::col(lane, e) < 256u ? fs[0] : fs[1];
+            else if (!in[e]) mo = 0.0f;
+            const float mn = fmaf(mo, beta1, __fmul_rn(om1, u)), df = u - mn;      // the reference's order
+            rs[i] = fmaf(df, df, rs[i]);
+            colacc[e] = fmaf(df, df, colacc[e]);
+            m[i][e] = mn;
+            if (MODE == CAME_MODE_TILE8) amax[V == 8 ? 0 : e & 1] = fmaxf(amax[V == 8 ? 0 : e & 1], fabsf(mn));
+        }
+    }
+    const int64_t at = ((int64_t)it.brow * it.C + it.col0);
+    const int live = it.R - it.brow;
+    if (MODE == CAME_MODE_TILE8) {
+        float q127[V == 8 ? 1 : 2];
+        const int tile_cols = (it.C + TILE - 1) / TILE;
+#pragma unroll
+        for (int q = 0; q < (V == 8 ? 1 : 2); ++q) {
+            float A = amax[q];
+            if (V == 8) {
+                A = fmaxf(A, __shfl_xor_sync(0xffffffffu, A, 1));
+                A = fmaxf(A, __shfl_xor_sync(0xffffffffu, A, 8));
+                A = fmaxf(A, __shfl_xor_sync(0xffffffffu, A, 16));
+            } else {
+#pragma unroll
+                for (int o = 1; o < 16; o <<= 1) A = fmaxf(A, __shfl_xor_sync(0xffffffffu, A, o));
+            }
+            A = fix_absmax(A);
+            // one lane per tile: the one that holds its first row and column
+            if (in[q] && (V == 8 ? (lane & 0x19) == 0 : (lane & 15) == 0))
+                absmax[(int64_t)(it.brow >> 4) * tile_cols + (it.col0 >> 4) + (V == 8 ? (lane & 7) >> 1 : (lane >> 4) + 2 * q)] = A;
+            // 127 / A overflows below 4e-37: there m and A are first scaled by 2^64 (exact)
+            q127[q] = QMAX_I8 / A;
+            if (__any_sync(0xffffffffu, A < 4e-37f)) {
+                const float up = A < 4e-37f ? 18446744073709551616.0f : 1.0f;
+                q127[q] = QMAX_I8 / (A * up);
+#pragma unroll
+                for (int i = 0; i < NR; ++i)
+#pragma unroll
+                    for (int e = 0; e < E; ++e)
+                        if (V == 8 || e == q) m[i][e] *= up;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+            const int r = Lane<V>::row(lane, i);
+            int8_t* dst = reinterpret_cast<int8_t*>(m_base) + at + (int64_t)r * it.C + Lane<V>::col(lane, 0);
+            uint32_t y[E];      // the low byte of m * (127 / A) + 1.5 * 2^23 is the code (see fast_tile8.cu)
+#pragma unroll
+            for (int e = 0; e < E; ++e) y[e] = __float_as_uint(fmaf(m[i][e], q127[V == 8 ? 0 : e & 1], ROUND_MAGIC));
+            if constexpr (V == 8) {
+                if (r < live && in[0])
+                    *reinterpret_cast<uint2*>(dst) = make_uint2(__byte_perm(__byte_perm(y[0], y[1], 0x0040u), __byte_perm(y[2], y[3], 0x0040u), 0x5410u),
+                                                                __byte_perm(__byte_perm(y[4], y[5], 0x0040u), __byte_perm(y[6], y[7], 0x0040u), 0x5410u));
+            } else {
+                if (r < live && in[0]) dst[0] = (int8_t)y[0];
+                if (r < live && in[1]) dst[32] = (int8_t)y[1];
+            }
+        }
+    } else if (MODE == CAME_MODE_FP32) {
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+            const int r = Lane<V>::row(lane, i);
+            float* dst = reinterpret_cast<float*>(m_base) + at + (int64_t)r * it.C + Lane<V>::col(lane, 0);
+            if constexpr (V == 8) {
+                if (r < live && in[0]) store_run<8, true>(dst, 0, 0, 8, m[i]);
+            } else {
+                if (r < live && in[0]) dst[0] = m[i][0];
+                if (r < live && in[1]) dst[32] = m[i][1];
+            }
+        }
+    }
+    band_row_sums<V>(it, rowpart, rs, lane);
+    if (it.k == it.nb - 1) tile_col_sums<V>(it, colpart, colacc, lane);
+}
+
+// ---- A --------------------------------------------------------------------------------------------------------
+template <typename TP>
+__device__ __forceinline__ float g_apply_one(const Buf<TP>& b, float pv, float upd, const CameHyper& h, int wd) {
+    return apply_step(pv, upd, h.lr, h.wd_lr, h.decay_mul, wd, [&](float x) { return b.round(x); });
+}
+
+// p -= lr m R'_i C'_j with m read back from the state (came_kernels.cu:3332-3366, 2487-2511)
+template <typename TP, int MODE, int V>
+__device__ __forceinline__ void band_apply(const StepArgs& a, const CameHyper* hyp, const Item& it, const char* st, float& mean) {
+    using S = Stage<TP, MODE>;
+    constexpr int NR = Lane<V>::NR, E = Lane<V>::E;
+    const CameTensorDesc& d = a.descs[it.tensor];
+    const Scratch& s = a.scr[it.tensor];
+    const CameHyper h = hyp[d.group];      // (a copy: the stores below could alias the table)
+    const int lane = threadIdx.x & 31, esz = size_of<TP>(d.p_dtype), dt = d.p_dtype, msz = MODE == CAME_MODE_FP32 ? 4 : 1;
+    const int low = low_bits(d.p, it, esz), grow = it.C * esz, mlow = low_bits(d.m, it, msz), mgrow = it.C * msz;
+    const int wd = wd_form(h, d.flags);
+    if (it.k == 0) mean = read_mean(s.rowblk2, s.nbR, it.R, d.flags & CAME_F_RESROW_FIX, d.flags & CAME_F_RESROW_CLAMP, lane);
+    const float f = band_row_factor(it, reinterpret_cast<const float*>(st + S::OFF_V), mean, d.flags & CAME_F_RESROW_CLAMP, 1.0f, lane);
+    const float* xs = reinterpret_cast<const float*>(st + S::OFF_X);
+    float cf[E], sc[V == 8 ? 1 : 2];
+    bool in[E];
+    band_col_factors<V>(it, reinterpret_cast<const float*>(st + S::OFF_C), lane, cf);
+#pragma unroll
+    for (int e = 0; e < E; ++e) in[e] = it.col0 + Lane<V>::col(lane, e) < it.C;
+#pragma unroll
+    for (int q = 0; q < (V == 8 ? 1 : 2); ++q) {
+        sc[q] = 1.0f;
+        if (MODE == CAME_MODE_TILE8) {
+            const float A = in[q] ? xs[V == 8 ? (lane & 7) >> 1 : (lane >> 4) + 2 * q] : 0.0f;
+            sc[q] = A > 0.0f ? A / QMAX_I8 : 0.0f;
+        }
+    }
+    const Buf<TP> p(d.p, dt);
+    const int64_t at = (int64_t)it.brow * it.C + it.col0 + Lane<V>::col(lane, 0);
+    const int live = it.R - it.brow, n_push = a.n_push;
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+        const int r = Lane<V>::row(lane, i);
+        const float rf = __shfl_sync(0xffffffffu, f, r);
+        float x[E], m[E];
+        read_row<V, TP>(st, S::PA, dt, (low + r * grow) & 15, r, lane, x);
+        if constexpr (MODE == CAME_MODE_FP32) read_row<V, float>(st + S::OFF_M, S::PM, 0, (mlow + r * mgrow) & 15, r, lane, m);
+        else read_codes<V>(st + S::OFF_M, S::PM, (mlow + r * mgrow) & 15, r, lane, m);
+#pragma unroll
+        for (int e = 0; e < E; ++e) x[e] = g_apply_one(p, x[e], (m[e] * (rf * sc[V == 8 ? 0 : e & 1])) * cf[e], h, wd);
+        const int64_t o = at + (int64_t)r * it.C;
+        if (r < live) {
+            if constexpr (V == 8) {
+                if (in[0]) p.put8(o, x);
+                if (n_push && in[0])
+                    for (int q = 0; q < n_push; ++q) p.put8(o, x, a.push_delta[q]);
+            } else {
+                if (in[0]) p.put(o, x[0]);
+                if (in[1]) p.put(o + 32, x[1]);
+                if (n_push)
+                    for (int q = 0; q < n_push; ++q) {
+                        if (in[0]) p.put(o, x[0], a.push_delta[q]);
+                        if (in[1]) p.put(o + 32, x[1], a.push_delta[q]);
+                    }
+            }
+        }
+    }
+}
+
+// flat layout: a warp owns a block of 256 consecutive elements, whatever rows they belong to (the un-quantised momentum
+// feeds the update: came_kernels.cu:2246-2305, 2487-2511)
+template <typename TG, typename TP, int V>
+__device__ __forceinline__ void phase_apply_flat(const StepArgs& a, const CameHyper* hyp, const Work& w) {
+    const CameTensorDesc d = a.descs[w.tensor];
+    const Scratch s = a.scr[w.tensor];
+    const CameHyper h = hyp[d.group];
+    const Buf<TG> g(d.g, d.g_dtype);
+    const Buf<TP> p(d.p, d.p_dtype);
+    const int lane = threadIdx.x & 31, C = (int)d.cols, blk = w.tile;
+    const int64_t n = d.rows * d.cols;
+    const int wd = wd_form(h, d.flags);
+    const float inv_clip = read_inv_clip(s, h, n, lane);
+    const float mean = read_mean(s.rowblk2, s.nbR, (int)d.rows, d.flags & CAME_F_RESROW_FIX, d.flags & CAME_F_RESROW_CLAMP, lane), inv = 1.0f / mean;
+    const bool clamp = d.flags & CAME_F_RESROW_CLAMP, easy = mean > 1e-30f && mean < 1e30f;
+    int8_t* mq = reinterpret_cast<int8_t*>(d.m);
+    constexpr int STEP = V == 8 ? 1 : 32;      // distance between a lane's elements
+    const int64_t i0 = (int64_t)blk * QBLOCK + (V == 8 ? 8 * lane : lane);
+    float x[8], m[8], pv[8];
+    int cnt;      // elements of this lane (they end where the tensor does)
+    if (V == 8) {
+        cnt = i0 >= n ? 0 : 8;      // n is a multiple of 8
+        if (cnt) {
+            g.get8(i0, x);
+            p.get8(i0, pv);
+            const uint2 r = *reinterpret_cast<const uint2*>(mq + i0);
+            const uint32_t y[2] = {r.x ^ 0x80808080u, r.y ^ 0x80808080u};
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) { const u64 f = codes_to_f2(y[e >> 2], e & 3); m[e] = f.x; m[e + 1] = f.y; }
+        }
+    } else {
+        cnt = i0 >= n ? 0 : (int)min((int64_t)8, (n - i0 + 31) >> 5);
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (e < cnt) { x[e] = g.get(i0 + 32 * e); pv[e] = p.get(i0 + 32 * e); m[e] = (float)mq[i0 + 32 * e]; }
+    }
+    const float sc = __ldcg(d.m_absmax + blk) / QMAX_I8;
+    int row, col;
+    if (n < 0x7fffffff) { row = (int)((uint32_t)i0 / (uint32_t)C); col = (int)i0 - row * C; }
+    else { row = (int)(i0 / C); col = (int)(i0 - (int64_t)row * C); }
+    float upd[8], amax = 0.0f, r = 0.0f, rr = 0.0f;
+    int have = -1;      // row the factors r, rr belong to
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        upd[e] = 0.0f;
+        if (e >= cnt) m[e] = 0.0f;
+        if (e < cnt) {
+            if (row != have) {
+                have = row;
+                r = __ldcg(s.fac + row);
+                const float y = __ldcg(s.Rr + row);
+                float ratio = easy ? div_by(y, mean, inv) : y / mean;
+                if (clamp) ratio = fmaxf(ratio, 1e-30f);
+                rr = inv_sqrt(ratio);
+            }
+            const float u = ((x[e] * r) * __ldcg(s.vc + col)) * inv_clip;
+            m[e] = fmaf(m[e] * sc, h.beta1, __fmul_rn(h.om_beta1, u));
+            amax = fmaxf(amax, fabsf(m[e]));
+            upd[e] = (m[e] * rr) * __ldcg(s.Rc + col);
+            col += STEP;
+            while (col >= C) { col -= C; ++row; }
+        }
+    }
+    const float A = fix_absmax(warp_max(amax)), scale = quant_scale<true>(A);
+    if (lane == 0) d.m_absmax[blk] = A;      // (every lane has read the old value: the reduction is behind them)
+    const uint32_t lo = quant_pack4<true>(make_float4(m[0], m[1], m[2], m[3]), A, scale);
+    const uint32_t hi = quant_pack4<true>(make_float4(m[4], m[5], m[6], m[7]), A, scale);
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+        if (e < cnt) pv[e] = g_apply_one(p, pv[e], upd[e], h, wd);
+    if (V == 8) {
+        if (cnt) {
+            *reinterpret_cast<uint2*>(mq + i0) = make_uint2(lo, hi);
+            p.put8(i0, pv);
+            for (int k = 0; k < a.n_push; ++k) p.put8(i0, pv, a.push_delta[k]);
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (e < cnt) {
+                mq[i0 + 32 * e] = (int8_t)((e < 4 ? lo : hi) >> (8 * (e & 3)));
+                p.put(i0 + 32 * e, pv[e]);
+                for (int k = 0; k < a.n_push; ++k) p.put(i0 + 32 * e, pv[e], a.push_delta[k]);
+            }
+    }
+}
+
+// ---- F1 / F2 ------------------------------------------------------------------------------------------------------
+// One block of 256 entries of a row or column vector, by a CTA: partials -> EMA with the dequantised old state ->
+// requantised state, fresh fp32 row values / column factors, the sum of a row block
+// (came_kernels.cu:77-93, 215-242, 298-333, 2685-2706, 2742-2779).  Warp w adds the partials w, w + 8, ... of all 256
+// entries, then thread t has entry t: one entry per thread keeps the code short, and cold code is what takes the time
+// (8 entries per lane of one warp: 5 us a block, like this 2 us).
+template <bool RES>
+__device__ __forceinline__ void phase_finalize(const StepArgs& a, const CameHyper* hyp, const Work& w, GShared& sh) {
+    const CameTensorDesc& d = a.descs[w.tensor];
+    const Scratch& s = a.scr[w.tensor];
+    const CameHyper& h = hyp[d.group];
+    const int R = (int)d.rows, C = (int)d.cols, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool is_col = w.tile >= s.nbR, quant = d.mode != CAME_MODE_FP32;
+    const int b = is_col ? w.tile - s.nbR : w.tile, n = is_col ? C : R, idx = b * QBLOCK + threadIdx.x;
+    const int parts = is_col ? s.tiles_r : s.tiles_c;
+    const float* part = (is_col ? s.colpart : s.rowpart) + b * QBLOCK + lane;
+    void* state = RES ? (is_col ? d.res_col : d.res_row) : (is_col ? d.sq_col : d.sq_row);
+    float* absmax = RES ? (is_col ? d.res_col_absmax : d.res_row_absmax) : (is_col ? d.sq_col_absmax : d.sq_row_absmax);
+    float old = 0.0f;
+    if (idx < n) old = quant ? (float)reinterpret_cast<const uint8_t*>(state)[idx] * (absmax[b] / QMAX_U8) : reinterpret_cast<const float*>(state)[idx];
+    const int left = n - b * QBLOCK - lane;
+    float acc[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[e] = 0.0f;
+#pragma unroll 2
+    for (int t = warp; t < parts; t += G_WARPS)
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (32 * e < left) acc[e] += __ldcg(part + (int64_t)t * n + 32 * e);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) sh.col[warp][32 * e + lane] = acc[e];
+    __syncthreads();
+    float v = 0.0f, sum = 0.0f;
+#pragma unroll
+    for (int k = 0; k < G_WARPS; ++k) sum += sh.col[k][threadIdx.x];
+    if (idx < n) {
+        if (!RES) sum *= h.grad_scale * h.grad_scale;
+        v = ema_update(old, RES ? h.beta3 : h.beta2, RES ? h.om_beta3 : h.om_beta2, mean_plus_eps(sum, (float)(is_col ? R : C), RES ? h.eps1 : h.eps0));
+        const bool clamp = d.flags & (RES ? CAME_F_RESCOL_CLAMP : CAME_F_SQ_CLAMP);
+        if (is_col) (RES ? s.Rc : s.vc)[idx] = inv_sqrt(clamp ? fmaxf(v, 1e-30f) : v);
+        else (RES ? s.Rr : s.vr)[idx] = v;
+    }
+    if (quant) {
+        const float bmax = fix_absmax(block_max(v, sh.red));      // syncs: every old absmax read is done
+        if (threadIdx.x == 0) absmax[b] = bmax;
+        if (idx < n) reinterpret_cast<uint8_t*>(state)[idx] = (uint8_t)quant_u8_div(v, bmax);
+    } else if (idx < n) {
+        reinterpret_cast<float*>(state)[idx] = v;
+    }
+    if (!is_col) {
+        float* blk = RES ? s.rowblk2 : s.rowblk;
+        const float bs = block_sum(v, sh.red);
+        if (threadIdx.x == 0) blk[b] = bs;
+    }
+    __syncthreads();      // (the shared arrays are free for the next item)
+}
+
+// ---- 1-D tensors --------------------------------------------------------------------------------------------------
+// (reference: kCameNonfactoredSqUpdateAndQuant[TypedUpdate] came_kernels.cu:1013-1122,
+// kCameNonfactoredExpAvgParamUpdate[TypedUpdate] came_kernels.cu:1489-1601; CAMECUDA.py:247-273; no confidence term,
+// CAME.py:163-164).  A CTA owns a block of 256 elements.
+template <typename TG>
+__device__ __forceinline__ void vector_element(const CameTensorDesc& d, const CameHyper& h, int b, int64_t idx, float& v, float& u) {
+    v = 0.0f; u = 0.0f;
+    if (idx >= d.rows) return;
+    const float g = Buf<TG>(d.g, d.g_dtype).get(idx) * h.grad_scale;
+    const float old = d.mode != CAME_MODE_FP32 ? (float)reinterpret_cast<const uint8_t*>(d.sq_row)[idx] * (d.sq_row_absmax[b] / QMAX_U8)
+                                               : reinterpret_cast<const float*>(d.sq_row)[idx];
+    v = nf_second_moment(old, g, h);
+    u = nf_update(v, g, d.flags);
+}
+constexpr int VECTOR_DIRECT = 512;      // block partials that every reader adds by itself (beyond: the last block does)
+template <typename TG>
+__device__ __forceinline__ void phase_vector_sq(const StepArgs& a, const CameHyper* hyp, const Work& w, GShared& sh) {
+    const CameTensorDesc& d = a.descs[w.tensor];
+    const Scratch& s = a.scr[w.tensor];
+    float v, u;
+    vector_element<TG>(d, hyp[d.group], w.tile, (int64_t)w.tile * QBLOCK + threadIdx.x, v, u);
+    const float t = block_sum(u * u, sh.red);
+    if (threadIdx.x == 0) s.spart[w.tile] = t;
+    if (s.nbR > VECTOR_DIRECT && last_cta(s.counters, s.nbR, sh)) {
+        const float S = block_vector_sum_cg(s.spart, s.nbR, sh.red);
+        if (threadIdx.x == 0) s.scal[0] = S;
+    }
+    __syncthreads();
+}
+template <typename TG, typename TP>
+__device__ __forceinline__ void phase_vector_apply(const StepArgs& a, const CameHyper* hyp, const Work& w, GShared& sh) {
+    const CameTensorDesc& d = a.descs[w.tensor];
+    const CameHyper& h = hyp[d.group];
+    const int b = w.tile;
+    const int64_t idx = (int64_t)b * QBLOCK + threadIdx.x;
+    const bool in = idx < d.rows, quant = d.mode != CAME_MODE_FP32;
+    const Buf<TP> p(d.p, d.p_dtype);
+    float v, u, m = 0.0f;
+    vector_element<TG>(d, h, b, idx, v, u);
+    if (in) m = quant ? (float)reinterpret_cast<const int8_t*>(d.m)[idx] * (d.m_absmax[b] / QMAX_I8) : reinterpret_cast<const float*>(d.m)[idx];
+    const float pv = in ? p.get(idx) : 0.0f;
+    const Scratch& s = a.scr[w.tensor];
+    const float S = s.nbR > VECTOR_DIRECT ? __ldcg(s.scal) : block_vector_sum_cg(s.spart, s.nbR, sh.red);
+    const float clip = nf_clip(S, d.rows, h);
+    m = in ? nf_momentum(m, u, clip, 1.0f / clip, d.flags, h) : 0.0f;
+    if (in) p.put(idx, g_apply_one(p, pv, m, h, wd_form(h, d.flags)));
+    if (quant) {
+        const float vmax = fix_absmax(block_max(v, sh.red)), mmax = fix_absmax(block_max(fabsf(m), sh.red));      // (syncs)
+        if (threadIdx.x == 0) { d.sq_row_absmax[b] = vmax; d.m_absmax[b] = mmax; }
+        if (in) {
+            reinterpret_cast<uint8_t*>(d.sq_row)[idx] = (uint8_t)quant_u8_div(v, vmax);
+            reinterpret_cast<int8_t*>(d.m)[idx] = (int8_t)quant_i8_div(m, mmax);
+        }
+    } else if (in) {
+        reinterpret_cast<float*>(d.sq_row)[idx] = v;
+        reinterpret_cast<float*>(d.m)[idx] = m;
+    }
+}
+
+// ---- the kernel ---------------------------------------------------------------------------------------------------
+struct GenericArgs {
+    StepArgs a;
+    GenericLists l;
+    int n_hyp;                        // records in `hyp`: the step's hyper-parameters; 0: a.hyp holds them
+    CameHyper hyp[GENERIC_MAX_HYP];
+};
+
+template <typename TG, typename TP, int MODE>
+__global__ void __launch_bounds__(THREADS, 3) k_step_generic(const __grid_constant__ GenericArgs ga) {
+    using S = Stage<TG, MODE>;
+    extern __shared__ __align__(128) char g_smem[];
+    __shared__ GShared sh;
+    const StepArgs& a = ga.a;
+    const GenericLists& l = ga.l;
+    const CameHyper* hyp = ga.n_hyp ? ga.hyp : a.hyp;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    char* const stages = g_smem + warp * (S::COUNT * S::BYTES);
+    auto stage = [&](int k) { return stages + k * S::BYTES; };
+    // warp items: across the SMs first, then over the warps; CTA items of 1-D tensors: from the last CTA on, which comes
+    // last in the deal of the others
+    const int first = warp * gridDim.x + blockIdx.x, stride = G_WARPS * gridDim.x, back = gridDim.x - 1 - blockIdx.x;
+    float colacc[8];
+
+    for (int i = back; i < l.n_ones; i += gridDim.x) phase_vector_sq<TG>(a, hyp, l.ones[i], sh);
+    stream<S::COUNT>(a, l.tiles, l.n_tiles, first, stride,
+        [&](const Item& it, int k) {
+            const CameTensorDesc& d = a.descs[it.tensor];
+            stage_rows(stage(k), S::PA, d.g, size_of<TG>(d.g_dtype), it, lane);
+        },
+        [&](const Item& it, int k) {
+            if (it.v8) band_sq<TG, 8>(a, it, stage(k), S::PA, colacc);
+            else band_sq<TG, 1>(a, it, stage(k), S::PA, colacc);
+        });
+    if (!grid_barrier(l.bar, a.status)) return;
+
+    for (int i = back; i < l.n_ones; i += gridDim.x) phase_vector_apply<TG, TP>(a, hyp, l.ones[i], sh);
+    if (l.n_tiles == 0) return;
+    for (int i = blockIdx.x; i < l.n_vecs; i += gridDim.x) phase_finalize<false>(a, hyp, l.vecs[i], sh);
+    if (!grid_barrier(l.bar, a.status)) return;
+
+    float acc = 0.0f, mean = 1.0f, inv_clip = 1.0f;      // of the item in work
+    stream<S::COUNT>(a, l.tiles, l.n_tiles, first, stride,
+        [&](const Item& it, int k) {
+            const CameTensorDesc& d = a.descs[it.tensor];
+            const Scratch& s = a.scr[it.tensor];
+            stage_vectors(stage(k), S::OFF_V, S::OFF_C, s.vr, s.vc, it, lane);
+            stage_rows(stage(k), S::PA, d.g, size_of<TG>(d.g_dtype), it, lane);
+        },
+        [&](const Item& it, int k) {
+            if (it.v8) band_clip<TG, S, 8>(a, it, stage(k), acc, mean);
+            else band_clip<TG, S, 1>(a, it, stage(k), acc, mean);
+        });
+    if (!grid_barrier(l.bar, a.status)) return;
+
+    stream<S::COUNT>(a, l.tiles, l.n_tiles, first, stride,
+        [&](const Item& it, int k) {
+            const CameTensorDesc& d = a.descs[it.tensor];
+            const Scratch& s = a.scr[it.tensor];
+            stage_vectors(stage(k), S::OFF_V, S::OFF_C, s.vr, s.vc, it, lane);
+            stage_absmax<MODE>(stage(k) + S::OFF_X, d.m_absmax, it, lane);
+            stage_rows(stage(k), S::PA, d.g, size_of<TG>(d.g_dtype), it, lane);
+            stage_rows(stage(k) + S::OFF_M, S::PM, d.m, MODE == CAME_MODE_FP32 ? 4 : 1, it, lane);
+        },
+        [&](const Item& it, int k) {
+            if (it.v8) band_moment<TG, MODE, 8>(a, hyp, it, stage(k), colacc, mean, inv_clip);
+            else band_moment<TG, MODE, 1>(a, hyp, it, stage(k), colacc, mean, inv_clip);
+        });
+    if (!grid_barrier(l.bar, a.status)) return;
+
+    for (int i = blockIdx.x; i < l.n_vecs; i += gridDim.x) phase_finalize<true>(a, hyp, l.vecs[i], sh);
+    if (!grid_barrier(l.bar, a.status)) return;
+
+    if constexpr (MODE == CAME_MODE_FLAT8) {
+        for (int i = first; i < l.n_flats; i += stride) {
+            const Work w = l.flats[i];
+            if (a.scr[w.tensor].g_v == 8) phase_apply_flat<TG, TP, 8>(a, hyp, w);
+            else phase_apply_flat<TG, TP, 1>(a, hyp, w);
+        }
+    } else {
+        stream<S::COUNT>(a, l.tiles, l.n_tiles, first, stride,
+            [&](const Item& it, int k) {
+                const CameTensorDesc& d = a.descs[it.tensor];
+                const Scratch& s = a.scr[it.tensor];
+                stage_vectors(stage(k), S::OFF_V, S::OFF_C, s.Rr, s.Rc, it, lane);
+                stage_absmax<MODE>(stage(k) + S::OFF_X, d.m_absmax, it, lane);
+                stage_rows(stage(k), S::PA, d.p, size_of<TP>(d.p_dtype), it, lane);
+                stage_rows(stage(k) + S::OFF_M, S::PM, d.m, MODE == CAME_MODE_FP32 ? 4 : 1, it, lane);
+            },
+            [&](const Item& it, int k) {
+                if (it.v8) band_apply<TP, MODE, 8>(a, hyp, it, stage(k), mean);
+                else band_apply<TP, MODE, 1>(a, hyp, it, stage(k), mean);
+            });
+    }
+}
+
+struct GenericKernel {
+    void (*fn)(const GenericArgs);
+    int smem;
+};
+template <typename TG, typename TP, int MODE> GenericKernel generic_kernel() {
+    return {k_step_generic<TG, TP, MODE>, G_WARPS * Stage<TG, MODE>::COUNT * Stage<TG, MODE>::BYTES};
+}
+template <typename TG, typename TP> GenericKernel pick_mode(int mode) {
+    switch (mode) {
+        case CAME_MODE_FP32: return generic_kernel<TG, TP, CAME_MODE_FP32>();
+        case CAME_MODE_TILE8: return generic_kernel<TG, TP, CAME_MODE_TILE8>();
+        default: return generic_kernel<TG, TP, CAME_MODE_FLAT8>();
+    }
+}
+GenericKernel pick_generic(int g, int p, int mode) {
+    if (g != p) return pick_mode<Any, Any>(mode);
+    if (g == CAME_DT_F32) return pick_mode<float, float>(mode);
+    if (g == CAME_DT_F16) return pick_mode<__half, __half>(mode);
+    return pick_mode<__nv_bfloat16, __nv_bfloat16>(mode);
+}
+
+}  // namespace
+
+int generic_tile_cols() { return G_CW; }
+
+cudaError_t launch_generic(const KernelKey& key, const StepArgs& a, const CameHyper* host_hyp, int n_hyp, const GenericLists& l,
+                           cudaStream_t st) {
+    const GenericKernel kernel = pick_generic(key.g_dtype, key.p_dtype, key.mode);
+    const void* fn = reinterpret_cast<const void*>(kernel.fn);
+    static std::mutex mu;
+    static std::map<std::pair<int, const void*>, int> cache;      // CTAs an SM holds, per device and kernel
+    int dev = 0, per_sm = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        auto it = cache.find({dev, fn});
+        if (it == cache.end()) {
+            e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kernel.smem);
+            if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, THREADS, kernel.smem);
+            if (e != cudaSuccess) return e;
+            cache[{dev, fn}] = per_sm;
+        } else {
+            per_sm = it->second;
+        }
+    }
+    const int most = std::max({l.n_tiles + l.n_ones, l.n_vecs + l.n_ones, l.n_flats});
+    const int grid = std::min(most, std::max(1, per_sm) * persistent_grid_limit());
+    GenericArgs ga{};
+    ga.a = a;
+    ga.l = l;
+    if (host_hyp && n_hyp <= GENERIC_MAX_HYP) {
+        ga.n_hyp = n_hyp;
+        for (int i = 0; i < n_hyp; ++i) ga.hyp[i] = host_hyp[i];
+    }
+    void* params[] = {&ga};
+    return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(THREADS), params, (size_t)kernel.smem, st);
+}
+
+}  // namespace came

@@ -27,7 +27,7 @@ struct KernelKey {
     int g_dtype;
     int p_dtype;
     int mode;
-    int variant;   // 0: scalar loads, any shape; 1: 16-byte vector loads; 2: shared-memory staged fast path
+    int variant;   // 1: 16-byte vector loads; 2: shared-memory staged path (N-D tensors: small matrices)
 };
 
 enum KernelId {
@@ -38,9 +38,9 @@ enum KernelId {
     KID_MOMENT,
     KID_RES_FINALIZE,
     KID_APPLY,
-    KID_FACTORS,
+    KID_FACTORS,           // (part of KID_GENERIC)
     KID_APPLY_FLAT,
-    KID_NF_PARTIAL,
+    KID_NF_PARTIAL,        // (1-D tensors: part of KID_GENERIC; the numbers of the others stay)
     KID_NF_APPLY,
     KID_NF_REDUCE,
     KID_ND_SQ,             // tensors of more than two dimensions (nd.cu)
@@ -51,6 +51,7 @@ enum KernelId {
     KID_ND_RESMEAN,
     KID_ND_APPLY,
     KID_MOMENT_APPLY,      // momentum + residual finalize + apply of the tile layout as one kernel (fused_ma.cu)
+    KID_GENERIC,           // whole step of small sets, odd shapes and 1-D tensors (generic.cu)
     KID_COUNT
 };
 
@@ -75,8 +76,20 @@ int persistent_grid_limit();
 constexpr int S_FIN_CHUNK = 2048;      // factor-vector entries one CTA of the clip finalize writes
 void fused_sq_geometry(int64_t cols, int elem_bytes, int* groups, int* ng, int* rb, int* slot_kb);
 bool fused_sq_eligible(int64_t cols, int elem_bytes);
-cudaError_t launch_nonfactored(int kernel, const KernelKey& key, const StepArgs& a, const Work* work, int n,
-                               cudaStream_t st);
+// whole-step kernel (generic.cu): its work lists and the two words of its grid barrier (zero before the first launch)
+struct GenericLists {
+    const Work* tiles;      // matrix tiles
+    const Work* vecs;       // blocks of 256 entries of the row, then the column vector
+    const Work* flats;      // flat layout: blocks of 256 elements
+    const Work* ones;       // 1-D tensors: blocks of 256 elements
+    int n_tiles, n_vecs, n_flats, n_ones;
+    int* bar;
+};
+constexpr int GENERIC_MAX_HYP = 8;      // hyper-parameter records that travel as kernel arguments
+int generic_tile_cols();                 // columns of a warp's item
+// host_hyp: the records of this step (null: they are in a.hyp, uploaded by the caller)
+cudaError_t launch_generic(const KernelKey& key, const StepArgs& a, const CameHyper* host_hyp, int n_hyp, const GenericLists& l,
+                           cudaStream_t st);
 
 cudaError_t launch_nd(int kernel, const KernelKey& key, const StepArgs& a, const Work* work, int n, cudaStream_t st);
 // tensors of more than two dimensions made of small matrices: matrices of a chunk (0: other kernels), launch key

@@ -253,13 +253,8 @@ __global__ void __launch_bounds__(THREADS) k_nd_apply(StepArgs a, const Work* __
         const float rr = row_factor(s.Rr[b * sh.R + i], s.rowblk2[b], d.flags & CAME_F_RESROW_CLAMP);
         const float rc = col_factor(s.Rc[b * sh.C + j], d.flags & CAME_F_RESCOL_CLAMP);
         const float upd = (m * rr) * rc;
-        float pv = nd_load(d.p, d.p_dtype, f);
-        if (h.weight_decay != 0.0f) {
-            if (d.flags & CAME_F_WD_MUL2) pv = nd_round(pv * h.decay_mul, d.p_dtype);
-            else if (d.flags & CAME_F_WD_ADD2) pv = nd_round(pv - h.wd_lr * pv, d.p_dtype);
-            else pv = pv - h.wd_lr * pv;
-        }
-        nd_store(d.p, d.p_dtype, f, pv - h.lr * upd);
+        nd_store(d.p, d.p_dtype, f, apply_step(nd_load(d.p, d.p_dtype, f), upd, h.lr, h.wd_lr, h.decay_mul, wd_form(h, d.flags),
+                                               [&](float x) { return nd_round(x, d.p_dtype); }));
     }
     if (d.mode == CAME_MODE_FP32) {
         if (valid) reinterpret_cast<float*>(d.m)[f] = m;
@@ -525,7 +520,7 @@ __global__ void __launch_bounds__(THREADS) k_nds_step(StepArgs a, const Work* __
     const uint32_t flags = d.flags;
     const NdsChunk k = nds_chunk<R0, C0>(d, s, w.tile, nds_smem);
     const bool quant = d.mode != CAME_MODE_FP32;
-    const int ne = k.nm * k.RC, nr = k.nm * k.R, nc = k.nm * k.C, lane = threadIdx.x & 31;
+    const int ne = k.nm * k.RC, nr = k.nm * k.R, nc = k.nm * k.C, lane = threadIdx.x & 31, wd = wd_form(h, flags);
     const float inv_clip = 1.0f / s.scal[1];
     nds_stage<R0>(d.g, d.g_dtype, k.e0, ne, h.grad_scale, k.el);
     if (quant) nds_stage_codes<R0, true>(d.m, d.m_absmax, k.e0, ne, k.m);
@@ -589,15 +584,8 @@ __global__ void __launch_bounds__(THREADS) k_nds_step(StepArgs a, const Work* __
             const float upd[4] = {u4.x, u4.y, u4.z, u4.w}, mv[4] = {m[t].x, m[t].y, m[t].z, m[t].w};
             const uint32_t codes = quant ? quant_pack4<true>(m[t], A, sc) : 0u;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                float x = pv[t][e];
-                if (h.weight_decay != 0.0f) {
-                    if (flags & CAME_F_WD_MUL2) x = nd_round(x * h.decay_mul, d.p_dtype);
-                    else if (flags & CAME_F_WD_ADD2) x = nd_round(x - h.wd_lr * x, d.p_dtype);
-                    else x = x - h.wd_lr * x;
-                }
-                pv[t][e] = x - h.lr * upd[e];
-            }
+            for (int e = 0; e < 4; ++e)
+                pv[t][e] = apply_step(pv[t][e], upd[e], h.lr, h.wd_lr, h.decay_mul, wd, [&](float x) { return nd_round(x, d.p_dtype); });
             if (vec && i + 4 <= ne) {
                 nd_store4(d.p, d.p_dtype, f, pv[t]);
                 if (quant) *reinterpret_cast<uint32_t*>(reinterpret_cast<int8_t*>(d.m) + f) = codes;

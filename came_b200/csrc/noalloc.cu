@@ -63,25 +63,22 @@ __device__ __forceinline__ void store_any(void* base, int dtype, int64_t i, floa
     else reinterpret_cast<__nv_bfloat16*>(base)[i] = __float2bfloat16_rn(x);
 }
 
-// v = beta2 v + (1-beta2)(g^2 + eps0), u = g / sqrt(v)   (came_kernels.cu:1035-1042)
-__device__ __forceinline__ void noalloc_second_moment(const NoallocArgs& a, int b, int64_t idx, bool valid, float& g,
-                                                      float& v, float& u) {
-    g = 0.0f; v = 0.0f; u = 0.0f;
+__device__ __forceinline__ void noalloc_second_moment(const NoallocArgs& a, int b, int64_t idx, bool valid, float& v, float& u) {
+    v = 0.0f; u = 0.0f;
     if (!valid) return;
-    g = load_any(a.g, a.g_dtype, idx) * a.h.grad_scale;
+    const float g = load_any(a.g, a.g_dtype, idx) * a.h.grad_scale;
     const float old = a.quant ? (float)reinterpret_cast<const uint8_t*>(a.v)[idx] * (a.v_absmax[b] / QMAX_U8)
                               : reinterpret_cast<const float*>(a.v)[idx];
-    v = old * a.h.beta2 + a.h.om_beta2 * fmaf(g, g, a.h.eps0);
-    const float vv = (a.flags & CAME_F_RSQRT_CLAMP) ? fmaxf(v, 1e-30f) : v;
-    u = (1.0f / sqrtf(vv)) * g;
+    v = nf_second_moment(old, g, a.h);
+    u = nf_update(v, g, a.flags);
 }
 
 __global__ void __launch_bounds__(THREADS) k_noalloc_partial(NoallocArgs a) {
     __shared__ float red[33];
     const int b = blockIdx.x;
     const int64_t idx = (int64_t)b * QBLOCK + threadIdx.x;
-    float g, v, u;
-    noalloc_second_moment(a, b, idx, idx < a.n, g, v, u);
+    float v, u;
+    noalloc_second_moment(a, b, idx, idx < a.n, v, u);
     const float t = block_sum(u * u, red);
     if (threadIdx.x == 0) a.partials[b] = t;      // every entry the second kernel reads is written here first
 }
@@ -99,25 +96,18 @@ __global__ void __launch_bounds__(THREADS) k_noalloc_apply(NoallocArgs a, int nb
     const int64_t idx = (int64_t)b * QBLOCK + threadIdx.x;
     const bool valid = idx < a.n;
     const float S = a.partials[NOALLOC_MAX_BLOCKS];
-    const float clip = fmaxf(1.0f, sqrtf(S / (float)a.n) / a.h.clip_threshold);
-    float g, v, u;
-    noalloc_second_moment(a, b, idx, valid, g, v, u);
-    if (a.flags & CAME_F_UPDATE_F16) u = __half2float(__float2half_rn(u));
-    u = u / clip;
+    const float clip = nf_clip(S, a.n, a.h);
+    float v, u;
+    noalloc_second_moment(a, b, idx, valid, v, u);
     float m_old = 0.0f;
     if (valid)
         m_old = a.quant ? (float)reinterpret_cast<const int8_t*>(a.m)[idx] * (a.m_absmax[b] / QMAX_I8)
                         : reinterpret_cast<const float*>(a.m)[idx];
-    const float m = m_old * a.h.beta1 + a.h.om_beta1 * u;
-    if (valid) {
-        float pv = load_any(a.p, a.p_dtype, idx);
-        if (a.h.weight_decay != 0.0f) {
-            if (a.flags & CAME_F_WD_MUL2) pv = round_any(pv * a.h.decay_mul, a.p_dtype);
-            else if (a.flags & CAME_F_WD_ADD2) pv = round_any(pv - a.h.wd_lr * pv, a.p_dtype);
-            else pv = pv - a.h.wd_lr * pv;
-        }
-        store_any(a.p, a.p_dtype, idx, pv - a.h.lr * m);
-    }
+    const float m = nf_momentum(m_old, u, clip, 1.0f / clip, a.flags, a.h);
+    if (valid)
+        store_any(a.p, a.p_dtype, idx, apply_step(load_any(a.p, a.p_dtype, idx), m, a.h.lr, a.h.wd_lr, a.h.decay_mul,
+                                                  wd_form(a.h, a.flags),
+                                                  [&](float x) { return round_any(x, a.p_dtype); }));
     if (a.quant) {
         const float vmax = fix_absmax(block_max(valid ? v : 0.0f, red));
         const float mmax = fix_absmax(block_max(valid ? fabsf(m) : 0.0f, red));
