@@ -1,4 +1,5 @@
-"""Builds libcame_b200.so in-tree with nvcc for sm_100a (no JIT cache, no torch extension machinery).
+"""Builds libcame_b200.so in-tree with nvcc for sm_100a, and the host module _host.so (g++, against torch's headers) that
+links to it.  No JIT cache.
 
     python came_b200/_build.py [--force] [--verbose]
 """
@@ -8,6 +9,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 PKG = os.path.dirname(os.path.abspath(__file__))
@@ -16,6 +18,7 @@ CSRC = os.path.join(PKG, "csrc")
 INCLUDE = os.path.join(ROOT, "include")
 OBJDIR = os.path.join(CSRC, "build")
 LIB = os.path.join(PKG, "libcame_b200.so")
+HOST = os.path.join(PKG, "_host.so")
 SOURCES = ["capi.cu", "codec.cu", "factored.cu", "fast_tile8.cu", "fp_wide.cu", "fused_ma.cu", "fused_sq.cu", "generic.cu", "nd.cu", "noalloc.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-I", INCLUDE, "-I", CSRC]
@@ -30,17 +33,38 @@ def find_nvcc() -> str:
 
 
 def _newest_source_mtime() -> float:
-    paths = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh", ".h"))]
+    paths = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh", ".h", ".cpp"))]
     paths.append(os.path.join(INCLUDE, "came_b200.h"))
     return max(os.path.getmtime(p) for p in paths)
 
 
 def is_stale() -> bool:
-    return (not os.path.exists(LIB)) or os.path.getmtime(LIB) < _newest_source_mtime()
+    built = [os.path.getmtime(p) for p in (LIB, HOST) if os.path.exists(p)]
+    return len(built) < 2 or min(built) < _newest_source_mtime()
+
+
+def build_host() -> None:
+    """The CPython extension module: plain g++ with the include and library paths of the installed torch."""
+    import torch
+    from torch.utils import cpp_extension
+    cuda = os.path.dirname(os.path.dirname(find_nvcc()))
+    libs = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-w",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I", INCLUDE,
+           "-I", sysconfig.get_path("include"), "-I", os.path.join(cuda, "include")]
+    for inc in cpp_extension.include_paths():
+        cmd += ["-isystem", inc]
+    tmp = HOST + ".tmp"
+    cmd += [os.path.join(CSRC, "host.cpp"), "-o", tmp, "-L", PKG, "-l:libcame_b200.so", "-Wl,-rpath,$ORIGIN", "-L", libs,
+            "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed on host.cpp:\n{res.stdout}\n{res.stderr}")
+    os.replace(tmp, HOST)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compiles every translation unit for sm_100a and links the shared library; returns its path."""
+    """Compiles every translation unit for sm_100a, links the shared library and the host module; returns the library's path."""
     if not force and not is_stale():
         return LIB
     nvcc = find_nvcc()
@@ -64,6 +88,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if res.returncode != 0:
         raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
     os.replace(tmp, LIB)
+    build_host()
     return LIB
 
 

@@ -71,12 +71,12 @@ struct VecFlags {
     bool operator==(const VecFlags& o) const { return k == o.k && wide == o.wide && v == o.v; }
 };
 
-VecFlags vec_flags(const CameTensorDesc& d) {
+VecFlags vec_flags(const CameTensorDesc& d, bool fast) {
     VecFlags f{0, 0, 0};
     if (d.cols == 0 || is_nd(d)) return f;      // 1-D and N-D tensors have kernels of their own
     const bool aligned = aligned16(d.g) && aligned16(d.m) && aligned16(d.p);
     f.v = aligned && d.cols % 8 == 0 ? 8 : 1;
-    f.wide = !disable_fast() && aligned &&
+    f.wide = fast && aligned &&
              ((d.mode != CAME_MODE_FLAT8 && d.cols % 64 == 0) ||
               (d.mode == CAME_MODE_FLAT8 && d.cols % 256 == 0 && d.g_dtype == d.p_dtype));
     // (tensors with the 1e-30 clamps take the fused first pass too: its closed form for the clip sum holds whenever no
@@ -84,6 +84,8 @@ VecFlags vec_flags(const CameTensorDesc& d) {
     if (f.wide) f.k = fused_sq_eligible(d.cols, elem_bytes(d.g_dtype)) ? 2 : 1;
     return f;
 }
+
+VecFlags vec_flags(const CameTensorDesc& d) { return vec_flags(d, !disable_fast()); }
 
 // Small sets: every matrix of a set with fewer elements than this on the staged path takes the whole-step kernel.
 // CAME_B200_SMALL_SET_ELEMS overrides the line (0: none; read whenever a plan is sized or created).
@@ -712,20 +714,31 @@ int came_b200_plan_set_pointers(came_plan_t* plan, const void* const* g, void* c
     if (!plan) return fail(CAME_E_INVALID, "set_pointers: plan is null");
     if (n_tensors != plan->n_tensors) return fail(CAME_E_INVALID, "set_pointers: %d tensors given, plan has %d", n_tensors, plan->n_tensors);
     if (!g && !p) return CAME_OK;
-    std::vector<CameTensorDesc> next = plan->descs;
+    // (only the addresses change: nothing is copied back when one of them is refused)
+    const bool fast = !disable_fast();
     for (int i = 0; i < n_tensors; ++i) {
-        if (g) next[i].g = g[i];
-        if (p) next[i].p = p[i];
-        if (!next[i].g || !next[i].p) return fail(CAME_E_INVALID, "set_pointers: tensor %d: null pointer", i);
-        if (!(vec_flags(next[i]) == plan->vflags[i]))
+        CameTensorDesc next = plan->descs[i];
+        if (g) next.g = g[i];
+        if (p) next.p = p[i];
+        if (!next.g || !next.p) return fail(CAME_E_INVALID, "set_pointers: tensor %d: null pointer", i);
+        if (!(vec_flags(next, fast) == plan->vflags[i]))
             return fail(CAME_E_INVALID, "set_pointers: tensor %d changes 16-byte alignment class; create a new plan", i);
-        if (plan->n_push > 0 && plan->pushable[i] && !pushed_param_in_range(*plan, next[i]))
+        if (plan->n_push > 0 && plan->pushable[i] && !pushed_param_in_range(*plan, next))
             return fail(CAME_E_INVALID, "set_pointers: tensor %d leaves the buffer the push mode was set up for", i);
     }
-    plan->descs.swap(next);
-    const cudaError_t e = cudaMemcpyAsync(plan->ws + plan->L.off_descs, plan->descs.data(),
-                                          (size_t)n_tensors * sizeof(CameTensorDesc), cudaMemcpyHostToDevice, (cudaStream_t)stream);
-    return e == cudaSuccess ? CAME_OK : fail(CAME_E_CUDA, "set_pointers: %s", cudaGetErrorString(e));
+    for (int i = 0; i < n_tensors; ++i) {
+        if (g) plan->descs[i].g = g[i];
+        if (p) plan->descs[i].p = p[i];
+    }
+    // pageable copies up to 64 KB return as soon as they are staged; longer ones wait for the stream
+    const size_t total = (size_t)n_tensors * sizeof(CameTensorDesc), piece = 48 * 1024;
+    const char* src = reinterpret_cast<const char*>(plan->descs.data());
+    for (size_t at = 0; at < total; at += piece) {
+        const cudaError_t e = cudaMemcpyAsync(plan->ws + plan->L.off_descs + at, src + at, std::min(piece, total - at),
+                                              cudaMemcpyHostToDevice, (cudaStream_t)stream);
+        if (e != cudaSuccess) return fail(CAME_E_CUDA, "set_pointers: %s", cudaGetErrorString(e));
+    }
+    return CAME_OK;
 }
 
 int came_b200_plan_set_hyper(came_plan_t* plan, const CameHyper* hypers, int n_groups) {

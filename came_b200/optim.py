@@ -19,17 +19,19 @@ scratch tensor in the optimizer state and no CPU / eager fallback: parameters mu
 from __future__ import annotations
 
 import copy
+import importlib
 import math
 import warnings
 
 import torch
 import torch.optim
 
-from . import _lib
+from . import _host, _lib
 from .engine import Entry, StepEngine, make_hyper
 
 BLOCK = 256
 TILE = 16
+_torch_optimizer_module = importlib.import_module("torch.optim.optimizer")
 
 _FLAGS_CAME = _lib.F_WD_ADD2
 _FLAGS_CUDAFP_2D = _lib.F_SQ_CLAMP | _lib.F_RESROW_CLAMP | _lib.F_RESCOL_CLAMP
@@ -49,6 +51,12 @@ _SCRATCH_KEYS = frozenset({
     "grad_fp32", "exp_avg_fp32", "row_absmax_scratch", "_cuda_nonfactored_update_fp16", "sum_update_slice",
     "sum_update_equiv", "sum_update_chunk",
 })
+
+
+def _global_hooks() -> bool:
+    """Whether hooks for the steps of all optimizers are registered."""
+    m = _torch_optimizer_module
+    return bool(getattr(m, "_global_optimizer_pre_hooks", None) or getattr(m, "_global_optimizer_post_hooks", None))
 
 
 def _num_blocks(n: int) -> int:
@@ -271,52 +279,60 @@ class _CameB200Optimizer(torch.optim.Optimizer):
             hypers.append(make_hyper(*hp, python_scalars=True, grad_scale=gs))
         return hypers
 
-    def _signature(self):
-        """What decides the tensor table of a step: per parameter its gradient's address, dtype and shape (None for a
-        parameter without gradient).  While it stays the same the plans of the previous step are stepped again
-        without rebuilding the per-tensor entries (hyper-parameters are re-read every step all the same)."""
-        sig = []
-        for group in self.param_groups:
-            for p in group["params"]:
-                g = p.grad
-                if g is None:
-                    sig.append(None)
-                elif g.is_sparse or not (g.is_contiguous() and p.is_contiguous()):
-                    return None            # slow path: raises / copies as the reference does
-                else:
-                    sig.append((p.data_ptr(), g.data_ptr(), g.dtype, p.shape))
-        return sig
+    # The tensor table of a step (per parameter its address, its gradient's address, dtype and shape, or None) is kept by
+    # a native StepTable.  While it stands, or only gradient addresses moved, the plans of the previous step are stepped
+    # again from there without touching the per-tensor entries (hyper-parameters are re-read every step all the same).
+    def _remember(self, entries, copy_backs):
+        self._table = None
+        if not entries or copy_backs or any(e.keep for e in entries):
+            return
+        stepped = [self.state[p] for g in self.param_groups for p in g["params"]
+                   if p.grad is not None and "step" in self.state[p]]
+        plans = [(plan.handle.value, plan.device.index, plan, plan.n) for plan in self._engine.plans.values()]
+        table = _host.StepTable()
+        if all(isinstance(g["params"], list) for g in self.param_groups) and table.build(self.param_groups, plans, stepped):
+            self._table = table
+
+    def _step_again(self) -> bool:
+        """Steps the remembered table; False when the full path has to be taken."""
+        table = getattr(self, "_table", None)
+        if table is None:
+            return False
+        n = table.step(self.param_groups)
+        if n >= 0:
+            self.last_step_launches = n
+            return True
+        self._table = None
+        if n < -1:
+            _lib.check(n + 1000)
+        return False
 
     @torch.no_grad()
-    def step(self, closure=None):
+    def _step_full(self, closure=None):
         loss = None
         if closure is not None:
             with torch.enable_grad():
                 loss = closure()
-        sig = self._signature()
-        cached = getattr(self, "_step_cache", None)
-        if sig is not None and cached is not None and cached[0] == sig and cached[3] == len(self.param_groups):
-            _, plans, stepped_states, _ = cached
-            for st in stepped_states:
-                st["step"] += 1
-            hypers = self._hypers()
-            launches = 0
-            for plan in plans:
-                plan.step(hypers)
-                launches += plan.last_launches
-            self.last_step_launches = launches
+        if self._step_again():
             return loss
-        self._step_cache = None
         entries, hypers, copy_backs = self._collect()
         if entries:
             self.last_step_launches = self._engine.step(entries, hypers)
         for p, p_data in copy_backs:
             p.data.copy_(p_data)
-        if entries and sig is not None and not copy_backs and not any(e.keep for e in entries):
-            stepped = [self.state[p] for g in self.param_groups for p in g["params"]
-                       if p.grad is not None and "step" in self.state[p]]
-            self._step_cache = (sig, list(self._engine.plans.values()), stepped, len(self.param_groups))
+        self._remember(entries, copy_backs)
         return loss
+
+    # step() with torch's hooks and profiler range around it (what torch wraps around every optimizer's step)
+    _step_hooked = torch.optim.Optimizer.profile_hook_step(_step_full)
+
+    def step(self, closure=None):
+        if closure is None and not (self._optimizer_step_pre_hooks or self._optimizer_step_post_hooks or _global_hooks() or
+                                    torch.autograd._profiler_enabled()) and self._step_again():
+            return None
+        return self._step_hooked(closure)
+
+    step.hooked = True      # torch leaves it unwrapped: the wrapper costs as much as the step of a small set
 
     @torch.no_grad()
     def prime_for_cuda_graph(self) -> None:
@@ -366,11 +382,11 @@ class _CameB200Optimizer(torch.optim.Optimizer):
             if st.get("_mode") == "full8bit" and st.get("factored", False) and "factored_row_q" in st:
                 bind_flat_views(st)
         self._engine.invalidate()
-        self._step_cache = None
+        self._table = None
 
     def add_param_group(self, param_group):
         super().add_param_group(param_group)
-        self._step_cache = None
+        self._table = None
 
 
 # ----------------------------------------------------------------------------------------------
