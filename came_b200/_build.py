@@ -19,7 +19,7 @@ INCLUDE = os.path.join(ROOT, "include")
 OBJDIR = os.path.join(CSRC, "build")
 LIB = os.path.join(PKG, "libcame_b200.so")
 HOST = os.path.join(PKG, "_host.so")
-SOURCES = ["capi.cu", "codec.cu", "factored.cu", "fast_tile8.cu", "fp_wide.cu", "fused_ma.cu", "fused_sq.cu", "generic.cu", "nd.cu", "noalloc.cu"]
+SOURCES = ["capi.cu", "codec.cu", "factored.cu", "fast_tile8.cu", "fp_wide.cu", "fused_ma.cu", "fused_sq.cu", "generic.cu", "nd.cu", "nd_fixed.cu", "noalloc.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-I", INCLUDE, "-I", CSRC]
 NVCC_FLAGS += os.environ.get("CAME_B200_NVCC_FLAGS", "").split()   # build-time experiment switches, e.g. -DCAME_TUNE

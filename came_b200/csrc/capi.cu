@@ -520,7 +520,11 @@ int came_b200_plan_create(const CameTensorDesc* descs, int n_tensors, void* work
     auto nmat = [&](int i) { return (int64_t)D[i].batch; };
     auto nblk = [&](int i) { return geo[i].flat_chunks; };
     auto ndlarge = [&](int i) { return isnd(i) && !nd_chunk(D[i]); };
-    auto ndkey = [&](int i) { return nd_chunk(D[i]) ? Key{0, 0, nd_small_key(D[i].rows, D[i].cols), 2} : Key{0, 0, 0, 0}; };
+    auto ndkey = [&](int i) {
+        if (!nd_chunk(D[i])) return Key{0, 0, 0, 0};
+        if (!nd_fixed_batch(D[i].rows, D[i].cols)) return Key{0, 0, nd_small_kb(D[i].rows, D[i].cols), 2};
+        return Key{D[i].g_dtype, D[i].p_dtype, (D[i].mode != CAME_MODE_FP32 ? 1 : 0) | (D[i].rows == 3 ? 2 : 0), 3};
+    };
     build(KID_ND_SQ, ndlarge, nokey, nvec);
     build(KID_ND_MEAN, ndlarge, nokey, nmat);
     build(KID_ND_SUMSQ, isnd, ndkey, nblk);

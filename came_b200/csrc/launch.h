@@ -27,7 +27,7 @@ struct KernelKey {
     int g_dtype;
     int p_dtype;
     int mode;
-    int variant;   // 1: 16-byte vector loads; 2: shared-memory staged path (N-D tensors: small matrices)
+    int variant;   // 1: 16-byte vector loads; 2: shared-memory staged path (N-D tensors: small matrices; 3: 3 x 3 and 1 x 1)
 };
 
 enum KernelId {
@@ -92,9 +92,12 @@ cudaError_t launch_generic(const KernelKey& key, const StepArgs& a, const CameHy
                            cudaStream_t st);
 
 cudaError_t launch_nd(int kernel, const KernelKey& key, const StepArgs& a, const Work* work, int n, cudaStream_t st);
-// tensors of more than two dimensions made of small matrices: matrices of a chunk (0: other kernels), launch key
+// tensors of more than two dimensions made of small matrices: matrices of a chunk (0: other kernels), KB of shared memory
 int nd_small_batch(int64_t rows, int64_t cols);
-int nd_small_key(int64_t rows, int64_t cols);
+int nd_small_kb(int64_t rows, int64_t cols);
+// the same for 3 x 3 and 1 x 1 (nd_fixed.cu); key: element types, mode = 8-bit states | 3 x 3 << 1
+int nd_fixed_batch(int64_t rows, int64_t cols);
+cudaError_t launch_nd_fixed(int kernel, const KernelKey& key, const StepArgs& a, const Work* work, int n, cudaStream_t st);
 cudaError_t launch_selftest_bounded_wait(int* status, int* observed, cudaStream_t st);
 
 cudaError_t launch_quantize_blockwise(const float* src, void* q, float* absmax, int64_t n, bool is_signed,

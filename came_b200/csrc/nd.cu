@@ -15,9 +15,9 @@
 //   nd_s               partials                  -> S, clip
 //   nd_apply (small)   g, m, p, states           -> all states, m, p (the second moment is formed again from g and the
 //                                                  old state: cheaper than 4 bytes per vector entry written and read)
-// Bound by instruction issue and latency, not by DRAM: ~240 thread instructions per element, most of them divisions and
-// square roots of the factors and the codec.  52 M elements of 3 x 3 and 1 x 1 kernels (fp16, flat layout): 1.0 ms a step;
-// with the kernels below (one CTA per matrix mean, one thread per vector entry) 27.5 ms.
+// 3 x 3 and 1 x 1 have kernels of their own (nd_fixed.cu), the other shapes up to 64 elements run below.  Bound by
+// instruction issue and latency, not by DRAM: ~240 thread instructions per element, most of them divisions and square
+// roots of the factors and the codec.
 //
 // Any other shape: one thread owns one entry of a state vector and walks its row (column); the element-wise passes own
 // one flat block of 256 elements per CTA.
@@ -272,27 +272,26 @@ __global__ void __launch_bounds__(THREADS) k_nd_apply(StepArgs a, const Work* __
 constexpr int NDS_SMEM_MAX = 200 * 1024;
 
 // Shared-memory position of entry i.  Threads own matrices, i.e. strides of R * C, R or C words: an odd stride is free of
-// bank conflicts; for the run-time shapes one word of padding every 32 spreads the even ones.
-template <int R0> __host__ __device__ __forceinline__ int nds_pos(int i) { return R0 ? i : i + (i >> 5); }
+// bank conflicts; one word of padding every 32 spreads the even ones.
+__host__ __device__ __forceinline__ int nds_pos(int i) { return i + (i >> 5); }
 
-// shared floats of a chunk of `nm` matrices: elements (g, then u, then the update), momentum, and the four vectors (old,
-// then fresh values); the run-time shapes also keep their factors there
+// shared floats of a chunk of `nm` matrices: elements (g, then u, then the update), momentum, the four vectors (old,
+// then fresh values) and two vectors of factors
 static size_t nds_floats(int nm, int64_t R, int64_t C) {
     auto up = [](int n) { return (size_t)((n + (n >> 5) + 4) & ~3); };
     return 2 * up((int)(nm * R * C)) + 3 * (up((int)(nm * R)) + up((int)(nm * C)));
 }
-static bool nds_fixed(int64_t R, int64_t C) { return (R == 1 && C == 1) || (R == 3 && C == 3); }
 
 // matrices of a chunk (a multiple of 256, about 2048 elements at least), 0: not a small matrix
 int nd_small_batch(int64_t rows, int64_t cols) {
     if (rows * cols > 64) return 0;
+    if (const int fixed = nd_fixed_batch(rows, cols)) return fixed;
     const int nm = QBLOCK * (int)(rows * cols >= 8 ? 1 : 8 / (rows * cols));
     return nds_floats(nm, rows, cols) * sizeof(float) <= (size_t)NDS_SMEM_MAX ? nm : 0;
 }
-// template instance and shared memory of a launch: bit 0 set: 1 x 1, bit 1: 3 x 3, else run-time shape; KB above
-int nd_small_key(int64_t rows, int64_t cols) {
-    const int kb = (int)((nds_floats(nd_small_batch(rows, cols), rows, cols) * sizeof(float) + 1023) / 1024);
-    return (nds_fixed(rows, cols) ? (rows == 1 ? 1 : 2) : 0) | (kb << 2);
+// KB of shared memory of a launch
+int nd_small_kb(int64_t rows, int64_t cols) {
+    return (int)((nds_floats(nd_small_batch(rows, cols), rows, cols) * sizeof(float) + 1023) / 1024);
 }
 
 struct NdsChunk {
@@ -300,11 +299,10 @@ struct NdsChunk {
     int64_t e0, r0, c0;        // first element, row entry, column entry
     float *el, *m, *row, *col, *rrow, *rcol, *frow, *fcol;
 };
-template <int R0, int C0>
 __device__ __forceinline__ NdsChunk nds_chunk(const CameTensorDesc& d, const Scratch& s, int tile, float* smem) {
     NdsChunk k;
     const int full = s.tiles_c;
-    k.R = R0 ? R0 : (int)d.rows; k.C = C0 ? C0 : (int)d.cols; k.RC = k.R * k.C;
+    k.R = (int)d.rows; k.C = (int)d.cols; k.RC = k.R * k.C;
     const int64_t mat0 = (int64_t)tile * full;
     k.nm = (int)min((int64_t)full, (int64_t)d.batch - mat0);
     k.e0 = mat0 * k.RC; k.r0 = mat0 * k.R; k.c0 = mat0 * k.C;
@@ -316,20 +314,17 @@ __device__ __forceinline__ NdsChunk nds_chunk(const CameTensorDesc& d, const Scr
 }
 
 // Four consecutive values of a chunk in shared memory, i a multiple of 4
-template <int R0> __device__ __forceinline__ void nds_put4(float* dst, int i, const float4& v) {
-    if (R0) { *reinterpret_cast<float4*>(dst + i) = v; return; }
-    float* p = dst + nds_pos<R0>(i);      // four entries never straddle a padding word
+__device__ __forceinline__ void nds_put4(float* dst, int i, const float4& v) {
+    float* p = dst + nds_pos(i);      // four entries never straddle a padding word
     p[0] = v.x; p[1] = v.y; p[2] = v.z; p[3] = v.w;
 }
-template <int R0> __device__ __forceinline__ float4 nds_get4(const float* src, int i) {
-    if (R0) return *reinterpret_cast<const float4*>(src + i);
-    const float* p = src + nds_pos<R0>(i);
+__device__ __forceinline__ float4 nds_get4(const float* src, int i) {
+    const float* p = src + nds_pos(i);
     return make_float4(p[0], p[1], p[2], p[3]);
 }
 
 // n values from element index `base` (a multiple of 256) of an array -> shared memory.  A group of 4 consecutive values
 // per thread; the last, short group and arrays off the alignment of four values go one by one.
-template <int R0>
 __device__ __forceinline__ void nds_stage(const void* src, int dtype, int64_t base, int n, float scale, float* dst) {
     const bool vec = (reinterpret_cast<uintptr_t>(src) & 15) == 0;
     for (int i = 4 * threadIdx.x; i < n; i += 4 * THREADS) {
@@ -338,11 +333,11 @@ __device__ __forceinline__ void nds_stage(const void* src, int dtype, int64_t ba
         else
 #pragma unroll
             for (int e = 0; e < 4; ++e) v[e] = i + e < n ? nd_load(src, dtype, base + i + e) : 0.0f;
-        nds_put4<R0>(dst, i, make_float4(v[0] * scale, v[1] * scale, v[2] * scale, v[3] * scale));
+        nds_put4(dst, i, make_float4(v[0] * scale, v[1] * scale, v[2] * scale, v[3] * scale));
     }
 }
 // the same for 8-bit codes with one absmax per 256 entries (a warp's 4 x 32 entries lie in one block)
-template <int R0, bool SIGNED>
+template <bool SIGNED>
 __device__ __forceinline__ void nds_stage_codes(const void* codes, const float* absmax, int64_t base, int n, float* dst) {
     const uint8_t* src = reinterpret_cast<const uint8_t*>(codes);
     const bool vec = (reinterpret_cast<uintptr_t>(src) & 3) == 0;
@@ -359,16 +354,14 @@ __device__ __forceinline__ void nds_stage_codes(const void* codes, const float* 
             const uint32_t b = (w >> (8 * e)) & 0xffu;
             v[e] = (SIGNED ? (float)(int8_t)b : (float)b) * sc;
         }
-        nds_put4<R0>(dst, i, make_float4(v[0], v[1], v[2], v[3]));
+        nds_put4(dst, i, make_float4(v[0], v[1], v[2], v[3]));
     }
 }
-template <int R0>
 __device__ __forceinline__ void nds_stage_vec(const void* state, const float* absmax, bool quant, int64_t base, int n, float* dst) {
-    if (quant) nds_stage_codes<R0, false>(state, absmax, base, n, dst);
-    else nds_stage<R0>(state, CAME_DT_F32, base, n, 1.0f, dst);
+    if (quant) nds_stage_codes<false>(state, absmax, base, n, dst);
+    else nds_stage(state, CAME_DT_F32, base, n, 1.0f, dst);
 }
 // fresh values back into a state vector: a warp owns a block of 256 entries, a lane entries 4 lane .. + 3 of each half
-template <int R0>
 __device__ __forceinline__ void nds_store_vec(void* state, float* absmax, bool quant, int64_t base, int n, const float* src) {
     const int lane = threadIdx.x & 31;
     uint8_t* q = reinterpret_cast<uint8_t*>(state);
@@ -380,7 +373,7 @@ __device__ __forceinline__ void nds_store_vec(void* state, float* absmax, bool q
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
             const int i = i0 + 128 * t;
-            v[t] = nds_get4<R0>(src, i);      // (entries past the end lie in the arrays' own shared memory)
+            v[t] = nds_get4(src, i);      // (entries past the end lie in the arrays' own shared memory)
             if (i >= n) v[t].x = 0.0f;
             if (i + 1 >= n) v[t].y = 0.0f;
             if (i + 2 >= n) v[t].z = 0.0f;
@@ -409,84 +402,41 @@ __device__ __forceinline__ void nds_store_vec(void* state, float* absmax, bool q
     }
 }
 
-// mean of `len` terms (a compile-time length of the fixed shapes: the quotient without a division)
-__device__ __forceinline__ float nds_mean(float acc, float len) {
-    return acc < 1e30f && acc > 1e-30f ? div_by(acc, len, 1.0f / len) : acc / len;
-}
-
 // Row and column vectors of matrix `mat` from the terms x(e): EMA with the old values in row / col (replaced by the
 // fresh ones), then out(e, r_i, c_j) for every element e.
-template <int R0, int C0, typename X, typename OUT>
+template <typename X, typename OUT>
 __device__ __forceinline__ void nds_matrix(const NdsChunk& k, int mat, float* row, float* col, X x, OUT out, float beta, float om,
                                            bool fix, bool clamp_row, bool clamp_col) {
     const int e0 = mat * k.RC, r0 = mat * k.R, c0 = mat * k.C;
-    if constexpr (R0 > 0) {
-        float rs[R0], cs[C0], total = 0.0f;
-#pragma unroll
-        for (int j = 0; j < C0; ++j) cs[j] = 0.0f;
-#pragma unroll
-        for (int i = 0; i < R0; ++i) {
-            float acc = 0.0f;
-#pragma unroll
-            for (int j = 0; j < C0; ++j) {
-                const float t = x(e0 + i * C0 + j);
-                acc += t;
-                cs[j] += t;
-            }
-            rs[i] = ema_update(row[r0 + i], beta, om, nds_mean(acc, (float)C0));
-            row[r0 + i] = rs[i];
-            total += rs[i];
-        }
-        const float mean = guard_mean(nds_mean(total, (float)R0), fix, clamp_row), inv = 1.0f / mean;
-        const bool easy = mean > 1e-30f && mean < 1e30f;
-#pragma unroll
-        for (int i = 0; i < R0; ++i) {
-            float ratio = easy ? div_by(rs[i], mean, inv) : rs[i] / mean;
-            if (clamp_row) ratio = fmaxf(ratio, 1e-30f);
-            rs[i] = inv_sqrt(ratio);
-        }
-#pragma unroll
-        for (int j = 0; j < C0; ++j) {
-            const float v = ema_update(col[c0 + j], beta, om, nds_mean(cs[j], (float)R0));
-            col[c0 + j] = v;
-            cs[j] = inv_sqrt(clamp_col ? fmaxf(v, 1e-30f) : v);
-        }
-#pragma unroll
-        for (int i = 0; i < R0; ++i)
-#pragma unroll
-            for (int j = 0; j < C0; ++j) out(e0 + i * C0 + j, rs[i], cs[j]);
-    } else {
-        float total = 0.0f;
-        for (int i = 0; i < k.R; ++i) {
-            float acc = 0.0f;
-            for (int j = 0; j < k.C; ++j) acc += x(e0 + i * k.C + j);
-            const float v = ema_update(row[nds_pos<0>(r0 + i)], beta, om, acc / (float)k.C);
-            row[nds_pos<0>(r0 + i)] = v;
-            total += v;
-        }
-        const float mean = guard_mean(total / (float)k.R, fix, clamp_row);
-        for (int i = 0; i < k.R; ++i) k.frow[nds_pos<0>(r0 + i)] = row_factor(row[nds_pos<0>(r0 + i)], mean, clamp_row);
-        for (int j = 0; j < k.C; ++j) {
-            float acc = 0.0f;
-            for (int i = 0; i < k.R; ++i) acc += x(e0 + i * k.C + j);
-            const float v = ema_update(col[nds_pos<0>(c0 + j)], beta, om, acc / (float)k.R);
-            col[nds_pos<0>(c0 + j)] = v;
-            k.fcol[nds_pos<0>(c0 + j)] = col_factor(v, clamp_col);
-        }
-        for (int i = 0; i < k.R; ++i) {
-            const float r = k.frow[nds_pos<0>(r0 + i)];
-            for (int j = 0; j < k.C; ++j) out(e0 + i * k.C + j, r, k.fcol[nds_pos<0>(c0 + j)]);
-        }
+    float total = 0.0f;
+    for (int i = 0; i < k.R; ++i) {
+        float acc = 0.0f;
+        for (int j = 0; j < k.C; ++j) acc += x(e0 + i * k.C + j);
+        const float v = ema_update(row[nds_pos(r0 + i)], beta, om, acc / (float)k.C);
+        row[nds_pos(r0 + i)] = v;
+        total += v;
+    }
+    const float mean = guard_mean(total / (float)k.R, fix, clamp_row);
+    for (int i = 0; i < k.R; ++i) k.frow[nds_pos(r0 + i)] = row_factor(row[nds_pos(r0 + i)], mean, clamp_row);
+    for (int j = 0; j < k.C; ++j) {
+        float acc = 0.0f;
+        for (int i = 0; i < k.R; ++i) acc += x(e0 + i * k.C + j);
+        const float v = ema_update(col[nds_pos(c0 + j)], beta, om, acc / (float)k.R);
+        col[nds_pos(c0 + j)] = v;
+        k.fcol[nds_pos(c0 + j)] = col_factor(v, clamp_col);
+    }
+    for (int i = 0; i < k.R; ++i) {
+        const float r = k.frow[nds_pos(r0 + i)];
+        for (int j = 0; j < k.C; ++j) out(e0 + i * k.C + j, r, k.fcol[nds_pos(c0 + j)]);
     }
 }
-template <int R0, int C0, typename OUT>
+template <typename OUT>
 __device__ __forceinline__ void nds_second_moment(const NdsChunk& k, int mat, const CameTensorDesc& d, const CameHyper& h, OUT out) {
     const bool clamp = d.flags & CAME_F_SQ_CLAMP;
-    nds_matrix<R0, C0>(k, mat, k.row, k.col, [&](int e) { const float g = k.el[nds_pos<R0>(e)]; return fmaf(g, g, h.eps0); },
+    nds_matrix(k, mat, k.row, k.col, [&](int e) { const float g = k.el[nds_pos(e)]; return fmaf(g, g, h.eps0); },
                        out, h.beta2, h.om_beta2, d.flags & CAME_F_SQ_FIX, clamp, clamp);
 }
 
-template <int R0, int C0>
 __global__ void __launch_bounds__(THREADS) k_nds_sumsq(StepArgs a, const Work* __restrict__ work) {
     extern __shared__ __align__(16) float nds_smem[];
     __shared__ float red[33];
@@ -494,23 +444,22 @@ __global__ void __launch_bounds__(THREADS) k_nds_sumsq(StepArgs a, const Work* _
     const CameTensorDesc& d = a.descs[w.tensor];
     const Scratch& s = a.scr[w.tensor];
     const CameHyper& h = a.hyp[d.group];
-    const NdsChunk k = nds_chunk<R0, C0>(d, s, w.tile, nds_smem);
+    const NdsChunk k = nds_chunk(d, s, w.tile, nds_smem);
     const bool quant = d.mode != CAME_MODE_FP32;
-    nds_stage<R0>(d.g, d.g_dtype, k.e0, k.nm * k.RC, h.grad_scale, k.el);
-    nds_stage_vec<R0>(d.sq_row, d.sq_row_absmax, quant, k.r0, k.nm * k.R, k.row);
-    nds_stage_vec<R0>(d.sq_col, d.sq_col_absmax, quant, k.c0, k.nm * k.C, k.col);
+    nds_stage(d.g, d.g_dtype, k.e0, k.nm * k.RC, h.grad_scale, k.el);
+    nds_stage_vec(d.sq_row, d.sq_row_absmax, quant, k.r0, k.nm * k.R, k.row);
+    nds_stage_vec(d.sq_col, d.sq_col_absmax, quant, k.c0, k.nm * k.C, k.col);
     __syncthreads();
     float acc = 0.0f;
     for (int mat = threadIdx.x; mat < k.nm; mat += THREADS)
-        nds_second_moment<R0, C0>(k, mat, d, h, [&](int e, float r, float c) {
-            const float u = (k.el[nds_pos<R0>(e)] * r) * c;
+        nds_second_moment(k, mat, d, h, [&](int e, float r, float c) {
+            const float u = (k.el[nds_pos(e)] * r) * c;
             acc = fmaf(u, u, acc);
         });
     const float t = block_sum(acc, red);
     if (threadIdx.x == 0) s.spart[w.tile] = t;
 }
 
-template <int R0, int C0>
 __global__ void __launch_bounds__(THREADS) k_nds_step(StepArgs a, const Work* __restrict__ work) {
     extern __shared__ __align__(16) float nds_smem[];
     const Work w = work[blockIdx.x];
@@ -518,37 +467,37 @@ __global__ void __launch_bounds__(THREADS) k_nds_step(StepArgs a, const Work* __
     const Scratch& s = a.scr[w.tensor];
     const CameHyper h = a.hyp[d.group];
     const uint32_t flags = d.flags;
-    const NdsChunk k = nds_chunk<R0, C0>(d, s, w.tile, nds_smem);
+    const NdsChunk k = nds_chunk(d, s, w.tile, nds_smem);
     const bool quant = d.mode != CAME_MODE_FP32;
     const int ne = k.nm * k.RC, nr = k.nm * k.R, nc = k.nm * k.C, lane = threadIdx.x & 31, wd = wd_form(h, flags);
     const float inv_clip = 1.0f / s.scal[1];
-    nds_stage<R0>(d.g, d.g_dtype, k.e0, ne, h.grad_scale, k.el);
-    if (quant) nds_stage_codes<R0, true>(d.m, d.m_absmax, k.e0, ne, k.m);
-    else nds_stage<R0>(d.m, CAME_DT_F32, k.e0, ne, 1.0f, k.m);
-    nds_stage_vec<R0>(d.sq_row, d.sq_row_absmax, quant, k.r0, nr, k.row);
-    nds_stage_vec<R0>(d.sq_col, d.sq_col_absmax, quant, k.c0, nc, k.col);
-    nds_stage_vec<R0>(d.res_row, d.res_row_absmax, quant, k.r0, nr, k.rrow);
-    nds_stage_vec<R0>(d.res_col, d.res_col_absmax, quant, k.c0, nc, k.rcol);
+    nds_stage(d.g, d.g_dtype, k.e0, ne, h.grad_scale, k.el);
+    if (quant) nds_stage_codes<true>(d.m, d.m_absmax, k.e0, ne, k.m);
+    else nds_stage(d.m, CAME_DT_F32, k.e0, ne, 1.0f, k.m);
+    nds_stage_vec(d.sq_row, d.sq_row_absmax, quant, k.r0, nr, k.row);
+    nds_stage_vec(d.sq_col, d.sq_col_absmax, quant, k.c0, nc, k.col);
+    nds_stage_vec(d.res_row, d.res_row_absmax, quant, k.r0, nr, k.rrow);
+    nds_stage_vec(d.res_col, d.res_col_absmax, quant, k.c0, nc, k.rcol);
     __syncthreads();
     for (int mat = threadIdx.x; mat < k.nm; mat += THREADS) {
         // u in place of g, the new momentum in place of the old
-        nds_second_moment<R0, C0>(k, mat, d, h, [&](int e, float r, float c) {
-            const int at = nds_pos<R0>(e);
+        nds_second_moment(k, mat, d, h, [&](int e, float r, float c) {
+            const int at = nds_pos(e);
             const float u = ((k.el[at] * r) * c) * inv_clip;
             k.el[at] = u;
             k.m[at] = k.m[at] * h.beta1 + h.om_beta1 * u;
         });
         // the update in place of u
-        nds_matrix<R0, C0>(k, mat, k.rrow, k.rcol,
-            [&](int e) { const int at = nds_pos<R0>(e); const float df = k.el[at] - k.m[at]; return fmaf(df, df, h.eps1); },
-            [&](int e, float r, float c) { const int at = nds_pos<R0>(e); k.el[at] = (k.m[at] * r) * c; },
+        nds_matrix(k, mat, k.rrow, k.rcol,
+            [&](int e) { const int at = nds_pos(e); const float df = k.el[at] - k.m[at]; return fmaf(df, df, h.eps1); },
+            [&](int e, float r, float c) { const int at = nds_pos(e); k.el[at] = (k.m[at] * r) * c; },
             h.beta3, h.om_beta3, flags & CAME_F_RESROW_FIX, flags & CAME_F_RESROW_CLAMP, flags & CAME_F_RESCOL_CLAMP);
     }
     __syncthreads();
-    nds_store_vec<R0>(d.sq_row, d.sq_row_absmax, quant, k.r0, nr, k.row);
-    nds_store_vec<R0>(d.sq_col, d.sq_col_absmax, quant, k.c0, nc, k.col);
-    nds_store_vec<R0>(d.res_row, d.res_row_absmax, quant, k.r0, nr, k.rrow);
-    nds_store_vec<R0>(d.res_col, d.res_col_absmax, quant, k.c0, nc, k.rcol);
+    nds_store_vec(d.sq_row, d.sq_row_absmax, quant, k.r0, nr, k.row);
+    nds_store_vec(d.sq_col, d.sq_col_absmax, quant, k.c0, nc, k.col);
+    nds_store_vec(d.res_row, d.res_row_absmax, quant, k.r0, nr, k.rrow);
+    nds_store_vec(d.res_col, d.res_col_absmax, quant, k.c0, nc, k.rcol);
     // momentum and parameter, a warp per flat block of 256 elements
     const bool vec = (reinterpret_cast<uintptr_t>(d.p) & 15) == 0 && (reinterpret_cast<uintptr_t>(d.m) & 15) == 0;
     for (int b = threadIdx.x >> 5; b * QBLOCK < ne; b += THREADS / 32) {
@@ -567,7 +516,7 @@ __global__ void __launch_bounds__(THREADS) k_nds_step(StepArgs a, const Work* __
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
             const int i = i0 + 128 * t;
-            m[t] = nds_get4<R0>(k.m, i);
+            m[t] = nds_get4(k.m, i);
             if (i >= ne) m[t].x = 0.0f;
             if (i + 1 >= ne) m[t].y = 0.0f;
             if (i + 2 >= ne) m[t].z = 0.0f;
@@ -580,7 +529,7 @@ __global__ void __launch_bounds__(THREADS) k_nds_step(StepArgs a, const Work* __
         for (int t = 0; t < 2; ++t) {
             const int i = i0 + 128 * t;
             const int64_t f = k.e0 + i;
-            const float4 u4 = nds_get4<R0>(k.el, i);
+            const float4 u4 = nds_get4(k.el, i);
             const float upd[4] = {u4.x, u4.y, u4.z, u4.w}, mv[4] = {m[t].x, m[t].y, m[t].z, m[t].w};
             const uint32_t codes = quant ? quant_pack4<true>(m[t], A, sc) : 0u;
 #pragma unroll
@@ -603,10 +552,9 @@ __global__ void __launch_bounds__(THREADS) k_nds_step(StepArgs a, const Work* __
     }
 }
 
-template <int R0, int C0>
 static cudaError_t launch_nds(int kernel, const StepArgs& a, const Work* work, int n, int smem, cudaStream_t st) {
     if (kernel != KID_ND_SUMSQ && kernel != KID_ND_APPLY) return cudaErrorInvalidValue;
-    auto fn = kernel == KID_ND_SUMSQ ? k_nds_sumsq<R0, C0> : k_nds_step<R0, C0>;
+    auto fn = kernel == KID_ND_SUMSQ ? k_nds_sumsq : k_nds_step;
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, NDS_SMEM_MAX);
     if (e != cudaSuccess) return e;
     fn<<<n, THREADS, smem, st>>>(a, work);
@@ -615,14 +563,8 @@ static cudaError_t launch_nds(int kernel, const StepArgs& a, const Work* work, i
 
 cudaError_t launch_nd(int kernel, const KernelKey& key, const StepArgs& a, const Work* work, int n, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    if (key.variant == 2) {      // small matrices (nd_small_key)
-        const int smem = (key.mode >> 2) * 1024;
-        switch (key.mode & 3) {
-            case 1: return launch_nds<1, 1>(kernel, a, work, n, smem, st);
-            case 2: return launch_nds<3, 3>(kernel, a, work, n, smem, st);
-            default: return launch_nds<0, 0>(kernel, a, work, n, smem, st);
-        }
-    }
+    if (key.variant == 3) return launch_nd_fixed(kernel, key, a, work, n, st);
+    if (key.variant == 2) return launch_nds(kernel, a, work, n, key.mode * 1024, st);      // small matrices of any shape
     switch (kernel) {
         case KID_ND_SQ: k_nd_vec<false><<<n, THREADS, 0, st>>>(a, work); break;
         case KID_ND_MEAN: k_nd_mean<false><<<n, THREADS, 0, st>>>(a, work); break;
