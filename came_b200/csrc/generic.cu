@@ -642,8 +642,20 @@ __device__ __forceinline__ void band_apply(const StepArgs& a, const CameHyper* h
 
 // flat layout: a warp owns a block of 256 consecutive elements, whatever rows they belong to (the un-quantised momentum
 // feeds the update: came_kernels.cu:2246-2305, 2487-2511)
+struct FlatTensor {      // what a warp's blocks of one tensor share: formed once, not per block of 8 elements per lane
+    int tensor = -1;
+    float inv_clip, mean;
+    __device__ __forceinline__ void use(const StepArgs& a, const CameHyper* hyp, int t, int lane) {
+        if (t == tensor) return;
+        tensor = t;
+        const CameTensorDesc& d = a.descs[t];
+        const Scratch& s = a.scr[t];
+        inv_clip = read_inv_clip(s, hyp[d.group], d.rows * d.cols, lane);
+        mean = read_mean(s.rowblk2, s.nbR, (int)d.rows, d.flags & CAME_F_RESROW_FIX, d.flags & CAME_F_RESROW_CLAMP, lane);
+    }
+};
 template <typename TG, typename TP, int V>
-__device__ __forceinline__ void phase_apply_flat(const StepArgs& a, const CameHyper* hyp, const Work& w) {
+__device__ __forceinline__ void phase_apply_flat(const StepArgs& a, const CameHyper* hyp, const Work& w, const FlatTensor& ft) {
     const CameTensorDesc d = a.descs[w.tensor];
     const Scratch s = a.scr[w.tensor];
     const CameHyper h = hyp[d.group];
@@ -652,11 +664,9 @@ __device__ __forceinline__ void phase_apply_flat(const StepArgs& a, const CameHy
     const int lane = threadIdx.x & 31, C = (int)d.cols, blk = w.tile;
     const int64_t n = d.rows * d.cols;
     const int wd = wd_form(h, d.flags);
-    const float inv_clip = read_inv_clip(s, h, n, lane);
-    const float mean = read_mean(s.rowblk2, s.nbR, (int)d.rows, d.flags & CAME_F_RESROW_FIX, d.flags & CAME_F_RESROW_CLAMP, lane), inv = 1.0f / mean;
+    const float inv_clip = ft.inv_clip, mean = ft.mean, inv = 1.0f / mean;
     const bool clamp = d.flags & CAME_F_RESROW_CLAMP, easy = mean > 1e-30f && mean < 1e30f;
     int8_t* mq = reinterpret_cast<int8_t*>(d.m);
-    constexpr int STEP = V == 8 ? 1 : 32;      // distance between a lane's elements
     const int64_t i0 = (int64_t)blk * QBLOCK + (V == 8 ? 8 * lane : lane);
     float x[8], m[8], pv[8];
     int cnt;      // elements of this lane (they end where the tensor does)
@@ -680,27 +690,46 @@ __device__ __forceinline__ void phase_apply_flat(const StepArgs& a, const CameHy
     int row, col;
     if (n < 0x7fffffff) { row = (int)((uint32_t)i0 / (uint32_t)C); col = (int)i0 - row * C; }
     else { row = (int)(i0 / C); col = (int)(i0 - (int64_t)row * C); }
+    // (plain loads of the factors: the grid barriers order them behind other SMs' stores, and lines are used many times)
     float upd[8], amax = 0.0f, r = 0.0f, rr = 0.0f;
-    int have = -1;      // row the factors r, rr belong to
+    auto row_factors = [&] {
+        r = s.fac[row];
+        const float y = s.Rr[row];
+        float ratio = easy ? div_by(y, mean, inv) : y / mean;
+        if (clamp) ratio = fmaxf(ratio, 1e-30f);
+        rr = inv_sqrt(ratio);
+    };
+    auto element = [&](int e, float c, float rc) {
+        const float u = ((x[e] * r) * c) * inv_clip;
+        m[e] = fmaf(m[e] * sc, h.beta1, __fmul_rn(h.om_beta1, u));
+        amax = fmaxf(amax, fabsf(m[e]));
+        upd[e] = (m[e] * rr) * rc;
+    };
+    if (V == 8) {      // the columns are a multiple of 8: a lane's elements lie in one row
+        float c[8], rc[8];
+        if (cnt) {
+            row_factors();
+            load_run<8, true>(s.vc, col, 0, 8, c);
+            load_run<8, true>(s.Rc, col, 0, 8, rc);
+        }
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        upd[e] = 0.0f;
-        if (e >= cnt) m[e] = 0.0f;
-        if (e < cnt) {
-            if (row != have) {
-                have = row;
-                r = __ldcg(s.fac + row);
-                const float y = __ldcg(s.Rr + row);
-                float ratio = easy ? div_by(y, mean, inv) : y / mean;
-                if (clamp) ratio = fmaxf(ratio, 1e-30f);
-                rr = inv_sqrt(ratio);
+        for (int e = 0; e < 8; ++e) {
+            upd[e] = 0.0f;
+            if (cnt) element(e, c[e], rc[e]);
+            else m[e] = 0.0f;
+        }
+    } else {
+        int have = -1;      // row the factors r, rr belong to
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            upd[e] = 0.0f;
+            if (e >= cnt) m[e] = 0.0f;
+            if (e < cnt) {
+                if (row != have) { have = row; row_factors(); }
+                element(e, s.vc[col], s.Rc[col]);
+                col += 32;
+                while (col >= C) { col -= C; ++row; }
             }
-            const float u = ((x[e] * r) * __ldcg(s.vc + col)) * inv_clip;
-            m[e] = fmaf(m[e] * sc, h.beta1, __fmul_rn(h.om_beta1, u));
-            amax = fmaxf(amax, fabsf(m[e]));
-            upd[e] = (m[e] * rr) * __ldcg(s.Rc + col);
-            col += STEP;
-            while (col >= C) { col -= C; ++row; }
         }
     }
     const float A = fix_absmax(warp_max(amax)), scale = quant_scale<true>(A);
@@ -917,10 +946,12 @@ __global__ void __launch_bounds__(THREADS, 3) k_step_generic(const __grid_consta
     if (!grid_barrier(l.bar, a.status)) return;
 
     if constexpr (MODE == CAME_MODE_FLAT8) {
+        FlatTensor ft;
         for (int i = first; i < l.n_flats; i += stride) {
             const Work w = l.flats[i];
-            if (a.scr[w.tensor].g_v == 8) phase_apply_flat<TG, TP, 8>(a, hyp, w);
-            else phase_apply_flat<TG, TP, 1>(a, hyp, w);
+            ft.use(a, hyp, w.tensor, lane);
+            if (a.scr[w.tensor].g_v == 8) phase_apply_flat<TG, TP, 8>(a, hyp, w, ft);
+            else phase_apply_flat<TG, TP, 1>(a, hyp, w, ft);
         }
     } else {
         stream<S::COUNT>(a, l.tiles, l.n_tiles, first, stride,
