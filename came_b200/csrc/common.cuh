@@ -333,7 +333,8 @@ __device__ __forceinline__ float col_factor(float v, bool clamp) {
 static __device__ __noinline__ float inv_sqrt_plain(float x) { return 1.0f / sqrtf(x); }      // (out of line: rare, and long)
 __device__ __forceinline__ float inv_sqrt(float x) {
     if (!(x > 1e-30f && x < 1e30f)) return inv_sqrt_plain(x);
-    const float y = rsqrtf(x);
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));      // (x is normal: no scaling of denormals around it)
     return fmaf(0.5f * y, fmaf(-x * y, y, 1.0f), y);
 }
 
