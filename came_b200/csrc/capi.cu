@@ -111,13 +111,14 @@ Context context(const CameTensorDesc* descs, int n) {
     double staged = 0.0;
     for (int i = 0; i < n; ++i)
         if (vec_flags(descs[i]).wide) staged += (double)descs[i].rows * (double)descs[i].cols;
-    Context c{staged < line, 4};
-    // as few bands per item as it takes to give every resident warp of the GPU (24 per SM) two items
+    Context c{staged < line, 16};
+    // As few bands per item as it takes to give every resident warp of the GPU (24 per SM) two items; more than 4, which
+    // only saves column partials and their summation, where every warp (16 per SM) still has eight to even the load out.
     for (; c.bands > 1; c.bands /= 2) {
         int64_t tiles = 0;
         for (int i = 0; i < n; ++i)
             if (c.generic(descs[i])) tiles += generic_tiles(descs[i], c.bands);
-        if (tiles >= 2 * 24 * 148) break;
+        if (tiles >= (c.bands > 4 ? 8 * 16 : 2 * 24) * 148) break;
     }
     return c;
 }
@@ -499,7 +500,15 @@ int came_b200_plan_create(const CameTensorDesc* descs, int n_tensors, void* work
         for (auto& kv : groups) {
             LaunchItem it{};
             it.kernel = KID_GENERIC;
-            it.key = KernelKey{std::get<0>(kv.first), std::get<1>(kv.first), std::get<2>(kv.first), 1};
+            // Two CTAs per SM with 128 registers a thread, or three with 80 (and spills).  More registers win (a bf16 set of
+            // widths 770 / 3083 / 50257: 589 against about 700 us) unless bands are mostly empty: where matrices are narrower than
+            // 64 columns a band is little work behind the same latency, and warps count (rank-16 factors: 196 against 225 us).
+            double elems = 0.0, room = 0.0;
+            for (int i : kv.second.first) {
+                elems += (double)D[i].rows * (double)D[i].cols;
+                room += (double)cdiv(D[i].rows, 16) * (double)cdiv(D[i].cols, generic_tile_cols()) * (16.0 * generic_tile_cols());
+            }
+            it.key = KernelKey{std::get<0>(kv.first), std::get<1>(kv.first), std::get<2>(kv.first), elems < 0.5 * room ? 3 : 2};
             it.bar = (int)plan->launches.size();
             auto list = [&](const std::vector<int>& ids, auto count) {
                 const size_t off = work.size();

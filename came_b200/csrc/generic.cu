@@ -173,8 +173,8 @@ __device__ __forceinline__ float read_mean(const float* blk, int nb, int n, bool
 // ---- a warp's item of a matrix ---------------------------------------------------------------------------------
 constexpr int G_CW = 64;      // columns of an item
 
-template <typename T> struct Size { static constexpr int BYTES = sizeof(T); };
-template <> struct Size<Any> { static constexpr int BYTES = 4; };      // the largest
+template <typename T> struct Size { static constexpr int BYTES = sizeof(T), FIXED = sizeof(T); };
+template <> struct Size<Any> { static constexpr int BYTES = 4, FIXED = 0; };      // the largest; not known
 template <typename T> __device__ __forceinline__ int size_of(int dt) {
     if constexpr (std::is_same<T, Any>::value) return dt == CAME_DT_F32 ? 4 : 2;
     else return (int)sizeof(T);
@@ -214,14 +214,40 @@ struct Item {
     }
 };
 
-// The band's rows of an array of R x C elements of `esz` bytes.  Rows past the end are zero-filled; the columns past the
-// end of a row are the next row's (the reader masks them).  A chunk may begin before the array or end behind it only
-// inside the same 16 bytes, and of the last one only the array's bytes are read.
+// The band's rows of an array of R x C elements of `esz` bytes (ESZ: the same, or 0 for a size known at run time).  Rows
+// past the end are zero-filled; the columns past the end of a row are the next row's (the reader masks them).  A chunk may
+// begin before the array or end behind it only inside the same 16 bytes, and of the last one only the array's bytes are
+// read.  Whole bands away from the array's end need none of those tests, and rows on 16-byte boundaries no ninth chunk and
+// no division (bf16: about 20 instructions a lane instead of 110, of the 250 to 900 that a band takes in a phase).
+template <int ESZ>
 __device__ __forceinline__ void stage_rows(char* dst, int pitch, const void* base, int esz, const Item& it, int lane) {
-    const int nch = G_CW / 16 * esz + 1, rows = min(16, it.R - it.brow), width = min(G_CW, it.C - it.col0) * esz;
-    const uintptr_t b = reinterpret_cast<uintptr_t>(base), end = b + (uintptr_t)((int64_t)it.R * it.C * esz);
+    const uintptr_t b = reinterpret_cast<uintptr_t>(base);
     const uintptr_t first = b + (uintptr_t)(((int64_t)it.brow * it.C + it.col0) * esz);
     const int pitch_g = it.C * esz;      // (rows of a chunk below 2^31 bytes: C < 2^29)
+    if constexpr (ESZ > 0) {
+        constexpr int NCH = G_CW * ESZ / 16;
+        if (it.brow + 16 <= it.R && it.col0 + G_CW <= it.C) {
+            if (((first | (uintptr_t)pitch_g) & 15) == 0) {
+                const int r = lane / NCH, ch = lane % NCH;
+                const char* src = reinterpret_cast<const char*>(first) + (int64_t)r * pitch_g + 16 * ch;
+                char* to = dst + r * pitch + 16 * ch;
+#pragma unroll
+                for (int k = 0; k < NCH / 2; ++k, src += (int64_t)(32 / NCH) * pitch_g, to += 32 / NCH * pitch) cp16(to, src, 16);
+                return;
+            }
+            if (it.brow + 16 < it.R) {      // (a row follows: the last chunk stays inside the array)
+#pragma unroll
+                for (int k = 0; k < (16 * (NCH + 1) + 31) / 32; ++k) {
+                    const int j = lane + 32 * k, r = j / (NCH + 1), ch = j - r * (NCH + 1);
+                    const uintptr_t src = ((first + (uintptr_t)((int64_t)r * pitch_g)) & ~(uintptr_t)15) + 16 * ch;
+                    if (j < 16 * (NCH + 1)) cp16(dst + r * pitch + 16 * ch, reinterpret_cast<const void*>(src), 16);
+                }
+                return;
+            }
+        }
+    }
+    const int nch = G_CW / 16 * esz + 1, rows = min(16, it.R - it.brow), width = min(G_CW, it.C - it.col0) * esz;
+    const uintptr_t end = b + (uintptr_t)((int64_t)it.R * it.C * esz);
     for (int j = lane; j < 16 * nch; j += 32) {
         const int r = j / nch, ch = j - r * nch;
         const uintptr_t row = first + (uintptr_t)((int64_t)r * pitch_g), src = (row & ~(uintptr_t)15) + 16 * ch;
@@ -325,6 +351,11 @@ __device__ __forceinline__ int low_bits(const void* base, const Item& it, int es
     return (int)((reinterpret_cast<uintptr_t>(base) + (uintptr_t)(((int64_t)it.brow * it.C + it.col0) * esz)) & 15);
 }
 
+// Squares of a pair added to a row's sum: V = 8 two chains, V = 1 (one pair a row) one chain in .x
+template <int V> __device__ __forceinline__ u64 add_squares(const u64& y, const u64& sum) {
+    if (V == 8) return fma2(y, y, sum);
+    return pk(fmaf(y.y, y.y, fmaf(y.x, y.x, sum.x)), 0.0f);
+}
 // Sums over a row's lanes of the NR row values a lane holds -> the band's row partials.  Halving butterfly: each step
 // exchanges half of the rows.
 template <int V>
@@ -344,8 +375,11 @@ __device__ __forceinline__ void band_row_sums(const Item& it, float* rowpart, fl
     if ((lane & 1) == 0 && row < it.R) rowpart[(int64_t)it.tc * it.R + row] = v;
 }
 template <int V>
-__device__ __forceinline__ void tile_col_sums(const Item& it, float* colpart, float* acc, int lane) {
+__device__ __forceinline__ void tile_col_sums(const Item& it, float* colpart, const u64* pairs, int lane) {
     float* dst = colpart + (int64_t)it.tr * it.C + it.col0;
+    float acc[Lane<V>::E];
+#pragma unroll
+    for (int e = 0; e < Lane<V>::E / 2; ++e) upk(pairs[e], acc[2 * e], acc[2 * e + 1]);
     if constexpr (V == 8) {
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
@@ -369,37 +403,41 @@ __device__ __forceinline__ float band_row_factor(const Item& it, const float* v,
 }
 // column factors of a lane (0 past the end: those columns then take no part in anything)
 template <int V>
-__device__ __forceinline__ void band_col_factors(const Item& it, const float* c, int lane, float* cf) {
+__device__ __forceinline__ void band_col_factors(const Item& it, const float* c, int lane, u64* cf) {
 #pragma unroll
-    for (int e = 0; e < Lane<V>::E; ++e) {
-        const int col = Lane<V>::col(lane, e);
-        cf[e] = it.col0 + col < it.C ? c[col] : 0.0f;
+    for (int e = 0; e < Lane<V>::E; e += 2) {
+        const int c0 = Lane<V>::col(lane, e), c1 = Lane<V>::col(lane, e + 1);
+        cf[e / 2] = pk(it.col0 + c0 < it.C ? c[c0] : 0.0f, it.col0 + c1 < it.C ? c[c1] : 0.0f);
     }
 }
 
 // ---- S1 -------------------------------------------------------------------------------------------------------
 template <typename TG, int V>
-__device__ __forceinline__ void band_sq(const StepArgs& a, const Item& it, const char* st, int pitch, float* colacc) {
+__device__ __forceinline__ void band_sq(const StepArgs& a, const Item& it, const char* st, int pitch, u64* colacc) {
     constexpr int NR = Lane<V>::NR, E = Lane<V>::E;
     const CameTensorDesc& d = a.descs[it.tensor];
     const int lane = threadIdx.x & 31, esz = size_of<TG>(d.g_dtype), dt = d.g_dtype;
     const int low = low_bits(d.g, it, esz), grow = it.C * esz;
     float rs[NR];
+    bool in[V == 8 ? 1 : 2];      // V = 8: the columns are a multiple of 8, a lane's 8 lie inside or outside together
+#pragma unroll
+    for (int q = 0; q < (V == 8 ? 1 : 2); ++q) in[q] = it.col0 + Lane<V>::col(lane, q) < it.C;
     if (it.k == 0)
 #pragma unroll
-        for (int e = 0; e < E; ++e) colacc[e] = 0.0f;
+        for (int e = 0; e < E / 2; ++e) colacc[e] = F2ZERO;
 #pragma unroll
     for (int i = 0; i < NR; ++i) {
         const int r = Lane<V>::row(lane, i);
         float x[E];
         read_row<V, TG>(st, pitch, dt, (low + r * grow) & 15, r, lane, x);
-        rs[i] = 0.0f;
+        u64 sum = F2ZERO;
 #pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const float y = it.col0 + Lane<V>::col(lane, e) < it.C ? x[e] : 0.0f;
-            rs[i] = fmaf(y, y, rs[i]);
-            colacc[e] = fmaf(y, y, colacc[e]);
+        for (int e = 0; e < E; e += 2) {
+            const u64 y = pk(in[0] ? x[e] : 0.0f, in[V == 8 ? 0 : 1] ? x[e + 1] : 0.0f);
+            sum = add_squares<V>(y, sum);
+            colacc[e / 2] = fma2(y, y, colacc[e / 2]);
         }
+        rs[i] = V == 8 ? sum.x + sum.y : sum.x;
     }
     const Scratch& s = a.scr[it.tensor];
     float* colpart = s.colpart;
@@ -420,20 +458,21 @@ __device__ __forceinline__ void band_clip(const StepArgs& a, const Item& it, con
         mean = read_mean(s.rowblk, s.nbR, it.R, d.flags & CAME_F_SQ_FIX, d.flags & CAME_F_SQ_CLAMP, lane);
     }
     const float f = band_row_factor(it, reinterpret_cast<const float*>(st + S::OFF_V), mean, d.flags & CAME_F_SQ_CLAMP, 1.0f, lane);
-    float cf[E];
+    u64 cf[E / 2], sum = F2ZERO;
     band_col_factors<V>(it, reinterpret_cast<const float*>(st + S::OFF_C), lane, cf);
 #pragma unroll
     for (int i = 0; i < NR; ++i) {
         const int r = Lane<V>::row(lane, i);
-        const float rf = __shfl_sync(0xffffffffu, f, r);
+        const u64 rf = splat(__shfl_sync(0xffffffffu, f, r));
         float x[E];
         read_row<V, TG>(st, S::PA, dt, (low + r * grow) & 15, r, lane, x);
 #pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const float u = (x[e] * rf) * cf[e];
-            acc = fmaf(u, u, acc);
+        for (int e = 0; e < E; e += 2) {
+            const u64 u = mul2(mul2(pk(x[e], x[e + 1]), rf), cf[e / 2]);
+            sum = fma2(u, u, sum);
         }
     }
+    acc += sum.x + sum.y;
     if (s.fac && it.tc == 0 && lane < 16 && it.brow + lane < it.R) s.fac[it.brow + lane] = f;      // for the flat apply phase
     if (it.k == it.nb - 1) leave_partial(s.spart, s.counters, it.tile, s.tiles_r * s.tiles_c, warp_sum(acc), lane);
 }
@@ -448,7 +487,7 @@ __device__ __forceinline__ float read_inv_clip(const Scratch& s, const CameHyper
 // tile layout (came_kernels.cu:2584-2683): m re-quantised per 16 x 16 tile; fp32 (came_kernels.cu:2307-2342): m written;
 // flat layout: nothing written, the apply phase forms m again (came_kernels.cu:2246-2305 keeps it in fp32 scratch)
 template <typename TG, int MODE, int V>
-__device__ __forceinline__ void band_moment(const StepArgs& a, const CameHyper* hyp, const Item& it, const char* st, float* colacc, float& mean,
+__device__ __forceinline__ void band_moment(const StepArgs& a, const CameHyper* hyp, const Item& it, const char* st, u64* colacc, float& mean,
                                             float& inv_clip) {
     using S = Stage<TG, MODE>;
     constexpr int NR = Lane<V>::NR, E = Lane<V>::E;
@@ -467,14 +506,17 @@ __device__ __forceinline__ void band_moment(const StepArgs& a, const CameHyper* 
     float* const absmax = d.m_absmax;
     float* const rowpart = s.rowpart;
     float* const colpart = s.colpart;
-    float cf[E], m[NR][E], rs[NR], amax[V == 8 ? 1 : 2], sc[V == 8 ? 1 : 2];
-    bool in[E];
+    u64 cf[E / 2];
+    float m[NR][E], rs[NR], amax[V == 8 ? 1 : 2], sc[V == 8 ? 1 : 2];
+    bool in[V == 8 ? 1 : 2];
     band_col_factors<V>(it, reinterpret_cast<const float*>(st + S::OFF_C), lane, cf);
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-        in[e] = it.col0 + Lane<V>::col(lane, e) < it.C;
-        if (it.k == 0) colacc[e] = 0.0f;
-    }
+    for (int q = 0; q < (V == 8 ? 1 : 2); ++q) in[q] = it.col0 + Lane<V>::col(lane, q) < it.C;
+    if (it.k == 0)
+#pragma unroll
+        for (int e = 0; e < E / 2; ++e) colacc[e] = F2ZERO;
+    const u64 b2 = splat(beta1), o2 = splat(om1), clip2 = splat(inv_clip);
+    const float dq = MODE == CAME_MODE_FLAT8 ? xs[lane] / QMAX_I8 : 0.0f;      // of the two blocks of row lane / 2
 #pragma unroll
     for (int q = 0; q < (V == 8 ? 1 : 2); ++q) {
         amax[q] = 0.0f;
@@ -487,28 +529,33 @@ __device__ __forceinline__ void band_moment(const StepArgs& a, const CameHyper* 
 #pragma unroll
     for (int i = 0; i < NR; ++i) {
         const int r = Lane<V>::row(lane, i);
-        const float rf = __shfl_sync(0xffffffffu, f, r);
+        const u64 rf = splat(__shfl_sync(0xffffffffu, f, r));
         float x[E];
         read_row<V, TG>(st, S::PA, dt, (low + r * grow) & 15, r, lane, x);
         if constexpr (MODE == CAME_MODE_FP32) read_row<V, float>(st + S::OFF_M, S::PM, 0, (mlow + r * mgrow) & 15, r, lane, m[i]);
         else read_codes<V>(st + S::OFF_M, S::PM, (mlow + r * mgrow) & 15, r, lane, m[i]);
         float fs[2];
-        if (MODE == CAME_MODE_FLAT8) { fs[0] = xs[2 * r] / QMAX_I8; fs[1] = xs[2 * r + 1] / QMAX_I8; }
+        if (MODE == CAME_MODE_FLAT8) { fs[0] = __shfl_sync(0xffffffffu, dq, 2 * r); fs[1] = __shfl_sync(0xffffffffu, dq, 2 * r + 1); }
         const uint32_t o8 = MODE == CAME_MODE_FLAT8 ? (uint32_t)(((uint32_t)(it.brow + r) * (uint32_t)it.C + (uint32_t)it.col0) & 255u) : 0u;
-        rs[i] = 0.0f;
+        u64 sum = F2ZERO;
 #pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const float u = ((x[e] * rf) * cf[e]) * inv_clip;
-            float mo = m[i][e];
-            if (MODE == CAME_MODE_TILE8) mo *= sc[V == 8 ? 0 : e & 1];
-            else if (MODE == CAME_MODE_FLAT8) mo *= !in[e] ? 0.0f : o8 + Lane<V>::col(lane, e) < 256u ? fs[0] : fs[1];
-            else if (!in[e]) mo = 0.0f;
-            const float mn = fmaf(mo, beta1, __fmul_rn(om1, u)), df = u - mn;      // the reference's order
-            rs[i] = fmaf(df, df, rs[i]);
-            colacc[e] = fmaf(df, df, colacc[e]);
-            m[i][e] = mn;
-            if (MODE == CAME_MODE_TILE8) amax[V == 8 ? 0 : e & 1] = fmaxf(amax[V == 8 ? 0 : e & 1], fabsf(mn));
+        for (int e = 0; e < E; e += 2) {
+            const u64 u = mul2(mul2(mul2(pk(x[e], x[e + 1]), rf), cf[e / 2]), clip2);
+            u64 mo = pk(m[i][e], m[i][e + 1]);
+            constexpr int Q1 = V == 8 ? 0 : 1;      // the second of a pair: V = 1 another tile, 32 columns on
+            if (MODE == CAME_MODE_TILE8) mo = mul2(mo, pk(sc[0], sc[Q1]));
+            else if (MODE == CAME_MODE_FLAT8) {      // V = 8: a lane's columns lie in one block
+                const uint32_t c0 = Lane<V>::col(lane, V == 8 ? 0 : e), c1 = Lane<V>::col(lane, V == 8 ? 0 : e + 1);
+                mo = mul2(mo, pk(!in[0] ? 0.0f : o8 + c0 < 256u ? fs[0] : fs[1], !in[Q1] ? 0.0f : o8 + c1 < 256u ? fs[0] : fs[1]));
+            }
+            else { if (!in[0]) mo.x = 0.0f; if (!in[Q1]) mo.y = 0.0f; }
+            const u64 mn = fma2(mo, b2, mul2(o2, u)), df = sub2(u, mn);      // the reference's order
+            sum = add_squares<V>(df, sum);
+            colacc[e / 2] = fma2(df, df, colacc[e / 2]);
+            m[i][e] = mn.x; m[i][e + 1] = mn.y;
+            if (MODE == CAME_MODE_TILE8) { amax[0] = fmaxf(amax[0], fabsf(mn.x)); amax[Q1] = fmaxf(amax[Q1], fabsf(mn.y)); }
         }
+        rs[i] = V == 8 ? sum.x + sum.y : sum.x;
     }
     const int64_t at = ((int64_t)it.brow * it.C + it.col0);
     const int live = it.R - it.brow;
@@ -548,7 +595,10 @@ __device__ __forceinline__ void band_moment(const StepArgs& a, const CameHyper* 
             int8_t* dst = reinterpret_cast<int8_t*>(m_base) + at + (int64_t)r * it.C + Lane<V>::col(lane, 0);
             uint32_t y[E];      // the low byte of m * (127 / A) + 1.5 * 2^23 is the code (see fast_tile8.cu)
 #pragma unroll
-            for (int e = 0; e < E; ++e) y[e] = __float_as_uint(fmaf(m[i][e], q127[V == 8 ? 0 : e & 1], ROUND_MAGIC));
+            for (int e = 0; e < E; e += 2) {
+                const u64 t = fma2(pk(m[i][e], m[i][e + 1]), pk(q127[0], q127[V == 8 ? 0 : 1]), splat(ROUND_MAGIC));
+                y[e] = __float_as_uint(t.x); y[e + 1] = __float_as_uint(t.y);
+            }
             if constexpr (V == 8) {
                 if (r < live && in[0])
                     *reinterpret_cast<uint2*>(dst) = make_uint2(__byte_perm(__byte_perm(y[0], y[1], 0x0040u), __byte_perm(y[2], y[3], 0x0040u), 0x5410u),
@@ -595,19 +645,22 @@ __device__ __forceinline__ void band_apply(const StepArgs& a, const CameHyper* h
     if (it.k == 0) mean = read_mean(s.rowblk2, s.nbR, it.R, d.flags & CAME_F_RESROW_FIX, d.flags & CAME_F_RESROW_CLAMP, lane);
     const float f = band_row_factor(it, reinterpret_cast<const float*>(st + S::OFF_V), mean, d.flags & CAME_F_RESROW_CLAMP, 1.0f, lane);
     const float* xs = reinterpret_cast<const float*>(st + S::OFF_X);
-    float cf[E], sc[V == 8 ? 1 : 2];
-    bool in[E];
+    u64 cf[E / 2];
+    float sc[V == 8 ? 1 : 2];
+    bool in[V == 8 ? 1 : 2];
     band_col_factors<V>(it, reinterpret_cast<const float*>(st + S::OFF_C), lane, cf);
 #pragma unroll
-    for (int e = 0; e < E; ++e) in[e] = it.col0 + Lane<V>::col(lane, e) < it.C;
-#pragma unroll
     for (int q = 0; q < (V == 8 ? 1 : 2); ++q) {
+        in[q] = it.col0 + Lane<V>::col(lane, q) < it.C;
         sc[q] = 1.0f;
         if (MODE == CAME_MODE_TILE8) {
             const float A = in[q] ? xs[V == 8 ? (lane & 7) >> 1 : (lane >> 4) + 2 * q] : 0.0f;
             sc[q] = A > 0.0f ? A / QMAX_I8 : 0.0f;
         }
     }
+    // decay as one packed operation k p + base (apply_step's forms: 0 and 2 multiply, 1 and 3 subtract; x + -0 is x)
+    const bool subtract = wd & 1;
+    const u64 k2 = splat(subtract ? -h.wd_lr : wd == 2 ? h.decay_mul : 1.0f), lr2 = splat(-h.lr);
     const Buf<TP> p(d.p, dt);
     const int64_t at = (int64_t)it.brow * it.C + it.col0 + Lane<V>::col(lane, 0);
     const int live = it.R - it.brow, n_push = a.n_push;
@@ -620,7 +673,20 @@ __device__ __forceinline__ void band_apply(const StepArgs& a, const CameHyper* h
         if constexpr (MODE == CAME_MODE_FP32) read_row<V, float>(st + S::OFF_M, S::PM, 0, (mlow + r * mgrow) & 15, r, lane, m);
         else read_codes<V>(st + S::OFF_M, S::PM, (mlow + r * mgrow) & 15, r, lane, m);
 #pragma unroll
-        for (int e = 0; e < E; ++e) x[e] = g_apply_one(p, x[e], (m[e] * (rf * sc[V == 8 ? 0 : e & 1])) * cf[e], h, wd);
+        for (int e = 0; e < E; e += 2) {
+            const u64 pv = pk(x[e], x[e + 1]);
+            const u64 t = fma2(k2, pv, subtract ? pv : splat(-0.0f));
+            x[e] = t.x; x[e + 1] = t.y;
+        }
+        if (wd >= 2)
+#pragma unroll
+            for (int e = 0; e < E; ++e) x[e] = p.round(x[e]);
+#pragma unroll
+        for (int e = 0; e < E; e += 2) {
+            const u64 upd = mul2(mul2(pk(m[e], m[e + 1]), pk(rf * sc[0], rf * sc[V == 8 ? 0 : 1])), cf[e / 2]);
+            const u64 t = fma2(lr2, upd, pk(x[e], x[e + 1]));
+            x[e] = t.x; x[e + 1] = t.y;
+        }
         const int64_t o = at + (int64_t)r * it.C;
         if (r < live) {
             if constexpr (V == 8) {
@@ -641,7 +707,31 @@ __device__ __forceinline__ void band_apply(const StepArgs& a, const CameHyper* h
 }
 
 // flat layout: a warp owns a block of 256 consecutive elements, whatever rows they belong to (the un-quantised momentum
-// feeds the update: came_kernels.cu:2246-2305, 2487-2511)
+// feeds the update: came_kernels.cu:2246-2305, 2487-2511).  The blocks of g, p and the codes come to the warp's shared
+// memory, in the room its bands had, some blocks ahead; buffers off the 16-byte boundary are read where they are.
+template <typename T, int MODE> struct FlatSlot {
+    static constexpr int ESZ = Size<T>::BYTES, OFF_P = QBLOCK * ESZ, OFF_M = 2 * OFF_P, OFF_X = OFF_M + QBLOCK, BYTES = OFF_X + 16;
+    static constexpr int ROOM = Stage<T, MODE>::COUNT * Stage<T, MODE>::BYTES / BYTES, COUNT = ROOM < 4 ? ROOM : 4;
+    static_assert(COUNT >= 2, "a block is computed while the next is on its way");
+};
+__device__ __forceinline__ bool flat_staged(const CameTensorDesc& d) {
+    return ((reinterpret_cast<uintptr_t>(d.g) | reinterpret_cast<uintptr_t>(d.p) | reinterpret_cast<uintptr_t>(d.m)) & 15) == 0;
+}
+template <typename TG, typename TP, typename S>
+__device__ __forceinline__ void issue_flat(const StepArgs& a, const Work& w, char* slot, int lane) {
+    const CameTensorDesc& d = a.descs[w.tensor];
+    if (!flat_staged(d)) return;
+    const int64_t i0 = (int64_t)w.tile * QBLOCK;
+    const int cnt = (int)min((int64_t)QBLOCK, d.rows * d.cols - i0);
+    auto rows = [&](char* dst, const void* base, int esz) {
+        const char* src = reinterpret_cast<const char*>(base) + i0 * esz;
+        for (int j = 16 * lane; j < cnt * esz; j += 512) cp16(dst + j, src + j, min(16, cnt * esz - j));
+    };
+    rows(slot, d.g, size_of<TG>(d.g_dtype));
+    rows(slot + S::OFF_P, d.p, size_of<TP>(d.p_dtype));
+    rows(slot + S::OFF_M, d.m, 1);
+    if (lane == 0) cp4(slot + S::OFF_X, d.m_absmax + w.tile);
+}
 struct FlatTensor {      // what a warp's blocks of one tensor share: formed once, not per block of 8 elements per lane
     int tensor = -1;
     float inv_clip, mean;
@@ -654,28 +744,33 @@ struct FlatTensor {      // what a warp's blocks of one tensor share: formed onc
         mean = read_mean(s.rowblk2, s.nbR, (int)d.rows, d.flags & CAME_F_RESROW_FIX, d.flags & CAME_F_RESROW_CLAMP, lane);
     }
 };
-template <typename TG, typename TP, int V>
-__device__ __forceinline__ void phase_apply_flat(const StepArgs& a, const CameHyper* hyp, const Work& w, const FlatTensor& ft) {
+template <typename TG, typename TP, typename S, int V>
+__device__ __forceinline__ void phase_apply_flat(const StepArgs& a, const CameHyper* hyp, const Work& w, const FlatTensor& ft, const char* slot) {
     const CameTensorDesc d = a.descs[w.tensor];
     const Scratch s = a.scr[w.tensor];
     const CameHyper h = hyp[d.group];
-    const Buf<TG> g(d.g, d.g_dtype);
-    const Buf<TP> p(d.p, d.p_dtype);
     const int lane = threadIdx.x & 31, C = (int)d.cols, blk = w.tile;
-    const int64_t n = d.rows * d.cols;
+    const int64_t n = d.rows * d.cols, b0 = (int64_t)blk * QBLOCK;
     const int wd = wd_form(h, d.flags);
     const float inv_clip = ft.inv_clip, mean = ft.mean, inv = 1.0f / mean;
     const bool clamp = d.flags & CAME_F_RESROW_CLAMP, easy = mean > 1e-30f && mean < 1e30f;
     int8_t* mq = reinterpret_cast<int8_t*>(d.m);
-    const int64_t i0 = (int64_t)blk * QBLOCK + (V == 8 ? 8 * lane : lane);
+    const Buf<TP> p(d.p, d.p_dtype);
+    // the block's elements: in the slot, or where they lie (V = 8: always in the slot)
+    const bool staged = V == 8 || flat_staged(d);
+    const Buf<TG> gs(staged ? slot : reinterpret_cast<const char*>(d.g) + b0 * size_of<TG>(d.g_dtype), d.g_dtype);
+    const Buf<TP> ps(staged ? slot + S::OFF_P : reinterpret_cast<const char*>(d.p) + b0 * size_of<TP>(d.p_dtype), d.p_dtype);
+    const int8_t* ms = staged ? reinterpret_cast<const int8_t*>(slot + S::OFF_M) : mq + b0;
+    const int j0 = V == 8 ? 8 * lane : lane;
+    const int64_t i0 = b0 + j0;
     float x[8], m[8], pv[8];
     int cnt;      // elements of this lane (they end where the tensor does)
     if (V == 8) {
         cnt = i0 >= n ? 0 : 8;      // n is a multiple of 8
         if (cnt) {
-            g.get8(i0, x);
-            p.get8(i0, pv);
-            const uint2 r = *reinterpret_cast<const uint2*>(mq + i0);
+            gs.get8(j0, x);
+            ps.get8(j0, pv);
+            const uint2 r = *reinterpret_cast<const uint2*>(ms + j0);
             const uint32_t y[2] = {r.x ^ 0x80808080u, r.y ^ 0x80808080u};
 #pragma unroll
             for (int e = 0; e < 8; e += 2) { const u64 f = codes_to_f2(y[e >> 2], e & 3); m[e] = f.x; m[e + 1] = f.y; }
@@ -684,9 +779,9 @@ __device__ __forceinline__ void phase_apply_flat(const StepArgs& a, const CameHy
         cnt = i0 >= n ? 0 : (int)min((int64_t)8, (n - i0 + 31) >> 5);
 #pragma unroll
         for (int e = 0; e < 8; ++e)
-            if (e < cnt) { x[e] = g.get(i0 + 32 * e); pv[e] = p.get(i0 + 32 * e); m[e] = (float)mq[i0 + 32 * e]; }
+            if (e < cnt) { x[e] = gs.get(j0 + 32 * e); pv[e] = ps.get(j0 + 32 * e); m[e] = (float)ms[j0 + 32 * e]; }
     }
-    const float sc = __ldcg(d.m_absmax + blk) / QMAX_I8;
+    const float sc = (staged ? *reinterpret_cast<const float*>(slot + S::OFF_X) : __ldcg(d.m_absmax + blk)) / QMAX_I8;
     int row, col;
     if (n < 0x7fffffff) { row = (int)((uint32_t)i0 / (uint32_t)C); col = (int)i0 - row * C; }
     else { row = (int)(i0 / C); col = (int)(i0 - (int64_t)row * C); }
@@ -780,7 +875,9 @@ __device__ __forceinline__ void phase_finalize(const StepArgs& a, const CameHype
     float acc[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) acc[e] = 0.0f;
-#pragma unroll 2
+    // (32 loads in flight: the 785 partials of a column of a 50257-row matrix are 98 steps for the one CTA that adds them,
+    // while the other CTAs wait at the next barrier)
+#pragma unroll 4
     for (int t = warp; t < parts; t += G_WARPS)
 #pragma unroll
         for (int e = 0; e < 8; ++e)
@@ -880,8 +977,8 @@ struct GenericArgs {
     CameHyper hyp[GENERIC_MAX_HYP];
 };
 
-template <typename TG, typename TP, int MODE>
-__global__ void __launch_bounds__(THREADS, 3) k_step_generic(const __grid_constant__ GenericArgs ga) {
+template <typename TG, typename TP, int MODE, int CTAS>
+__global__ void __launch_bounds__(THREADS, CTAS) k_step_generic(const __grid_constant__ GenericArgs ga) {
     using S = Stage<TG, MODE>;
     extern __shared__ __align__(128) char g_smem[];
     __shared__ GShared sh;
@@ -894,13 +991,13 @@ __global__ void __launch_bounds__(THREADS, 3) k_step_generic(const __grid_consta
     // warp items: across the SMs first, then over the warps; CTA items of 1-D tensors: from the last CTA on, which comes
     // last in the deal of the others
     const int first = warp * gridDim.x + blockIdx.x, stride = G_WARPS * gridDim.x, back = gridDim.x - 1 - blockIdx.x;
-    float colacc[8];
+    u64 colacc[4];
 
     for (int i = back; i < l.n_ones; i += gridDim.x) phase_vector_sq<TG>(a, hyp, l.ones[i], sh);
     stream<S::COUNT>(a, l.tiles, l.n_tiles, first, stride,
         [&](const Item& it, int k) {
             const CameTensorDesc& d = a.descs[it.tensor];
-            stage_rows(stage(k), S::PA, d.g, size_of<TG>(d.g_dtype), it, lane);
+            stage_rows<Size<TG>::FIXED>(stage(k), S::PA, d.g, size_of<TG>(d.g_dtype), it, lane);
         },
         [&](const Item& it, int k) {
             if (it.v8) band_sq<TG, 8>(a, it, stage(k), S::PA, colacc);
@@ -919,7 +1016,7 @@ __global__ void __launch_bounds__(THREADS, 3) k_step_generic(const __grid_consta
             const CameTensorDesc& d = a.descs[it.tensor];
             const Scratch& s = a.scr[it.tensor];
             stage_vectors(stage(k), S::OFF_V, S::OFF_C, s.vr, s.vc, it, lane);
-            stage_rows(stage(k), S::PA, d.g, size_of<TG>(d.g_dtype), it, lane);
+            stage_rows<Size<TG>::FIXED>(stage(k), S::PA, d.g, size_of<TG>(d.g_dtype), it, lane);
         },
         [&](const Item& it, int k) {
             if (it.v8) band_clip<TG, S, 8>(a, it, stage(k), acc, mean);
@@ -933,8 +1030,8 @@ __global__ void __launch_bounds__(THREADS, 3) k_step_generic(const __grid_consta
             const Scratch& s = a.scr[it.tensor];
             stage_vectors(stage(k), S::OFF_V, S::OFF_C, s.vr, s.vc, it, lane);
             stage_absmax<MODE>(stage(k) + S::OFF_X, d.m_absmax, it, lane);
-            stage_rows(stage(k), S::PA, d.g, size_of<TG>(d.g_dtype), it, lane);
-            stage_rows(stage(k) + S::OFF_M, S::PM, d.m, MODE == CAME_MODE_FP32 ? 4 : 1, it, lane);
+            stage_rows<Size<TG>::FIXED>(stage(k), S::PA, d.g, size_of<TG>(d.g_dtype), it, lane);
+            stage_rows<(MODE == CAME_MODE_FP32 ? 4 : 1)>(stage(k) + S::OFF_M, S::PM, d.m, MODE == CAME_MODE_FP32 ? 4 : 1, it, lane);
         },
         [&](const Item& it, int k) {
             if (it.v8) band_moment<TG, MODE, 8>(a, hyp, it, stage(k), colacc, mean, inv_clip);
@@ -946,13 +1043,37 @@ __global__ void __launch_bounds__(THREADS, 3) k_step_generic(const __grid_consta
     if (!grid_barrier(l.bar, a.status)) return;
 
     if constexpr (MODE == CAME_MODE_FLAT8) {
+        using F = FlatSlot<TG, MODE>;
         FlatTensor ft;
-        for (int i = first; i < l.n_flats; i += stride) {
-            const Work w = l.flats[i];
-            ft.use(a, hyp, w.tensor, lane);
-            if (a.scr[w.tensor].g_v == 8) phase_apply_flat<TG, TP, 8>(a, hyp, w, ft);
-            else phase_apply_flat<TG, TP, 1>(a, hyp, w, ft);
+        Work ahead[F::COUNT];      // the blocks under way, the next to compute first
+#pragma unroll
+        for (int k = 0; k < F::COUNT - 1; ++k) {
+            const int i = first + k * stride;
+            if (i < l.n_flats) {
+                ahead[k] = l.flats[i];
+                issue_flat<TG, TP, F>(a, ahead[k], stages + k * F::BYTES, lane);
+            }
+            cp_commit();
         }
+        for (int i = first, slot = 0; i < l.n_flats; i += stride) {
+            const int j = i + (F::COUNT - 1) * stride, free = slot == 0 ? F::COUNT - 1 : slot - 1;      // (of the block before)
+            if (j < l.n_flats) {
+                ahead[F::COUNT - 1] = l.flats[j];
+                issue_flat<TG, TP, F>(a, ahead[F::COUNT - 1], stages + free * F::BYTES, lane);
+            }
+            cp_commit();
+            const Work w = ahead[0];
+            ft.use(a, hyp, w.tensor, lane);
+            cp_wait<F::COUNT - 1>();
+            __syncwarp();
+            if (a.scr[w.tensor].g_v == 8) phase_apply_flat<TG, TP, F, 8>(a, hyp, w, ft, stages + slot * F::BYTES);
+            else phase_apply_flat<TG, TP, F, 1>(a, hyp, w, ft, stages + slot * F::BYTES);
+            __syncwarp();      // the slot is read before it is filled again
+#pragma unroll
+            for (int k = 0; k < F::COUNT - 1; ++k) ahead[k] = ahead[k + 1];
+            if (++slot == F::COUNT) slot = 0;
+        }
+        cp_wait<0>();
     } else {
         stream<S::COUNT>(a, l.tiles, l.n_tiles, first, stride,
             [&](const Item& it, int k) {
@@ -960,8 +1081,8 @@ __global__ void __launch_bounds__(THREADS, 3) k_step_generic(const __grid_consta
                 const Scratch& s = a.scr[it.tensor];
                 stage_vectors(stage(k), S::OFF_V, S::OFF_C, s.Rr, s.Rc, it, lane);
                 stage_absmax<MODE>(stage(k) + S::OFF_X, d.m_absmax, it, lane);
-                stage_rows(stage(k), S::PA, d.p, size_of<TP>(d.p_dtype), it, lane);
-                stage_rows(stage(k) + S::OFF_M, S::PM, d.m, MODE == CAME_MODE_FP32 ? 4 : 1, it, lane);
+                stage_rows<Size<TP>::FIXED>(stage(k), S::PA, d.p, size_of<TP>(d.p_dtype), it, lane);
+                stage_rows<(MODE == CAME_MODE_FP32 ? 4 : 1)>(stage(k) + S::OFF_M, S::PM, d.m, MODE == CAME_MODE_FP32 ? 4 : 1, it, lane);
             },
             [&](const Item& it, int k) {
                 if (it.v8) band_apply<TP, MODE, 8>(a, hyp, it, stage(k), mean);
@@ -974,21 +1095,21 @@ struct GenericKernel {
     void (*fn)(const GenericArgs);
     int smem;
 };
-template <typename TG, typename TP, int MODE> GenericKernel generic_kernel() {
-    return {k_step_generic<TG, TP, MODE>, G_WARPS * Stage<TG, MODE>::COUNT * Stage<TG, MODE>::BYTES};
+template <typename TG, typename TP, int MODE> GenericKernel generic_kernel(int ctas) {
+    return {ctas == 2 ? k_step_generic<TG, TP, MODE, 2> : k_step_generic<TG, TP, MODE, 3>, G_WARPS * Stage<TG, MODE>::COUNT * Stage<TG, MODE>::BYTES};
 }
-template <typename TG, typename TP> GenericKernel pick_mode(int mode) {
+template <typename TG, typename TP> GenericKernel pick_mode(int mode, int ctas) {
     switch (mode) {
-        case CAME_MODE_FP32: return generic_kernel<TG, TP, CAME_MODE_FP32>();
-        case CAME_MODE_TILE8: return generic_kernel<TG, TP, CAME_MODE_TILE8>();
-        default: return generic_kernel<TG, TP, CAME_MODE_FLAT8>();
+        case CAME_MODE_FP32: return generic_kernel<TG, TP, CAME_MODE_FP32>(ctas);
+        case CAME_MODE_TILE8: return generic_kernel<TG, TP, CAME_MODE_TILE8>(ctas);
+        default: return generic_kernel<TG, TP, CAME_MODE_FLAT8>(ctas);
     }
 }
-GenericKernel pick_generic(int g, int p, int mode) {
-    if (g != p) return pick_mode<Any, Any>(mode);
-    if (g == CAME_DT_F32) return pick_mode<float, float>(mode);
-    if (g == CAME_DT_F16) return pick_mode<__half, __half>(mode);
-    return pick_mode<__nv_bfloat16, __nv_bfloat16>(mode);
+GenericKernel pick_generic(int g, int p, int mode, int ctas) {
+    if (g != p) return pick_mode<Any, Any>(mode, ctas);
+    if (g == CAME_DT_F32) return pick_mode<float, float>(mode, ctas);
+    if (g == CAME_DT_F16) return pick_mode<__half, __half>(mode, ctas);
+    return pick_mode<__nv_bfloat16, __nv_bfloat16>(mode, ctas);
 }
 
 }  // namespace
@@ -997,7 +1118,7 @@ int generic_tile_cols() { return G_CW; }
 
 cudaError_t launch_generic(const KernelKey& key, const StepArgs& a, const CameHyper* host_hyp, int n_hyp, const GenericLists& l,
                            cudaStream_t st) {
-    const GenericKernel kernel = pick_generic(key.g_dtype, key.p_dtype, key.mode);
+    const GenericKernel kernel = pick_generic(key.g_dtype, key.p_dtype, key.mode, key.variant);
     const void* fn = reinterpret_cast<const void*>(kernel.fn);
     static std::mutex mu;
     static std::map<std::pair<int, const void*>, int> cache;      // CTAs an SM holds, per device and kernel

@@ -27,7 +27,7 @@ struct KernelKey {
     int g_dtype;
     int p_dtype;
     int mode;
-    int variant;   // 1: 16-byte vector loads; 2: shared-memory staged path (N-D tensors: small matrices; 3: 3 x 3 and 1 x 1)
+    int variant;   // 1: 16-byte vector loads; 2: shared-memory staged path (whole-step kernel: its CTAs per SM; N-D tensors: small matrices; 3: 3 x 3 and 1 x 1)
 };
 
 enum KernelId {
