@@ -734,7 +734,7 @@ __device__ __forceinline__ void issue_flat(const StepArgs& a, const Work& w, cha
 }
 struct FlatTensor {      // what a warp's blocks of one tensor share: formed once, not per block of 8 elements per lane
     int tensor = -1;
-    float inv_clip, mean;
+    float inv_clip, mean, inv;
     __device__ __forceinline__ void use(const StepArgs& a, const CameHyper* hyp, int t, int lane) {
         if (t == tensor) return;
         tensor = t;
@@ -742,6 +742,7 @@ struct FlatTensor {      // what a warp's blocks of one tensor share: formed onc
         const Scratch& s = a.scr[t];
         inv_clip = read_inv_clip(s, hyp[d.group], d.rows * d.cols, lane);
         mean = read_mean(s.rowblk2, s.nbR, (int)d.rows, d.flags & CAME_F_RESROW_FIX, d.flags & CAME_F_RESROW_CLAMP, lane);
+        inv = 1.0f / mean;
     }
 };
 template <typename TG, typename TP, typename S, int V>
@@ -752,7 +753,7 @@ __device__ __forceinline__ void phase_apply_flat(const StepArgs& a, const CameHy
     const int lane = threadIdx.x & 31, C = (int)d.cols, blk = w.tile;
     const int64_t n = d.rows * d.cols, b0 = (int64_t)blk * QBLOCK;
     const int wd = wd_form(h, d.flags);
-    const float inv_clip = ft.inv_clip, mean = ft.mean, inv = 1.0f / mean;
+    const float inv_clip = ft.inv_clip, mean = ft.mean, inv = ft.inv;
     const bool clamp = d.flags & CAME_F_RESROW_CLAMP, easy = mean > 1e-30f && mean < 1e30f;
     int8_t* mq = reinterpret_cast<int8_t*>(d.m);
     const Buf<TP> p(d.p, d.p_dtype);
@@ -782,58 +783,116 @@ __device__ __forceinline__ void phase_apply_flat(const StepArgs& a, const CameHy
             if (e < cnt) { x[e] = gs.get(j0 + 32 * e); pv[e] = ps.get(j0 + 32 * e); m[e] = (float)ms[j0 + 32 * e]; }
     }
     const float sc = (staged ? *reinterpret_cast<const float*>(slot + S::OFF_X) : __ldcg(d.m_absmax + blk)) / QMAX_I8;
-    int row, col;
-    if (n < 0x7fffffff) { row = (int)((uint32_t)i0 / (uint32_t)C); col = (int)i0 - row * C; }
-    else { row = (int)(i0 / C); col = (int)(i0 - (int64_t)row * C); }
     // (plain loads of the factors: the grid barriers order them behind other SMs' stores, and lines are used many times)
-    float upd[8], amax = 0.0f, r = 0.0f, rr = 0.0f;
-    auto row_factors = [&] {
+    float upd[8], amax = 0.0f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        upd[e] = 0.0f;
+        if (e >= cnt) { x[e] = 0.0f; m[e] = 0.0f; pv[e] = 0.0f; }
+    }
+    auto row_factors = [&](int row, float& r, float& rr) {
         r = s.fac[row];
         const float y = s.Rr[row];
         float ratio = easy ? div_by(y, mean, inv) : y / mean;
         if (clamp) ratio = fmaxf(ratio, 1e-30f);
         rr = inv_sqrt(ratio);
     };
-    auto element = [&](int e, float c, float rc) {
-        const float u = ((x[e] * r) * c) * inv_clip;
-        m[e] = fmaf(m[e] * sc, h.beta1, __fmul_rn(h.om_beta1, u));
-        amax = fmaxf(amax, fabsf(m[e]));
-        upd[e] = (m[e] * rr) * rc;
+    // elements e and e + 1 (past the tensor's end g = m = 0 and the factors are 0: no part in anything)
+    const u64 clip2 = splat(inv_clip), sc2 = splat(sc), b2 = splat(h.beta1), o2 = splat(h.om_beta1);
+    auto pair = [&](int e, u64 r, u64 rr, u64 c, u64 rc) {
+        const u64 u = mul2(mul2(mul2(pk(x[e], x[e + 1]), r), c), clip2);
+        const u64 mn = fma2(mul2(pk(m[e], m[e + 1]), sc2), b2, mul2(o2, u));
+        const u64 up = mul2(mul2(mn, rr), rc);
+        amax = fmaxf(amax, fmaxf(fabsf(mn.x), fabsf(mn.y)));
+        m[e] = mn.x; m[e + 1] = mn.y; upd[e] = up.x; upd[e + 1] = up.y;
     };
+    // row and column of an element (most tensors: a 32-bit division)
+    auto locate = [&](int64_t i, int& row, int& col) {
+        if (n < 0x7fffffff) { row = (int)((uint32_t)i / (uint32_t)C); col = (int)i - row * C; }
+        else { row = (int)(i / C); col = (int)(i - (int64_t)row * C); }
+    };
+    int row, col;
     if (V == 8) {      // the columns are a multiple of 8: a lane's elements lie in one row
-        float c[8], rc[8];
         if (cnt) {
-            row_factors();
+            float r, rr, c[8], rc[8];
+            locate(i0, row, col);
+            row_factors(row, r, rr);
             load_run<8, true>(s.vc, col, 0, 8, c);
             load_run<8, true>(s.Rc, col, 0, 8, rc);
-        }
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            upd[e] = 0.0f;
-            if (cnt) element(e, c[e], rc[e]);
-            else m[e] = 0.0f;
+            for (int e = 0; e < 8; e += 2) pair(e, splat(r), splat(rr), pk(c[e], c[e + 1]), pk(rc[e], rc[e + 1]));
         }
     } else {
-        int have = -1;      // row the factors r, rr belong to
+        float r[8], rr[8], c[8], rc[8];
+        if (C >= QBLOCK) {
+            // The block lies in at most two rows: their factors once, and every column factor's load independent of the
+            // others (bf16 set of width 1001: 1842 us with each load behind a test for a new row, 1758 us)
+            float ra, rra, rb, rrb;
+            locate(b0, row, col);
+            row_factors(row, ra, rra);
+            row_factors(min(row + 1, (int)d.rows - 1), rb, rrb);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            upd[e] = 0.0f;
-            if (e >= cnt) m[e] = 0.0f;
-            if (e < cnt) {
-                if (row != have) { have = row; row_factors(); }
-                element(e, s.vc[col], s.Rc[col]);
-                col += 32;
-                while (col >= C) { col -= C; ++row; }
+            for (int e = 0; e < 8; ++e) {
+                const int at = col + j0 + 32 * e;
+                const bool next = at >= C;
+                c[e] = e < cnt ? s.vc[next ? at - C : at] : 0.0f;
+                rc[e] = e < cnt ? s.Rc[next ? at - C : at] : 0.0f;
+                r[e] = next ? rb : ra;
+                rr[e] = next ? rrb : rra;
+            }
+        } else {
+            int have = -1;      // row the factors r, rr belong to
+            locate(i0, row, col);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                r[e] = rr[e] = c[e] = rc[e] = 0.0f;
+                if (e < cnt) {
+                    if (row != have) { have = row; row_factors(row, r[e], rr[e]); }
+                    else { r[e] = r[e ? e - 1 : 0]; rr[e] = rr[e ? e - 1 : 0]; }
+                    c[e] = s.vc[col];
+                    rc[e] = s.Rc[col];
+                    col += 32;
+                    while (col >= C) { col -= C; ++row; }
+                }
             }
         }
-    }
-    const float A = fix_absmax(warp_max(amax)), scale = quant_scale<true>(A);
-    if (lane == 0) d.m_absmax[blk] = A;      // (every lane has read the old value: the reduction is behind them)
-    const uint32_t lo = quant_pack4<true>(make_float4(m[0], m[1], m[2], m[3]), A, scale);
-    const uint32_t hi = quant_pack4<true>(make_float4(m[4], m[5], m[6], m[7]), A, scale);
 #pragma unroll
-    for (int e = 0; e < 8; ++e)
-        if (e < cnt) pv[e] = g_apply_one(p, pv[e], upd[e], h, wd);
+        for (int e = 0; e < 8; e += 2) pair(e, pk(r[e], r[e + 1]), pk(rr[e], rr[e + 1]), pk(c[e], c[e + 1]), pk(rc[e], rc[e + 1]));
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (e >= cnt) m[e] = 0.0f;
+    }
+    const float A = fix_absmax(warp_max(amax));
+    if (lane == 0) d.m_absmax[blk] = A;      // (every lane has read the old value: the reduction is behind them)
+    uint32_t lo, hi;
+    if (recip_safe(A)) {      // the low byte of m * (127 / A) + 1.5 * 2^23 is the code (as in the fused kernel)
+        const u64 s127 = splat(QMAX_I8 / A), magic = splat(ROUND_MAGIC);
+        u64 y[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[e] = fma2(pk(m[2 * e], m[2 * e + 1]), s127, magic);
+        lo = pack_codes4(y[0], y[1]);
+        hi = pack_codes4(y[2], y[3]);
+    } else {
+        const float scale = quant_scale<true>(A);
+        lo = quant_pack4<true>(make_float4(m[0], m[1], m[2], m[3]), A, scale);
+        hi = quant_pack4<true>(make_float4(m[4], m[5], m[6], m[7]), A, scale);
+    }
+    // decay as in band_apply
+    const bool subtract = wd & 1;
+    const u64 k2 = splat(subtract ? -h.wd_lr : wd == 2 ? h.decay_mul : 1.0f), lr2 = splat(-h.lr);
+#pragma unroll
+    for (int e = 0; e < 8; e += 2) {
+        const u64 q = pk(pv[e], pv[e + 1]), t = fma2(k2, q, subtract ? q : splat(-0.0f));
+        pv[e] = t.x; pv[e + 1] = t.y;
+    }
+    if (wd >= 2)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) pv[e] = p.round(pv[e]);
+#pragma unroll
+    for (int e = 0; e < 8; e += 2) {
+        const u64 t = fma2(lr2, pk(upd[e], upd[e + 1]), pk(pv[e], pv[e + 1]));
+        pv[e] = t.x; pv[e + 1] = t.y;
+    }
     if (V == 8) {
         if (cnt) {
             *reinterpret_cast<uint2*>(mq + i0) = make_uint2(lo, hi);
