@@ -34,9 +34,8 @@ struct Param {
     int plan, pos;                // entry of a plan's tensor table
 };
 struct Plan {
-    came_plan_t* handle;
     int device;
-    PyObject* py;                 // the DevicePlan (owned)
+    PyObject* py;                 // the DevicePlan (owned); its `handle` is read at every step, None once it is closed
     std::vector<const void*> g;   // gradient addresses in table order
 };
 struct StepTable {
@@ -82,7 +81,7 @@ bool usable(const at::Tensor& p, const at::Tensor& g) {
     return g.layout() == at::kStrided && g.is_contiguous() && p.is_contiguous() && g.numel() == p.numel();
 }
 
-// build(param_groups, [(handle, device index, DevicePlan, n)], [state dict]): remembers the tensors of a step that the
+// build(param_groups, [(DevicePlan, device index, n)], [state dict]): remembers the tensors of a step that the
 // Python path has just made.  Parameters with a gradient fill the plans' tables in order, by device.  False when they do not.
 PyObject* table_build(PyObject* self, PyObject* args) {
     StepTable* s = reinterpret_cast<StepTable*>(self);
@@ -91,12 +90,11 @@ PyObject* table_build(PyObject* self, PyObject* args) {
     table_clear(s);
     std::vector<int> expect;
     for (Py_ssize_t i = 0; i < PyList_GET_SIZE(plans); ++i) {
-        unsigned long long handle;
         int device, n;
         PyObject* py;
-        if (!PyArg_ParseTuple(PyList_GET_ITEM(plans, i), "KiOi", &handle, &device, &py, &n)) return nullptr;
+        if (!PyArg_ParseTuple(PyList_GET_ITEM(plans, i), "Oii", &py, &device, &n)) return nullptr;
         Py_INCREF(py);
-        s->plans->push_back(Plan{reinterpret_cast<came_plan_t*>(static_cast<uintptr_t>(handle)), device, py, {}});
+        s->plans->push_back(Plan{device, py, {}});
         expect.push_back(n);
     }
     bool ok = true;
@@ -186,11 +184,28 @@ bool hypers_of(StepTable* s, PyObject* group, CameHyper* out) {
     return true;
 }
 
+// The plan as it stands, null when it has been closed (PyErr set on an error)
+came_plan_t* handle_of(const Plan& plan) {
+    PyObject* h = PyObject_GetAttrString(plan.py, "handle");      // ctypes.c_void_p or None
+    if (!h || h == Py_None) { Py_XDECREF(h); return nullptr; }
+    PyObject* v = PyObject_GetAttrString(h, "value");
+    Py_DECREF(h);
+    void* p = v && v != Py_None ? PyLong_AsVoidPtr(v) : nullptr;
+    Py_XDECREF(v);
+    return static_cast<came_plan_t*>(p);
+}
+
 // step(param_groups): launches (>= 0), SLOW or FAILED + code
 long step(StepTable* s, PyObject* groups) {
     if (s->plans->empty() || !PyList_Check(groups) || (size_t)PyList_GET_SIZE(groups) != s->groups->size()) return SLOW;
     const size_t n_groups = s->groups->size();
     if (2 * n_groups > 64) return SLOW;
+    std::vector<came_plan_t*> handles;
+    for (const Plan& plan : *s->plans) {
+        came_plan_t* h = handle_of(plan);
+        if (!h) return SLOW;
+        handles.push_back(h);
+    }
     bool moved = false;
     for (size_t gi = 0; gi < n_groups; ++gi) {
         std::vector<Param>& ps = (*s->groups)[gi];
@@ -220,10 +235,11 @@ long step(StepTable* s, PyObject* groups) {
             return SLOW;
         }
     if (moved)
-        for (Plan& plan : *s->plans) {
+        for (size_t k = 0; k < handles.size(); ++k) {
+            Plan& plan = (*s->plans)[k];
             if (PyObject_SetAttrString(plan.py, "addresses", Py_None) != 0) return SLOW;
             c10::cuda::CUDAGuard guard((c10::DeviceIndex)plan.device);
-            const int rc = came_b200_plan_set_pointers(plan.handle, plan.g.data(), nullptr, (int)plan.g.size(),
+            const int rc = came_b200_plan_set_pointers(handles[k], plan.g.data(), nullptr, (int)plan.g.size(),
                                                        c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)plan.device).stream());
             if (rc == CAME_E_INVALID) return SLOW;      // another alignment class: a new plan
             if (rc != CAME_OK) return FAILED + rc;
@@ -236,12 +252,13 @@ long step(StepTable* s, PyObject* groups) {
         Py_DECREF(next);
     }
     long launches = 0;
-    for (Plan& plan : *s->plans) {
+    for (size_t k = 0; k < handles.size(); ++k) {
+        const Plan& plan = (*s->plans)[k];
         c10::cuda::CUDAGuard guard((c10::DeviceIndex)plan.device);
-        const int rc = came_b200_step(plan.handle, hyp, (int)(2 * n_groups),
+        const int rc = came_b200_step(handles[k], hyp, (int)(2 * n_groups),
                                       c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)plan.device).stream());
         if (rc != CAME_OK) return FAILED + rc;
-        launches += came_b200_plan_last_launches(plan.handle);
+        launches += came_b200_plan_last_launches(handles[k]);
     }
     return launches;
 }

@@ -288,7 +288,7 @@ class _CameB200Optimizer(torch.optim.Optimizer):
             return
         stepped = [self.state[p] for g in self.param_groups for p in g["params"]
                    if p.grad is not None and "step" in self.state[p]]
-        plans = [(plan.handle.value, plan.device.index, plan, plan.n) for plan in self._engine.plans.values()]
+        plans = [(plan, plan.device.index, plan.n) for plan in self._engine.plans.values()]
         table = _host.StepTable()
         if all(isinstance(g["params"], list) for g in self.param_groups) and table.build(self.param_groups, plans, stepped):
             self._table = table
@@ -338,6 +338,7 @@ class _CameB200Optimizer(torch.optim.Optimizer):
     def prime_for_cuda_graph(self) -> None:
         """Allocates every state tensor and builds the device tensor table ahead of the first step
         (CAME8bit2D.py:52-72, CAME8bit.py:672-693)."""
+        self._table = None      # the plans it was built from may be replaced or re-pointed below
         entries, _, _ = self._collect()
         for group in self.param_groups:
             for p in group["params"]:

@@ -77,3 +77,35 @@ def test_hooks_closures_and_repeated_tables():
     opt.param_groups[0]["betas"] = (0.9, 0.99)
     with pytest.raises(Exception):
         opt.step()
+
+
+@pytest.mark.parametrize("kind", ["alignment", "dropped", "and back"])
+def test_plans_replaced_by_priming(kind):
+    """prime_for_cuda_graph() between two steps closes or re-points the plan that the table was built from."""
+    (pa, oa), (pb, ob) = _make(), _make()
+    for ps, opt in ((pa, oa), (pb, ob)):
+        sets = [_grads(0), _grads(1)]
+        if kind == "alignment":
+            big = torch.zeros(sets[1][3].numel() + 1, device="cuda", dtype=torch.bfloat16)
+            big[1:] = sets[1][3].reshape(-1)
+            sets[1][3] = big[1:].view(SHAPES[3])
+        elif kind == "dropped":
+            sets[1][2] = None
+        for k, gs in enumerate((sets[0], sets[0], sets[1])):
+            for p, g in zip(ps, gs):
+                p.grad = g
+            if k < 2:
+                opt.step()
+        if opt is ob:
+            ob._table = None
+        opt.prime_for_cuda_graph()
+        if kind == "and back":
+            for p, g in zip(ps, sets[0]):
+                p.grad = g
+        if opt is ob:
+            ob._table = None
+        opt.step()
+        opt.step()
+    assert oa.last_step_launches == ob.last_step_launches
+    for p, q in zip(pa, pb):
+        assert torch.equal(p.data, q.data)

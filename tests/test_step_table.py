@@ -1,0 +1,48 @@
+"""The native step table on the CPU, with a stand-in for the plan: what makes it hand a step back instead of launching."""
+import ctypes as C
+
+import pytest
+import torch
+
+import came_b200
+from came_b200 import _host
+
+
+class _Plan:
+    """The part of engine.DevicePlan the table uses."""
+
+    def __init__(self):
+        self.memory = C.create_string_buffer(1 << 16)
+        self.handle = C.c_void_p(C.addressof(self.memory))
+        self.addresses = ()
+
+
+def _group(*shapes):
+    ps = [torch.nn.Parameter(torch.zeros(s)) for s in shapes]
+    for p in ps:
+        p.grad = torch.zeros_like(p)
+    return ps, [dict(params=ps, lr=1e-3, betas=(0.9, 0.99, 0.999), eps=(1e-30, 1e-16), clip_threshold=1.0, weight_decay=0.0)]
+
+
+def _optimizer(cls=None):
+    opt = (cls or came_b200.CAME8bit)([torch.nn.Parameter(torch.zeros(4, 4))], lr=1e-3)
+    opt._collect = lambda: ([], [], [])      # (no GPU here: nothing to step)
+    return opt
+
+
+def test_a_closed_plan_is_not_stepped():
+    ps, groups = _group((4, 4), (3,))
+    plan, table = _Plan(), _host.StepTable()
+    assert table.build(groups, [(plan, -1, 2)], [])
+    plan.handle = None                       # what DevicePlan.close() leaves
+    assert table.step(groups) == -1
+    ps[0].grad = torch.ones(4, 4)            # gradients that moved: no pointer upload either
+    assert table.step(groups) == -1
+
+
+def test_priming_drops_the_table():
+    """prime_for_cuda_graph() may replace or re-point the plans the table was built from."""
+    opt = _optimizer()
+    opt._table = object()
+    opt.prime_for_cuda_graph()
+    assert opt._table is None
