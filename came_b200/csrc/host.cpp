@@ -14,6 +14,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -23,6 +24,9 @@ namespace {
 
 constexpr long SLOW = -1;         // the caller takes the Python path
 constexpr long FAILED = -1000;    // FAILED + code: the library refused (came_b200_last_error has the message)
+
+struct Unref { void operator()(PyObject* o) const { Py_XDECREF(o); } };
+using Owned = std::unique_ptr<PyObject, Unref>;
 
 struct Param {
     at::Tensor t;
@@ -228,6 +232,15 @@ long step(StepTable* s, PyObject* groups) {
             }
         }
     }
+    std::vector<Owned> counts;      // the states' new step counts: all of them are formed before the first is stored
+    for (PyObject* d : *s->states) {
+        PyObject* v = PyDict_GetItemWithError(d, s->k_step);
+        counts.emplace_back(v ? PyNumber_Add(v, s->one) : nullptr);
+        if (!counts.back()) {
+            PyErr_Clear();      // the Python path raises what there is to raise
+            return SLOW;
+        }
+    }
     CameHyper hyp[64];
     for (size_t gi = 0; gi < n_groups; ++gi)
         if (!hypers_of(s, PyList_GET_ITEM(groups, (Py_ssize_t)gi), hyp + 2 * gi)) {
@@ -244,13 +257,8 @@ long step(StepTable* s, PyObject* groups) {
             if (rc == CAME_E_INVALID) return SLOW;      // another alignment class: a new plan
             if (rc != CAME_OK) return FAILED + rc;
         }
-    for (PyObject* d : *s->states) {
-        PyObject* v = PyDict_GetItemWithError(d, s->k_step);
-        if (!v) return SLOW;
-        PyObject* next = PyNumber_Add(v, s->one);
-        if (!next || PyDict_SetItem(d, s->k_step, next) != 0) { Py_XDECREF(next); return SLOW; }
-        Py_DECREF(next);
-    }
+    for (size_t i = 0; i < counts.size(); ++i)
+        if (PyDict_SetItem((*s->states)[i], s->k_step, counts[i].get()) != 0) return SLOW;
     long launches = 0;
     for (size_t k = 0; k < handles.size(); ++k) {
         const Plan& plan = (*s->plans)[k];

@@ -298,11 +298,12 @@ class _CameB200Optimizer(torch.optim.Optimizer):
         table = getattr(self, "_table", None)
         if table is None:
             return False
+        self._table = None      # (it is kept only if it stepped: not past an exception either)
         n = table.step(self.param_groups)
         if n >= 0:
+            self._table = table
             self.last_step_launches = n
             return True
-        self._table = None
         if n < -1:
             _lib.check(n + 1000)
         return False

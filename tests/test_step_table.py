@@ -46,3 +46,27 @@ def test_priming_drops_the_table():
     opt._table = object()
     opt.prime_for_cuda_graph()
     assert opt._table is None
+
+
+def test_counts_go_up_for_all_or_none():
+    ps, groups = _group((4, 4), (3,))
+    states = [{"step": 3}, {}]               # the second has lost its count: the full path has to look at it
+    plan, table = _Plan(), _host.StepTable()
+    assert table.build(groups, [(plan, -1, 2)], states)
+    assert table.step(groups) == -1
+    assert states == [{"step": 3}, {}]
+    states[1]["step"] = object()             # what the full path raises for, the table leaves to it
+    assert table.step(groups) == -1
+    assert states[0] == {"step": 3}
+
+
+def test_an_exception_drops_the_table():
+    class Raises:
+        def step(self, groups):
+            raise RuntimeError("no")
+
+    opt = _optimizer()
+    opt._table = Raises()
+    with pytest.raises(RuntimeError):
+        opt.step()
+    assert opt._table is None
