@@ -28,9 +28,8 @@ constexpr long FAILED = -1000;    // FAILED + code: the library refused (came_b2
 struct Unref { void operator()(PyObject* o) const { Py_XDECREF(o); } };
 using Owned = std::unique_ptr<PyObject, Unref>;
 
-struct Param {
-    at::Tensor t;
-    PyObject* obj;                // borrowed from the group's list: compared, never dereferenced
+struct Param {                    // (no reference to the parameter: swap_tensors() and the garbage collector count them)
+    PyObject* obj;                // borrowed from the group's list: compared with what the list holds now
     bool has_grad;
     at::ScalarType p_type, g_type;
     const void *p_ptr, *g_ptr;
@@ -110,19 +109,20 @@ PyObject* table_build(PyObject* self, PyObject* args) {
         for (Py_ssize_t i = 0; ok && i < PyList_GET_SIZE(list); ++i) {
             PyObject* obj = PyList_GET_ITEM(list, i);
             if (!THPVariable_Check(obj)) { ok = false; break; }
-            Param e{THPVariable_Unpack(obj), obj, false, at::kFloat, at::kFloat, nullptr, nullptr, {}, -1, -1};
-            const at::Tensor& g = e.t.grad();
+            Param e{obj, false, at::kFloat, at::kFloat, nullptr, nullptr, {}, -1, -1};
+            const at::Tensor& t = THPVariable_Unpack(obj);
+            const at::Tensor& g = t.grad();
             if (g.defined()) {
                 int k = 0;
-                while (k < (int)s->plans->size() && (*s->plans)[k].device != e.t.device().index()) ++k;
-                if (k == (int)s->plans->size() || !usable(e.t, g)) { ok = false; break; }
+                while (k < (int)s->plans->size() && (*s->plans)[k].device != t.device().index()) ++k;
+                if (k == (int)s->plans->size() || !usable(t, g)) { ok = false; break; }
                 Plan& plan = (*s->plans)[k];
                 e.has_grad = true;
-                e.p_type = e.t.scalar_type();
+                e.p_type = t.scalar_type();
                 e.g_type = g.scalar_type();
-                e.p_ptr = e.t.const_data_ptr();
+                e.p_ptr = t.const_data_ptr();
                 e.g_ptr = g.const_data_ptr();
-                e.sizes = e.t.sizes().vec();
+                e.sizes = t.sizes().vec();
                 e.plan = k;
                 e.pos = (int)plan.g.size();
                 plan.g.push_back(e.g_ptr);
@@ -217,12 +217,13 @@ long step(StepTable* s, PyObject* groups) {
         if (!list || !PyList_Check(list) || (size_t)PyList_GET_SIZE(list) != ps.size()) return SLOW;
         for (size_t i = 0; i < ps.size(); ++i) {
             Param& e = ps[i];
-            if (PyList_GET_ITEM(list, (Py_ssize_t)i) != e.obj) return SLOW;
-            const at::Tensor& g = e.t.grad();
+            if (PyList_GET_ITEM(list, (Py_ssize_t)i) != e.obj || !THPVariable_Check(e.obj)) return SLOW;
+            const at::Tensor& t = THPVariable_Unpack(e.obj);
+            const at::Tensor& g = t.grad();
             if (g.defined() != e.has_grad) return SLOW;
             if (!e.has_grad) continue;
-            if (!usable(e.t, g) || g.scalar_type() != e.g_type || e.t.scalar_type() != e.p_type || e.t.const_data_ptr() != e.p_ptr ||
-                e.t.sizes() != at::IntArrayRef(e.sizes) || g.device() != e.t.device())
+            if (!usable(t, g) || g.scalar_type() != e.g_type || t.scalar_type() != e.p_type || t.const_data_ptr() != e.p_ptr ||
+                t.sizes() != at::IntArrayRef(e.sizes) || g.device() != t.device())
                 return SLOW;
             const void* at = g.const_data_ptr();
             if (at != e.g_ptr) {

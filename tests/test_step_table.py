@@ -70,3 +70,13 @@ def test_an_exception_drops_the_table():
     with pytest.raises(RuntimeError):
         opt.step()
     assert opt._table is None
+
+
+def test_the_table_holds_no_tensors():
+    """torch.utils.swap_tensors() and the garbage collector count a parameter's references."""
+    ps, groups = _group((4, 4), (4, 4))
+    plan, table = _Plan(), _host.StepTable()
+    assert table.build(groups, [(plan, -1, 2)], [])
+    ps[0].grad = ps[1].grad = None
+    torch.utils.swap_tensors(ps[0], torch.nn.Parameter(torch.ones(4, 4)))
+    assert table.step(groups) == -1
