@@ -327,7 +327,17 @@ class _CameB200Optimizer(torch.optim.Optimizer):
     # step() with torch's hooks and profiler range around it (what torch wraps around every optimizer's step)
     _step_hooked = torch.optim.Optimizer.profile_hook_step(_step_full)
 
+    _hooks_around_override = False      # a subclass's own step(), which torch has wrapped with the hooks, calls the one below
+
+    def _patch_step_function(self):
+        before = type(self).step
+        super()._patch_step_function()
+        if type(self).step is not before:
+            type(self)._hooks_around_override = True
+
     def step(self, closure=None):
+        if self._hooks_around_override:
+            return self._step_full(closure)
         if closure is None and not (self._optimizer_step_pre_hooks or self._optimizer_step_post_hooks or _global_hooks() or
                                     torch.autograd._profiler_enabled()) and self._step_again():
             return None

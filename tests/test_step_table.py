@@ -80,3 +80,24 @@ def test_the_table_holds_no_tensors():
     ps[0].grad = ps[1].grad = None
     torch.utils.swap_tensors(ps[0], torch.nn.Parameter(torch.ones(4, 4)))
     assert table.step(groups) == -1
+
+
+def test_hooks_run_once_under_an_overridden_step():
+    """torch wraps the subclass's step() with the hooks; the step it calls must not run them again."""
+    class Mine(came_b200.CAME8bit):
+        def step(self, closure=None):
+            return super().step(closure)
+
+    class Inherits(Mine):
+        pass
+
+    class Plain(came_b200.CAME8bit):
+        pass
+
+    for cls in (Mine, Inherits, Plain, came_b200.CAME8bit):
+        opt, calls = _optimizer(cls), []
+        opt.register_step_pre_hook(lambda *a: calls.append("pre"))
+        opt.register_step_post_hook(lambda *a: calls.append("post"))
+        opt.step()
+        assert opt.step(lambda: 2.0) == 2.0
+        assert calls == ["pre", "post"] * 2, cls
