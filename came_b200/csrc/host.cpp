@@ -25,6 +25,11 @@ namespace {
 constexpr long SLOW = -1;         // the caller takes the Python path
 constexpr long FAILED = -1000;    // FAILED + code: the library refused (came_b200_last_error has the message)
 
+// Without the interpreter's lock: a launch may wait for room in the stream's queue, an allocation for the device.
+struct NoGil {
+    PyThreadState* state = PyEval_SaveThread();
+    ~NoGil() { PyEval_RestoreThread(state); }
+};
 struct Unref { void operator()(PyObject* o) const { Py_XDECREF(o); } };
 using Owned = std::unique_ptr<PyObject, Unref>;
 
@@ -204,11 +209,19 @@ long step(StepTable* s, PyObject* groups) {
     if (s->plans->empty() || !PyList_Check(groups) || (size_t)PyList_GET_SIZE(groups) != s->groups->size()) return SLOW;
     const size_t n_groups = s->groups->size();
     if (2 * n_groups > 64) return SLOW;
-    std::vector<came_plan_t*> handles;
+    // (what is used without the lock below: the table may be dropped or rebuilt by another thread meanwhile)
+    struct Target {
+        came_plan_t* handle;
+        c10::DeviceIndex device;
+        Owned plan;
+        std::vector<const void*> g;
+    };
+    std::vector<Target> targets;
     for (const Plan& plan : *s->plans) {
         came_plan_t* h = handle_of(plan);
         if (!h) return SLOW;
-        handles.push_back(h);
+        Py_INCREF(plan.py);
+        targets.push_back(Target{h, (c10::DeviceIndex)plan.device, Owned(plan.py), {}});
     }
     bool moved = false;
     for (size_t gi = 0; gi < n_groups; ++gi) {
@@ -233,8 +246,10 @@ long step(StepTable* s, PyObject* groups) {
             }
         }
     }
-    std::vector<Owned> counts;      // the states' new step counts: all of them are formed before the first is stored
+    std::vector<Owned> states, counts;      // the states' new step counts: all of them are formed before the first is stored
     for (PyObject* d : *s->states) {
+        Py_INCREF(d);
+        states.emplace_back(d);
         PyObject* v = PyDict_GetItemWithError(d, s->k_step);
         counts.emplace_back(v ? PyNumber_Add(v, s->one) : nullptr);
         if (!counts.back()) {
@@ -248,26 +263,29 @@ long step(StepTable* s, PyObject* groups) {
             PyErr_Clear();      // the Python path raises what there is to raise
             return SLOW;
         }
-    if (moved)
-        for (size_t k = 0; k < handles.size(); ++k) {
-            Plan& plan = (*s->plans)[k];
-            if (PyObject_SetAttrString(plan.py, "addresses", Py_None) != 0) return SLOW;
-            c10::cuda::CUDAGuard guard((c10::DeviceIndex)plan.device);
-            const int rc = came_b200_plan_set_pointers(handles[k], plan.g.data(), nullptr, (int)plan.g.size(),
-                                                       c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)plan.device).stream());
+    if (moved) {
+        for (size_t k = 0; k < targets.size(); ++k) {
+            if (PyObject_SetAttrString(targets[k].plan.get(), "addresses", Py_None) != 0) return SLOW;
+            targets[k].g = (*s->plans)[k].g;
+        }
+        NoGil unlocked;
+        for (const Target& t : targets) {
+            c10::cuda::CUDAGuard guard(t.device);
+            const int rc = came_b200_plan_set_pointers(t.handle, t.g.data(), nullptr, (int)t.g.size(),
+                                                       c10::cuda::getCurrentCUDAStream(t.device).stream());
             if (rc == CAME_E_INVALID) return SLOW;      // another alignment class: a new plan
             if (rc != CAME_OK) return FAILED + rc;
         }
+    }
     for (size_t i = 0; i < counts.size(); ++i)
-        if (PyDict_SetItem((*s->states)[i], s->k_step, counts[i].get()) != 0) return SLOW;
+        if (PyDict_SetItem(states[i].get(), s->k_step, counts[i].get()) != 0) return SLOW;
     long launches = 0;
-    for (size_t k = 0; k < handles.size(); ++k) {
-        const Plan& plan = (*s->plans)[k];
-        c10::cuda::CUDAGuard guard((c10::DeviceIndex)plan.device);
-        const int rc = came_b200_step(handles[k], hyp, (int)(2 * n_groups),
-                                      c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)plan.device).stream());
+    NoGil unlocked;
+    for (const Target& t : targets) {
+        c10::cuda::CUDAGuard guard(t.device);
+        const int rc = came_b200_step(t.handle, hyp, (int)(2 * n_groups), c10::cuda::getCurrentCUDAStream(t.device).stream());
         if (rc != CAME_OK) return FAILED + rc;
-        launches += came_b200_plan_last_launches(handles[k]);
+        launches += came_b200_plan_last_launches(t.handle);
     }
     return launches;
 }
@@ -313,15 +331,20 @@ PyObject* quantize(PyObject*, PyObject* args) {
     if (!PyArg_ParseTuple(args, "Opp", &obj, &is_signed, &tile)) return nullptr;
     try {
         const at::Tensor in = THPVariable_Unpack(obj).detach();
-        c10::cuda::CUDAGuard guard(in.device());
-        const at::Tensor src = fp32_contiguous(in);
-        const int64_t n = src.numel(), blocks = tile ? ((src.size(0) + 15) / 16) * ((src.size(1) + 15) / 16) : std::max<int64_t>(1, (n + 255) / 256);
-        at::Tensor q = at::empty(src.sizes(), src.options().dtype(is_signed ? at::kChar : at::kByte));
-        at::Tensor a = at::empty({blocks}, src.options());
-        const int rc = tile ? came_b200_quantize_tile16(src.const_data_ptr<float>(), static_cast<int8_t*>(q.mutable_data_ptr()),
-                                                        a.mutable_data_ptr<float>(), src.size(0), src.size(1), stream_of(src))
-                            : came_b200_quantize_blockwise(src.const_data_ptr<float>(), q.mutable_data_ptr(), a.mutable_data_ptr<float>(), n,
-                                                           is_signed, stream_of(src));
+        at::Tensor q, a;
+        int rc;
+        {
+            NoGil unlocked;
+            c10::cuda::CUDAGuard guard(in.device());
+            const at::Tensor src = fp32_contiguous(in);
+            const int64_t n = src.numel(), blocks = tile ? ((src.size(0) + 15) / 16) * ((src.size(1) + 15) / 16) : std::max<int64_t>(1, (n + 255) / 256);
+            q = at::empty(src.sizes(), src.options().dtype(is_signed ? at::kChar : at::kByte));
+            a = at::empty({blocks}, src.options());
+            rc = tile ? came_b200_quantize_tile16(src.const_data_ptr<float>(), static_cast<int8_t*>(q.mutable_data_ptr()),
+                                                  a.mutable_data_ptr<float>(), src.size(0), src.size(1), stream_of(src))
+                      : came_b200_quantize_blockwise(src.const_data_ptr<float>(), q.mutable_data_ptr(), a.mutable_data_ptr<float>(), n,
+                                                     is_signed, stream_of(src));
+        }
         return status(rc, rc == CAME_OK ? Py_BuildValue("(NN)", THPVariable_Wrap(q), THPVariable_Wrap(a)) : nullptr);
     } catch (const std::exception& e) {
         return raise_from(e);
@@ -333,14 +356,19 @@ PyObject* dequantize(PyObject*, PyObject* args) {
     int is_signed, tile;
     if (!PyArg_ParseTuple(args, "OOpp", &qobj, &aobj, &is_signed, &tile)) return nullptr;
     try {
-        const at::Tensor q0 = THPVariable_Unpack(qobj);
-        c10::cuda::CUDAGuard guard(q0.device());
-        const at::Tensor q = q0.is_contiguous() ? q0 : q0.contiguous(), a = fp32_contiguous(THPVariable_Unpack(aobj));
-        at::Tensor out = at::empty(q.sizes(), q.options().dtype(at::kFloat));
-        const int rc = tile ? came_b200_dequantize_tile16(static_cast<const int8_t*>(q.const_data_ptr()), a.const_data_ptr<float>(),
-                                                          out.mutable_data_ptr<float>(), q.size(0), q.size(1), stream_of(q))
-                            : came_b200_dequantize_blockwise(q.const_data_ptr(), a.const_data_ptr<float>(), out.mutable_data_ptr<float>(),
-                                                             q.numel(), is_signed, stream_of(q));
+        const at::Tensor q0 = THPVariable_Unpack(qobj), a0 = THPVariable_Unpack(aobj);
+        at::Tensor out;
+        int rc;
+        {
+            NoGil unlocked;
+            c10::cuda::CUDAGuard guard(q0.device());
+            const at::Tensor q = q0.is_contiguous() ? q0 : q0.contiguous(), a = fp32_contiguous(a0);
+            out = at::empty(q.sizes(), q.options().dtype(at::kFloat));
+            rc = tile ? came_b200_dequantize_tile16(static_cast<const int8_t*>(q.const_data_ptr()), a.const_data_ptr<float>(),
+                                                    out.mutable_data_ptr<float>(), q.size(0), q.size(1), stream_of(q))
+                      : came_b200_dequantize_blockwise(q.const_data_ptr(), a.const_data_ptr<float>(), out.mutable_data_ptr<float>(),
+                                                       q.numel(), is_signed, stream_of(q));
+        }
         return status(rc, rc == CAME_OK ? THPVariable_Wrap(out) : nullptr);
     } catch (const std::exception& e) {
         return raise_from(e);

@@ -109,3 +109,40 @@ def test_plans_replaced_by_priming(kind):
     assert oa.last_step_launches == ob.last_step_launches
     for p, q in zip(pa, pb):
         assert torch.equal(p.data, q.data)
+
+
+def test_other_threads_run_while_launches_wait():
+    """A launch that waits for room in the stream's queue must not hold the interpreter's lock."""
+    import threading
+    import time
+    from came_b200 import quant
+    ps, opt = _make()
+    for p, g in zip(ps, _grads(0)):
+        p.grad = g
+    x = torch.ones(256, device="cuda")
+    opt.step(); opt.step(); quant.dequantize_blockwise(*quant.quantize_blockwise(x, signed=True), signed=True)
+    torch.cuda.synchronize()
+    stop, gaps = threading.Event(), []
+
+    def ticks():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.005)
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+
+    for work in (opt.step, lambda: quant.quantize_blockwise(x, signed=True)):
+        thread = threading.Thread(target=ticks)
+        gaps.clear()
+        stop.clear()
+        thread.start()
+        t0 = time.perf_counter()
+        torch.cuda._sleep(3_000_000_000)      # about 1.5 s, in front of more launches than a queue holds
+        for _ in range(3000):
+            work()
+        waited = time.perf_counter() - t0
+        torch.cuda.synchronize()
+        stop.set()
+        thread.join()
+        assert waited > 1.0 and max(gaps) < 0.5, (waited, max(gaps))
