@@ -12,6 +12,7 @@
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <memory>
@@ -91,16 +92,13 @@ bool usable(const at::Tensor& p, const at::Tensor& g) {
 
 // build(param_groups, [(DevicePlan, device index, n)], [state dict]): remembers the tensors of a step that the
 // Python path has just made.  Parameters with a gradient fill the plans' tables in order, by device.  False when they do not.
-PyObject* table_build(PyObject* self, PyObject* args) {
-    StepTable* s = reinterpret_cast<StepTable*>(self);
-    PyObject *groups, *plans, *states;
-    if (!PyArg_ParseTuple(args, "O!O!O!", &PyList_Type, &groups, &PyList_Type, &plans, &PyList_Type, &states)) return nullptr;
+bool build(StepTable* s, PyObject* groups, PyObject* plans, PyObject* states) {
     table_clear(s);
     std::vector<int> expect;
     for (Py_ssize_t i = 0; i < PyList_GET_SIZE(plans); ++i) {
         int device, n;
         PyObject* py;
-        if (!PyArg_ParseTuple(PyList_GET_ITEM(plans, i), "Oii", &py, &device, &n)) return nullptr;
+        if (!PyArg_ParseTuple(PyList_GET_ITEM(plans, i), "Oii", &py, &device, &n)) return false;
         Py_INCREF(py);
         s->plans->push_back(Plan{device, py, {}});
         expect.push_back(n);
@@ -143,9 +141,25 @@ PyObject* table_build(PyObject* self, PyObject* args) {
         Py_INCREF(d);
         s->states->push_back(d);
     }
-    if (!ok) table_clear(s);
+    return ok;
+}
+// Every entry below: what torch throws becomes the Python exception torch has for it (END_HANDLE_TH_ERRORS).
+PyObject* table_build(PyObject* self, PyObject* args) {
+    HANDLE_TH_ERRORS
+    StepTable* s = reinterpret_cast<StepTable*>(self);
+    PyObject *groups, *plans, *states;
+    if (!PyArg_ParseTuple(args, "O!O!O!", &PyList_Type, &groups, &PyList_Type, &plans, &PyList_Type, &states)) return nullptr;
+    bool ok = false;
+    try {
+        ok = build(s, groups, plans, states);
+    } catch (...) {
+        table_clear(s);
+        throw;
+    }
+    if (!ok || PyErr_Occurred()) table_clear(s);
     if (PyErr_Occurred()) return nullptr;
     return PyBool_FromLong(ok);
+    END_HANDLE_TH_ERRORS
 }
 
 bool number(PyObject* dict, PyObject* key, double* out) {
@@ -290,18 +304,12 @@ long step(StepTable* s, PyObject* groups) {
     return launches;
 }
 
-PyObject* raise_from(const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
-}
 PyObject* table_step(PyObject* self, PyObject* groups) {
-    try {
-        const long r = step(reinterpret_cast<StepTable*>(self), groups);
-        if (PyErr_Occurred()) return nullptr;
-        return PyLong_FromLong(r);
-    } catch (const std::exception& e) {
-        return raise_from(e);
-    }
+    HANDLE_TH_ERRORS
+    const long r = step(reinterpret_cast<StepTable*>(self), groups);
+    if (PyErr_Occurred()) return nullptr;
+    return PyLong_FromLong(r);
+    END_HANDLE_TH_ERRORS
 }
 PyObject* table_forget(PyObject* self, PyObject*) {
     table_clear(reinterpret_cast<StepTable*>(self));
@@ -319,60 +327,62 @@ cudaStream_t stream_of(const at::Tensor& t) { return c10::cuda::getCurrentCUDASt
 PyObject* status(int rc, PyObject* result) {
     if (rc == CAME_OK) return result;
     Py_XDECREF(result);
-    return PyErr_Format(PyExc_RuntimeError, "came_b200 error %d: %s", rc, came_b200_last_error());
+    const Owned lib(PyImport_ImportModule("came_b200._lib"));
+    const Owned type(lib ? PyObject_GetAttrString(lib.get(), "CameError") : nullptr);
+    return type ? PyErr_Format(type.get(), "came_b200 error %d: %s", rc, came_b200_last_error()) : nullptr;
+}
+const at::Tensor& tensor_of(PyObject* o) {
+    if (!THPVariable_Check(o)) throw torch::TypeError(std::string("expected a tensor, got ") + Py_TYPE(o)->tp_name);
+    return THPVariable_Unpack(o);
 }
 at::Tensor fp32_contiguous(const at::Tensor& t) {
     return t.scalar_type() == at::kFloat && t.is_contiguous() ? t : t.to(at::kFloat).contiguous();
 }
 
 PyObject* quantize(PyObject*, PyObject* args) {
+    HANDLE_TH_ERRORS
     PyObject* obj;
     int is_signed, tile;
     if (!PyArg_ParseTuple(args, "Opp", &obj, &is_signed, &tile)) return nullptr;
-    try {
-        const at::Tensor in = THPVariable_Unpack(obj).detach();
-        at::Tensor q, a;
-        int rc;
-        {
-            NoGil unlocked;
-            c10::cuda::CUDAGuard guard(in.device());
-            const at::Tensor src = fp32_contiguous(in);
-            const int64_t n = src.numel(), blocks = tile ? ((src.size(0) + 15) / 16) * ((src.size(1) + 15) / 16) : std::max<int64_t>(1, (n + 255) / 256);
-            q = at::empty(src.sizes(), src.options().dtype(is_signed ? at::kChar : at::kByte));
-            a = at::empty({blocks}, src.options());
-            rc = tile ? came_b200_quantize_tile16(src.const_data_ptr<float>(), static_cast<int8_t*>(q.mutable_data_ptr()),
-                                                  a.mutable_data_ptr<float>(), src.size(0), src.size(1), stream_of(src))
-                      : came_b200_quantize_blockwise(src.const_data_ptr<float>(), q.mutable_data_ptr(), a.mutable_data_ptr<float>(), n,
-                                                     is_signed, stream_of(src));
-        }
-        return status(rc, rc == CAME_OK ? Py_BuildValue("(NN)", THPVariable_Wrap(q), THPVariable_Wrap(a)) : nullptr);
-    } catch (const std::exception& e) {
-        return raise_from(e);
+    const at::Tensor in = tensor_of(obj).detach();
+    at::Tensor q, a;
+    int rc;
+    {
+        NoGil unlocked;
+        c10::cuda::CUDAGuard guard(in.device());
+        const at::Tensor src = fp32_contiguous(in);
+        const int64_t n = src.numel(), blocks = tile ? ((src.size(0) + 15) / 16) * ((src.size(1) + 15) / 16) : std::max<int64_t>(1, (n + 255) / 256);
+        q = at::empty(src.sizes(), src.options().dtype(is_signed ? at::kChar : at::kByte));
+        a = at::empty({blocks}, src.options());
+        rc = tile ? came_b200_quantize_tile16(src.const_data_ptr<float>(), static_cast<int8_t*>(q.mutable_data_ptr()),
+                                              a.mutable_data_ptr<float>(), src.size(0), src.size(1), stream_of(src))
+                  : came_b200_quantize_blockwise(src.const_data_ptr<float>(), q.mutable_data_ptr(), a.mutable_data_ptr<float>(), n,
+                                                 is_signed, stream_of(src));
     }
+    return status(rc, rc == CAME_OK ? Py_BuildValue("(NN)", THPVariable_Wrap(q), THPVariable_Wrap(a)) : nullptr);
+    END_HANDLE_TH_ERRORS
 }
 
 PyObject* dequantize(PyObject*, PyObject* args) {
+    HANDLE_TH_ERRORS
     PyObject *qobj, *aobj;
     int is_signed, tile;
     if (!PyArg_ParseTuple(args, "OOpp", &qobj, &aobj, &is_signed, &tile)) return nullptr;
-    try {
-        const at::Tensor q0 = THPVariable_Unpack(qobj), a0 = THPVariable_Unpack(aobj);
-        at::Tensor out;
-        int rc;
-        {
-            NoGil unlocked;
-            c10::cuda::CUDAGuard guard(q0.device());
-            const at::Tensor q = q0.is_contiguous() ? q0 : q0.contiguous(), a = fp32_contiguous(a0);
-            out = at::empty(q.sizes(), q.options().dtype(at::kFloat));
-            rc = tile ? came_b200_dequantize_tile16(static_cast<const int8_t*>(q.const_data_ptr()), a.const_data_ptr<float>(),
-                                                    out.mutable_data_ptr<float>(), q.size(0), q.size(1), stream_of(q))
-                      : came_b200_dequantize_blockwise(q.const_data_ptr(), a.const_data_ptr<float>(), out.mutable_data_ptr<float>(),
-                                                       q.numel(), is_signed, stream_of(q));
-        }
-        return status(rc, rc == CAME_OK ? THPVariable_Wrap(out) : nullptr);
-    } catch (const std::exception& e) {
-        return raise_from(e);
+    const at::Tensor q0 = tensor_of(qobj), a0 = tensor_of(aobj);
+    at::Tensor out;
+    int rc;
+    {
+        NoGil unlocked;
+        c10::cuda::CUDAGuard guard(q0.device());
+        const at::Tensor q = q0.is_contiguous() ? q0 : q0.contiguous(), a = fp32_contiguous(a0);
+        out = at::empty(q.sizes(), q.options().dtype(at::kFloat));
+        rc = tile ? came_b200_dequantize_tile16(static_cast<const int8_t*>(q.const_data_ptr()), a.const_data_ptr<float>(),
+                                                out.mutable_data_ptr<float>(), q.size(0), q.size(1), stream_of(q))
+                  : came_b200_dequantize_blockwise(q.const_data_ptr(), a.const_data_ptr<float>(), out.mutable_data_ptr<float>(),
+                                                   q.numel(), is_signed, stream_of(q));
     }
+    return status(rc, rc == CAME_OK ? THPVariable_Wrap(out) : nullptr);
+    END_HANDLE_TH_ERRORS
 }
 
 PyMethodDef module_methods[] = {{"quantize", quantize, METH_VARARGS, "(tensor, signed, tile) -> (codes, absmax)"},

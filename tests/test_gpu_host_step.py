@@ -146,3 +146,11 @@ def test_other_threads_run_while_launches_wait():
         stop.set()
         thread.join()
         assert waited > 1.0 and max(gaps) < 0.5, (waited, max(gaps))
+
+
+def test_out_of_memory_keeps_its_type():
+    from came_b200 import quant
+    x = torch.ones(1, device="cuda").expand(1 << 40)      # 4 TB once contiguous: refused at once
+    with pytest.raises(torch.OutOfMemoryError):
+        quant.quantize_blockwise(x, signed=True)
+    assert quant.quantize_blockwise(x[:300], signed=True)[1].tolist() == [1.0, 1.0]

@@ -101,3 +101,38 @@ def test_hooks_run_once_under_an_overridden_step():
         opt.step()
         assert opt.step(lambda: 2.0) == 2.0
         assert calls == ["pre", "post"] * 2, cls
+
+
+def test_entries_refuse_what_is_no_tensor():
+    for call in (lambda: _host.quantize(object(), True, False), lambda: _host.dequantize(object(), torch.zeros(1), True, False),
+                 lambda: _host.dequantize(torch.zeros(4, dtype=torch.int8), [1.0], True, False)):
+        with pytest.raises(TypeError):
+            call()
+
+
+class _Raises(torch.Tensor):
+    """A tensor whose layout is asked for in Python, which raises."""
+
+    @staticmethod
+    def __new__(cls, shape):
+        return torch.Tensor._make_wrapper_subclass(cls, shape, dispatch_sizes_strides_policy="strides")
+
+    @classmethod
+    def __torch_dispatch__(cls, func, types, args=(), kwargs=None):
+        raise KeyError("asked")
+
+
+def test_exceptions_out_of_tensors_reach_python():
+    """A C++ or Python exception below the module's entries is raised as what it is; it does not end the process."""
+    ps, groups = _group((4, 4))
+    plan, table = _Plan(), _host.StepTable()
+    assert table.build(groups, [(plan, -1, 1)], [])
+    bad = torch.nn.Parameter(torch.zeros(4, 4))
+    bad.grad = _Raises((4, 4))
+    groups[0]["params"] = [bad]
+    with pytest.raises(KeyError):
+        _host.StepTable().build(groups, [(plan, -1, 1)], [])
+    groups[0]["params"] = ps
+    ps[0].grad = _Raises((4, 4))
+    with pytest.raises(KeyError):
+        table.step(groups)
