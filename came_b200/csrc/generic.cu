@@ -209,7 +209,7 @@ struct Item {
         R = (int)d.rows; C = (int)d.cols;
         tr = w.tile / s.tiles_c; tc = w.tile - tr * s.tiles_c;
         brow = tr * s.g_nb * 16; col0 = tc * G_CW; k = 0;
-        nb = min(s.g_nb, (R - brow + 15) >> 4);
+        nb = min(s.g_nb, ((R - brow - 1) >> 4) + 1);
         v8 = s.g_v == 8;
     }
 };
@@ -223,23 +223,23 @@ template <int ESZ>
 __device__ __forceinline__ void stage_rows(char* dst, int pitch, const void* base, int esz, const Item& it, int lane) {
     const uintptr_t b = reinterpret_cast<uintptr_t>(base);
     const uintptr_t first = b + (uintptr_t)(((int64_t)it.brow * it.C + it.col0) * esz);
-    const int pitch_g = it.C * esz;      // (rows of a chunk below 2^31 bytes: C < 2^29)
+    auto rows_on = [&](int r) { return (int64_t)r * it.C * esz; };      // (bytes; a row may be longer than 2^31)
     if constexpr (ESZ > 0) {
         constexpr int NCH = G_CW * ESZ / 16;
-        if (it.brow + 16 <= it.R && it.col0 + G_CW <= it.C) {
-            if (((first | (uintptr_t)pitch_g) & 15) == 0) {
+        if (it.R - it.brow >= 16 && it.C - it.col0 >= G_CW) {
+            if (((first | (uintptr_t)rows_on(1)) & 15) == 0) {
                 const int r = lane / NCH, ch = lane % NCH;
-                const char* src = reinterpret_cast<const char*>(first) + (int64_t)r * pitch_g + 16 * ch;
+                const char* src = reinterpret_cast<const char*>(first) + rows_on(r) + 16 * ch;
                 char* to = dst + r * pitch + 16 * ch;
 #pragma unroll
-                for (int k = 0; k < NCH / 2; ++k, src += (int64_t)(32 / NCH) * pitch_g, to += 32 / NCH * pitch) cp16(to, src, 16);
+                for (int k = 0; k < NCH / 2; ++k, src += rows_on(32 / NCH), to += 32 / NCH * pitch) cp16(to, src, 16);
                 return;
             }
-            if (it.brow + 16 < it.R) {      // (a row follows: the last chunk stays inside the array)
+            if (it.R - it.brow > 16) {      // (a row follows: the last chunk stays inside the array)
 #pragma unroll
                 for (int k = 0; k < (16 * (NCH + 1) + 31) / 32; ++k) {
                     const int j = lane + 32 * k, r = j / (NCH + 1), ch = j - r * (NCH + 1);
-                    const uintptr_t src = ((first + (uintptr_t)((int64_t)r * pitch_g)) & ~(uintptr_t)15) + 16 * ch;
+                    const uintptr_t src = ((first + (uintptr_t)rows_on(r)) & ~(uintptr_t)15) + 16 * ch;
                     if (j < 16 * (NCH + 1)) cp16(dst + r * pitch + 16 * ch, reinterpret_cast<const void*>(src), 16);
                 }
                 return;
@@ -250,7 +250,7 @@ __device__ __forceinline__ void stage_rows(char* dst, int pitch, const void* bas
     const uintptr_t end = b + (uintptr_t)((int64_t)it.R * it.C * esz);
     for (int j = lane; j < 16 * nch; j += 32) {
         const int r = j / nch, ch = j - r * nch;
-        const uintptr_t row = first + (uintptr_t)((int64_t)r * pitch_g), src = (row & ~(uintptr_t)15) + 16 * ch;
+        const uintptr_t row = first + (uintptr_t)rows_on(r), src = (row & ~(uintptr_t)15) + 16 * ch;
         const bool want = r < rows && src < row + width;
         cp16(dst + r * pitch + 16 * ch, reinterpret_cast<const void*>(want ? src : b & ~(uintptr_t)15),
              want ? (int)min((uintptr_t)16, end - src) : 0);
@@ -270,7 +270,7 @@ __device__ __forceinline__ void stage_vectors(char* st, int off_v, int off_c, co
 template <int MODE>
 __device__ __forceinline__ void stage_absmax(char* x, const float* absmax, const Item& it, int lane) {
     if (MODE == CAME_MODE_TILE8) {
-        const int tile_cols = (it.C + TILE - 1) / TILE, t = (it.col0 >> 4) + lane;
+        const int tile_cols = ((it.C - 1) / TILE + 1), t = (it.col0 >> 4) + lane;
         if (lane < 4 && t < tile_cols) cp4(x + 4 * lane, absmax + (int64_t)(it.brow >> 4) * tile_cols + t);
     } else if (MODE == CAME_MODE_FLAT8) {
         const int row = min(it.brow + (lane >> 1), it.R - 1);
@@ -346,7 +346,7 @@ __device__ __forceinline__ void read_codes(const char* rows, int pitch, int low,
         x[0] = (float)p[lane]; x[1] = (float)p[lane + 32];
     }
 }
-// offset of row r of a band from a 16-byte boundary (and what it grows by per row), modulo 16
+// offset of a band's first row from a 16-byte boundary, and what the offset grows by per row, modulo 16
 __device__ __forceinline__ int low_bits(const void* base, const Item& it, int esz) {
     return (int)((reinterpret_cast<uintptr_t>(base) + (uintptr_t)(((int64_t)it.brow * it.C + it.col0) * esz)) & 15);
 }
@@ -362,6 +362,8 @@ template <int V>
 __device__ __forceinline__ void band_row_sums(const Item& it, float* rowpart, float* rs, int lane) {
     int o = V == 8 ? 4 : 16;
 #pragma unroll
+__device__ __forceinline__ int low_step(const Item& it, int esz) { return (int)(((uint32_t)it.C * (uint32_t)esz) & 15u); }
+
     for (int h = Lane<V>::NR / 2; h >= 1; h >>= 1, o >>= 1) {
         const bool up = (lane & o) != 0;
 #pragma unroll
@@ -417,7 +419,7 @@ __device__ __forceinline__ void band_sq(const StepArgs& a, const Item& it, const
     constexpr int NR = Lane<V>::NR, E = Lane<V>::E;
     const CameTensorDesc& d = a.descs[it.tensor];
     const int lane = threadIdx.x & 31, esz = size_of<TG>(d.g_dtype), dt = d.g_dtype;
-    const int low = low_bits(d.g, it, esz), grow = it.C * esz;
+    const int low = low_bits(d.g, it, esz), grow = low_step(it, esz);
     float rs[NR];
     bool in[V == 8 ? 1 : 2];      // V = 8: the columns are a multiple of 8, a lane's 8 lie inside or outside together
 #pragma unroll
@@ -452,7 +454,7 @@ __device__ __forceinline__ void band_clip(const StepArgs& a, const Item& it, con
     const CameTensorDesc& d = a.descs[it.tensor];
     const Scratch& s = a.scr[it.tensor];
     const int lane = threadIdx.x & 31, esz = size_of<TG>(d.g_dtype), dt = d.g_dtype;
-    const int low = low_bits(d.g, it, esz), grow = it.C * esz;
+    const int low = low_bits(d.g, it, esz), grow = low_step(it, esz);
     if (it.k == 0) {
         acc = 0.0f;
         mean = read_mean(s.rowblk, s.nbR, it.R, d.flags & CAME_F_SQ_FIX, d.flags & CAME_F_SQ_CLAMP, lane);
@@ -494,7 +496,7 @@ __device__ __forceinline__ void band_moment(const StepArgs& a, const CameHyper* 
     const CameTensorDesc& d = a.descs[it.tensor];
     const Scratch& s = a.scr[it.tensor];
     const int lane = threadIdx.x & 31, esz = size_of<TG>(d.g_dtype), dt = d.g_dtype, msz = MODE == CAME_MODE_FP32 ? 4 : 1;
-    const int low = low_bits(d.g, it, esz), grow = it.C * esz, mlow = low_bits(d.m, it, msz), mgrow = it.C * msz;
+    const int low = low_bits(d.g, it, esz), grow = low_step(it, esz), mlow = low_bits(d.m, it, msz), mgrow = low_step(it, msz);
     const float beta1 = hyp[d.group].beta1, om1 = hyp[d.group].om_beta1;
     if (it.k == 0) {
         mean = read_mean(s.rowblk, s.nbR, it.R, d.flags & CAME_F_SQ_FIX, d.flags & CAME_F_SQ_CLAMP, lane);
@@ -561,7 +563,7 @@ __device__ __forceinline__ void band_moment(const StepArgs& a, const CameHyper* 
     const int live = it.R - it.brow;
     if (MODE == CAME_MODE_TILE8) {
         float q127[V == 8 ? 1 : 2];
-        const int tile_cols = (it.C + TILE - 1) / TILE;
+        const int tile_cols = ((it.C - 1) / TILE + 1);
 #pragma unroll
         for (int q = 0; q < (V == 8 ? 1 : 2); ++q) {
             float A = amax[q];
@@ -640,7 +642,7 @@ __device__ __forceinline__ void band_apply(const StepArgs& a, const CameHyper* h
     const Scratch& s = a.scr[it.tensor];
     const CameHyper h = hyp[d.group];      // (a copy: the stores below could alias the table)
     const int lane = threadIdx.x & 31, esz = size_of<TP>(d.p_dtype), dt = d.p_dtype, msz = MODE == CAME_MODE_FP32 ? 4 : 1;
-    const int low = low_bits(d.p, it, esz), grow = it.C * esz, mlow = low_bits(d.m, it, msz), mgrow = it.C * msz;
+    const int low = low_bits(d.p, it, esz), grow = low_step(it, esz), mlow = low_bits(d.m, it, msz), mgrow = low_step(it, msz);
     const int wd = wd_form(h, d.flags);
     if (it.k == 0) mean = read_mean(s.rowblk2, s.nbR, it.R, d.flags & CAME_F_RESROW_FIX, d.flags & CAME_F_RESROW_CLAMP, lane);
     const float f = band_row_factor(it, reinterpret_cast<const float*>(st + S::OFF_V), mean, d.flags & CAME_F_RESROW_CLAMP, 1.0f, lane);
