@@ -351,6 +351,8 @@ __device__ __forceinline__ int low_bits(const void* base, const Item& it, int es
     return (int)((reinterpret_cast<uintptr_t>(base) + (uintptr_t)(((int64_t)it.brow * it.C + it.col0) * esz)) & 15);
 }
 
+__device__ __forceinline__ int low_step(const Item& it, int esz) { return (int)(((uint32_t)it.C * (uint32_t)esz) & 15u); }
+
 // Squares of a pair added to a row's sum: V = 8 two chains, V = 1 (one pair a row) one chain in .x
 template <int V> __device__ __forceinline__ u64 add_squares(const u64& y, const u64& sum) {
     if (V == 8) return fma2(y, y, sum);
@@ -362,8 +364,6 @@ template <int V>
 __device__ __forceinline__ void band_row_sums(const Item& it, float* rowpart, float* rs, int lane) {
     int o = V == 8 ? 4 : 16;
 #pragma unroll
-__device__ __forceinline__ int low_step(const Item& it, int esz) { return (int)(((uint32_t)it.C * (uint32_t)esz) & 15u); }
-
     for (int h = Lane<V>::NR / 2; h >= 1; h >>= 1, o >>= 1) {
         const bool up = (lane & o) != 0;
 #pragma unroll
