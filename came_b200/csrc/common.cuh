@@ -37,7 +37,7 @@ struct Scratch {
     float* rowpart;   // [max(tiles_c, ptiles_c) * rows]  per-CTA row partial sums
     float* colpart;   // [tiles_r * cols]                 per-CTA column partial sums
     float* spart;     // [tiles_r * tiles_c] partials of S; 1-D tensors: [nbR] block partials of sum u^2
-    float* fac;       // flat layout on generic.cu: row factors r_i [rows], else nullptr
+    float* fac;       // flat layout on generic.cu: row factors r_i times the gradient scale [rows], else nullptr
     float* tpart;     // fused first pass only: [tiles_r * cols] per-strip column sums of g^2 / v_row
     int32_t tiles_r, tiles_c;     // K_TR x K_TC grid
     int32_t ptiles_r, ptiles_c;   // W_TR x W_TC grid of the staged passes

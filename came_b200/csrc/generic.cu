@@ -415,32 +415,39 @@ __device__ __forceinline__ void band_col_factors(const Item& it, const float* c,
 
 // ---- S1 -------------------------------------------------------------------------------------------------------
 template <typename TG, int V>
-__device__ __forceinline__ void band_sq(const StepArgs& a, const Item& it, const char* st, int pitch, u64* colacc) {
+__device__ __forceinline__ void band_sq(const StepArgs& a, const CameHyper* hyp, const Item& it, const char* st, int pitch, u64* colacc, float& gs) {
     constexpr int NR = Lane<V>::NR, E = Lane<V>::E;
     const CameTensorDesc& d = a.descs[it.tensor];
     const int lane = threadIdx.x & 31, esz = size_of<TG>(d.g_dtype), dt = d.g_dtype;
     const int low = low_bits(d.g, it, esz), grow = low_step(it, esz);
+    if (it.k == 0) gs = hyp[d.group].grad_scale;
+    const u64 scale = splat(gs);      // (before the square: unscaled gradients may be too large or too small for one)
     float rs[NR];
-    bool in[V == 8 ? 1 : 2];      // V = 8: the columns are a multiple of 8, a lane's 8 lie inside or outside together
-#pragma unroll
-    for (int q = 0; q < (V == 8 ? 1 : 2); ++q) in[q] = it.col0 + Lane<V>::col(lane, q) < it.C;
     if (it.k == 0)
 #pragma unroll
         for (int e = 0; e < E / 2; ++e) colacc[e] = F2ZERO;
+    // What lies past the end of a row: zeros from the staging, except that for V = 1 its last 16 bytes may hold elements of
+    // the next row, which a band that ends there masks.
+    auto rows = [&](auto ends_here) {
+        bool in[2] = {true, true};
+        if constexpr (decltype(ends_here)::value) { in[0] = it.col0 + lane < it.C; in[1] = it.col0 + lane + 32 < it.C; }
 #pragma unroll
-    for (int i = 0; i < NR; ++i) {
-        const int r = Lane<V>::row(lane, i);
-        float x[E];
-        read_row<V, TG>(st, pitch, dt, (low + r * grow) & 15, r, lane, x);
-        u64 sum = F2ZERO;
+        for (int i = 0; i < NR; ++i) {
+            const int r = Lane<V>::row(lane, i);
+            float x[E];
+            read_row<V, TG>(st, pitch, dt, (low + r * grow) & 15, r, lane, x);
+            u64 sum = F2ZERO;
 #pragma unroll
-        for (int e = 0; e < E; e += 2) {
-            const u64 y = pk(in[0] ? x[e] : 0.0f, in[V == 8 ? 0 : 1] ? x[e + 1] : 0.0f);
-            sum = add_squares<V>(y, sum);
-            colacc[e / 2] = fma2(y, y, colacc[e / 2]);
+            for (int e = 0; e < E; e += 2) {
+                const u64 y = mul2(pk(in[0] ? x[e] : 0.0f, in[1] ? x[e + 1] : 0.0f), scale);
+                sum = add_squares<V>(y, sum);
+                colacc[e / 2] = fma2(y, y, colacc[e / 2]);
+            }
+            rs[i] = V == 8 ? sum.x + sum.y : sum.x;
         }
-        rs[i] = V == 8 ? sum.x + sum.y : sum.x;
-    }
+    };
+    if (V == 8 || it.C - it.col0 >= G_CW) rows(std::false_type{});
+    else rows(std::true_type{});
     const Scratch& s = a.scr[it.tensor];
     float* colpart = s.colpart;
     band_row_sums<V>(it, s.rowpart, rs, lane);
@@ -449,7 +456,7 @@ __device__ __forceinline__ void band_sq(const StepArgs& a, const Item& it, const
 
 // ---- S2 -------------------------------------------------------------------------------------------------------
 template <typename TG, typename S, int V>
-__device__ __forceinline__ void band_clip(const StepArgs& a, const Item& it, const char* st, float& acc, float& mean) {
+__device__ __forceinline__ void band_clip(const StepArgs& a, const CameHyper* hyp, const Item& it, const char* st, float& acc, float& mean, float& gs) {
     constexpr int NR = Lane<V>::NR, E = Lane<V>::E;
     const CameTensorDesc& d = a.descs[it.tensor];
     const Scratch& s = a.scr[it.tensor];
@@ -457,9 +464,11 @@ __device__ __forceinline__ void band_clip(const StepArgs& a, const Item& it, con
     const int low = low_bits(d.g, it, esz), grow = low_step(it, esz);
     if (it.k == 0) {
         acc = 0.0f;
+        gs = hyp[d.group].grad_scale;
         mean = read_mean(s.rowblk, s.nbR, it.R, d.flags & CAME_F_SQ_FIX, d.flags & CAME_F_SQ_CLAMP, lane);
     }
-    const float f = band_row_factor(it, reinterpret_cast<const float*>(st + S::OFF_V), mean, d.flags & CAME_F_SQ_CLAMP, 1.0f, lane);
+    // (the gradient scale rides on the row factors)
+    const float f = band_row_factor(it, reinterpret_cast<const float*>(st + S::OFF_V), mean, d.flags & CAME_F_SQ_CLAMP, gs, lane);
     u64 cf[E / 2], sum = F2ZERO;
     band_col_factors<V>(it, reinterpret_cast<const float*>(st + S::OFF_C), lane, cf);
 #pragma unroll
@@ -478,10 +487,9 @@ __device__ __forceinline__ void band_clip(const StepArgs& a, const Item& it, con
     if (s.fac && it.tc == 0 && lane < 16 && it.brow + lane < it.R) s.fac[it.brow + lane] = f;      // for the flat apply phase
     if (it.k == it.nb - 1) leave_partial(s.spart, s.counters, it.tile, s.tiles_r * s.tiles_c, warp_sum(acc), lane);
 }
-// gradient scale / clip divisor, clip = max(1, sqrt(S/n)/clip_threshold) (came_kernels.cu:2619-2620)
+// 1 / clip divisor, clip = max(1, sqrt(S/n)/clip_threshold) (came_kernels.cu:2619-2620)
 __device__ __forceinline__ float read_inv_clip(const Scratch& s, const CameHyper& h, int64_t n, int lane) {
-    const float gs = h.grad_scale, S = read_sum(s.spart, s.tiles_r * s.tiles_c, lane) * (gs * gs);
-    return gs / fmaxf(1.0f, sqrtf(S / (float)n) / h.clip_threshold);
+    return 1.0f / fmaxf(1.0f, sqrtf(read_sum(s.spart, s.tiles_r * s.tiles_c, lane) / (float)n) / h.clip_threshold);
 }
 
 // ---- M --------------------------------------------------------------------------------------------------------
@@ -490,7 +498,7 @@ __device__ __forceinline__ float read_inv_clip(const Scratch& s, const CameHyper
 // flat layout: nothing written, the apply phase forms m again (came_kernels.cu:2246-2305 keeps it in fp32 scratch)
 template <typename TG, int MODE, int V>
 __device__ __forceinline__ void band_moment(const StepArgs& a, const CameHyper* hyp, const Item& it, const char* st, u64* colacc, float& mean,
-                                            float& inv_clip) {
+                                            float& inv_clip, float& gs) {
     using S = Stage<TG, MODE>;
     constexpr int NR = Lane<V>::NR, E = Lane<V>::E;
     const CameTensorDesc& d = a.descs[it.tensor];
@@ -501,8 +509,9 @@ __device__ __forceinline__ void band_moment(const StepArgs& a, const CameHyper* 
     if (it.k == 0) {
         mean = read_mean(s.rowblk, s.nbR, it.R, d.flags & CAME_F_SQ_FIX, d.flags & CAME_F_SQ_CLAMP, lane);
         inv_clip = read_inv_clip(s, hyp[d.group], (int64_t)it.R * it.C, lane);
+        gs = hyp[d.group].grad_scale;
     }
-    const float f = band_row_factor(it, reinterpret_cast<const float*>(st + S::OFF_V), mean, d.flags & CAME_F_SQ_CLAMP, 1.0f, lane);
+    const float f = band_row_factor(it, reinterpret_cast<const float*>(st + S::OFF_V), mean, d.flags & CAME_F_SQ_CLAMP, gs, lane);
     const float* xs = reinterpret_cast<const float*>(st + S::OFF_X);
     char* const m_base = reinterpret_cast<char*>(d.m);
     float* const absmax = d.m_absmax;
@@ -950,7 +959,6 @@ __device__ __forceinline__ void phase_finalize(const StepArgs& a, const CameHype
 #pragma unroll
     for (int k = 0; k < G_WARPS; ++k) sum += sh.col[k][threadIdx.x];
     if (idx < n) {
-        if (!RES) sum *= h.grad_scale * h.grad_scale;
         v = ema_update(old, RES ? h.beta3 : h.beta2, RES ? h.om_beta3 : h.om_beta2, mean_plus_eps(sum, (float)(is_col ? R : C), RES ? h.eps1 : h.eps0));
         const bool clamp = d.flags & (RES ? CAME_F_RESCOL_CLAMP : CAME_F_SQ_CLAMP);
         if (is_col) (RES ? s.Rc : s.vc)[idx] = inv_sqrt(clamp ? fmaxf(v, 1e-30f) : v);
@@ -1053,6 +1061,7 @@ __global__ void __launch_bounds__(THREADS, CTAS) k_step_generic(const __grid_con
     // last in the deal of the others
     const int first = warp * gridDim.x + blockIdx.x, stride = G_WARPS * gridDim.x, back = gridDim.x - 1 - blockIdx.x;
     u64 colacc[4];
+    float acc = 0.0f, mean = 1.0f, inv_clip = 1.0f, gs = 1.0f;      // of the item in work
 
     for (int i = back; i < l.n_ones; i += gridDim.x) phase_vector_sq<TG>(a, hyp, l.ones[i], sh);
     stream<S::COUNT>(a, l.tiles, l.n_tiles, first, stride,
@@ -1061,8 +1070,8 @@ __global__ void __launch_bounds__(THREADS, CTAS) k_step_generic(const __grid_con
             stage_rows<Size<TG>::FIXED>(stage(k), S::PA, d.g, size_of<TG>(d.g_dtype), it, lane);
         },
         [&](const Item& it, int k) {
-            if (it.v8) band_sq<TG, 8>(a, it, stage(k), S::PA, colacc);
-            else band_sq<TG, 1>(a, it, stage(k), S::PA, colacc);
+            if (it.v8) band_sq<TG, 8>(a, hyp, it, stage(k), S::PA, colacc, gs);
+            else band_sq<TG, 1>(a, hyp, it, stage(k), S::PA, colacc, gs);
         });
     if (!grid_barrier(l.bar, a.status)) return;
 
@@ -1071,7 +1080,6 @@ __global__ void __launch_bounds__(THREADS, CTAS) k_step_generic(const __grid_con
     for (int i = blockIdx.x; i < l.n_vecs; i += gridDim.x) phase_finalize<false>(a, hyp, l.vecs[i], sh);
     if (!grid_barrier(l.bar, a.status)) return;
 
-    float acc = 0.0f, mean = 1.0f, inv_clip = 1.0f;      // of the item in work
     stream<S::COUNT>(a, l.tiles, l.n_tiles, first, stride,
         [&](const Item& it, int k) {
             const CameTensorDesc& d = a.descs[it.tensor];
@@ -1080,8 +1088,8 @@ __global__ void __launch_bounds__(THREADS, CTAS) k_step_generic(const __grid_con
             stage_rows<Size<TG>::FIXED>(stage(k), S::PA, d.g, size_of<TG>(d.g_dtype), it, lane);
         },
         [&](const Item& it, int k) {
-            if (it.v8) band_clip<TG, S, 8>(a, it, stage(k), acc, mean);
-            else band_clip<TG, S, 1>(a, it, stage(k), acc, mean);
+            if (it.v8) band_clip<TG, S, 8>(a, hyp, it, stage(k), acc, mean, gs);
+            else band_clip<TG, S, 1>(a, hyp, it, stage(k), acc, mean, gs);
         });
     if (!grid_barrier(l.bar, a.status)) return;
 
@@ -1095,8 +1103,8 @@ __global__ void __launch_bounds__(THREADS, CTAS) k_step_generic(const __grid_con
             stage_rows<(MODE == CAME_MODE_FP32 ? 4 : 1)>(stage(k) + S::OFF_M, S::PM, d.m, MODE == CAME_MODE_FP32 ? 4 : 1, it, lane);
         },
         [&](const Item& it, int k) {
-            if (it.v8) band_moment<TG, MODE, 8>(a, hyp, it, stage(k), colacc, mean, inv_clip);
-            else band_moment<TG, MODE, 1>(a, hyp, it, stage(k), colacc, mean, inv_clip);
+            if (it.v8) band_moment<TG, MODE, 8>(a, hyp, it, stage(k), colacc, mean, inv_clip, gs);
+            else band_moment<TG, MODE, 1>(a, hyp, it, stage(k), colacc, mean, inv_clip, gs);
         });
     if (!grid_barrier(l.bar, a.status)) return;
 
