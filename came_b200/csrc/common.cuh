@@ -365,10 +365,13 @@ __device__ __forceinline__ float nf_update(float v, float g, uint32_t flags) {
 __device__ __forceinline__ float nf_clip(float S, int64_t n, const CameHyper& h) {
     return fmaxf(1.0f, sqrtf(S / (float)n) / h.clip_threshold);
 }
-// (clip >= 1: the quotient by div_by is the correctly rounded one unless it is close to underflow)
+// (clip >= 1: the quotient by div_by is the correctly rounded one unless it is close to underflow; an infinite divisor or
+// dividend has no remainder to correct by)
+static __device__ __noinline__ float nf_plain_quotient(float u, float clip) { return u / clip; }      // (out of line: rare, and long)
 __device__ __forceinline__ float nf_momentum(float m_old, float u, float clip, float inv_clip, uint32_t flags, const CameHyper& h) {
     if (flags & CAME_F_UPDATE_F16) u = __half2float(__float2half_rn(u));
-    return fmaf(m_old, h.beta1, __fmul_rn(h.om_beta1, clip == 1.0f ? u : div_by(u, clip, inv_clip)));
+    if (clip != 1.0f) u = clip < 1e30f && fabsf(u) < 1e30f ? div_by(u, clip, inv_clip) : nf_plain_quotient(u, clip);
+    return fmaf(m_old, h.beta1, __fmul_rn(h.om_beta1, u));
 }
 
 // ------------------------------------------------------------------------------------------

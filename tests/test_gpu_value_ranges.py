@@ -34,3 +34,18 @@ def test_unscaled_gradients_whose_squares_leave_the_range(cls_name, dtype, power
     got = _final(cls, SHAPES, grads, params0, 2.0 ** -power, dtype)
     for a, b in zip(want, got):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("cls_name", ["CAMECUDA", "CAME8bitFull"])
+@pytest.mark.parametrize("n", [1, 255, 257, 5000])
+def test_vector_whose_clip_divisor_is_infinite(cls_name, n):
+    """beta2 = 1 keeps the second moment at zero: the clamped 1e-30 makes u = 1e15 g, whose squares overflow, and a finite
+    u over an infinite divisor is zero (CAMECUDA.py:262-269, came_kernels.cu:1509-1516): the parameter stays."""
+    import came_b200
+    p = torch.nn.Parameter(torch.linspace(-1, 1, n, device="cuda"))
+    p.grad = torch.linspace(1e5, 2e5, n, device="cuda")
+    before = p.data.clone()
+    opt = getattr(came_b200, cls_name)([p], lr=1e-2, betas=(0.9, 1.0, 0.999))
+    for _ in range(2):
+        opt.step()
+    assert torch.equal(p.data, before)
