@@ -297,7 +297,7 @@ Layout layout(const CameTensorDesc* descs, int n, const Context& ctx) {
     L.off_hyp = off;   off = align_up(off + (size_t)MAX_GROUPS * sizeof(CameHyper));
     L.off_status = off; off = align_up(off + sizeof(int));
     L.off_sync = off;  off = align_up(off + (2 * (size_t)n + 12) * sizeof(int));   // fused kernel: per-tensor item counters, list cursors
-    L.off_bar = off;   off = align_up(off + 2 * MAX_GENERIC_LAUNCHES * sizeof(int));      // grid barriers of the whole-step kernel
+    L.off_bar = off;   off = align_up(off + MAX_GENERIC_LAUNCHES * sizeof(uint32_t));      // grid barriers of the whole-step kernel
     L.n_work = count_work(descs, n, ctx);
     L.off_work = off;  off = align_up(off + L.n_work * sizeof(Work));
     L.off_float = off;
@@ -810,7 +810,7 @@ int came_b200_step(came_plan_t* plan, const CameHyper* hypers, int n_groups, cam
         }
         if (it.kernel == KID_GENERIC) {
             const GenericLists l{wbase + it.work_off, wbase + it.work2_off, wbase + it.work3_off, wbase + it.work4_off,
-                                 it.n, it.n2, it.n3, it.n4, reinterpret_cast<int*>(plan->ws + plan->L.off_bar) + 2 * it.bar};
+                                 it.n, it.n2, it.n3, it.n4, reinterpret_cast<uint32_t*>(plan->ws + plan->L.off_bar) + it.bar};
             e = launch_generic(it.key, a, by_value ? norm : nullptr, n_groups, l, st);
         }
         else if (it.kernel == KID_SQ_PARTIALS && it.key.variant == 2)
@@ -890,6 +890,15 @@ int came_b200_selftest_bounded_wait(int* device_words, came_stream_t stream) {
     if (e == cudaSuccess) e = cudaMemsetAsync(device_words, 0, sizeof(int), st);
     if (e == cudaSuccess) e = launch_selftest_bounded_wait(device_words, device_words + 1, st);
     return e == cudaSuccess ? CAME_OK : fail(CAME_E_CUDA, "selftest_bounded_wait: %s", cudaGetErrorString(e));
+}
+
+int came_b200_selftest_grid_barrier(int* device_words, came_stream_t stream) {
+    if (!device_words) return fail(CAME_E_INVALID, "selftest_grid_barrier: device_words is null");
+    cudaStream_t st = (cudaStream_t)stream;
+    cudaError_t e = cudaMemsetAsync(device_words, 0xff, 10 * sizeof(int), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(device_words, 0, 2 * sizeof(int), st);
+    if (e == cudaSuccess) e = launch_selftest_grid_barrier(device_words, st);
+    return e == cudaSuccess ? CAME_OK : fail(CAME_E_CUDA, "selftest_grid_barrier: %s", cudaGetErrorString(e));
 }
 
 int came_b200_plan_last_launches(const came_plan_t* plan) { return plan ? plan->last_launches : 0; }

@@ -82,28 +82,37 @@ __device__ __forceinline__ int atom_add_acq_rel(int* p, int x) {
     asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(x) : "memory");
     return old;
 }
-__device__ __forceinline__ int ld_acquire_gpu(const int* p) {
-    int v;
-    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+
+__device__ __forceinline__ uint32_t ld_acquire_gpu_u32(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
 
-// Grid-wide barrier of a cooperative launch.  bar[0] counts arrivals and is back at zero afterwards, bar[1] is the
-// generation.  False when the others did not arrive within the limit (the status word is set; the CTA then leaves).
-__device__ __forceinline__ bool grid_barrier(int* bar, int* status) {
+// Grid-wide barrier of a cooperative launch.  One word: arrivals in its low 16 bits, zero again once all have come, the
+// generation above.  False when the others did not arrive within the limit: the status word is set, the arrival is taken
+// back (unless the generation has moved on after all) and the CTA leaves, so that a later launch finds a clean word.
+constexpr uint32_t G_ARRIVALS = 0xffffu;
+__device__ __forceinline__ bool grid_barrier(uint32_t* bar, int* status, uint32_t limit = G_POLL_LIMIT) {
     __shared__ int s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
         s_ok = 1;
         fence_gpu();      // (the whole CTA's writes: they happened before the barrier above)
-        const int g = ld_acquire_gpu(bar + 1);
-        if (atom_add_acq_rel(bar, 1) == (int)gridDim.x - 1) {
-            *reinterpret_cast<volatile int*>(bar) = 0;
-            atom_add_acq_rel(bar + 1, 1);
+        const uint32_t before = (uint32_t)atom_add_acq_rel(reinterpret_cast<int*>(bar), 1), gen = before & ~G_ARRIVALS;
+        if ((before & G_ARRIVALS) == gridDim.x - 1) {
+            atom_add_acq_rel(reinterpret_cast<int*>(bar), (int)(G_ARRIVALS + 1 - gridDim.x));
         } else {
-            uint32_t polls = 0;
-            while (ld_acquire_gpu(bar + 1) == g)
-                if (++polls > G_POLL_LIMIT) { atomicExch(status, STATUS_MBAR_TIMEOUT); s_ok = 0; break; }
+            uint32_t now = ld_acquire_gpu_u32(bar), polls = 0;
+            while ((now & ~G_ARRIVALS) == gen) {
+                if (++polls > limit) {
+                    const uint32_t seen = atomicCAS(bar, now, now - 1);
+                    if (seen == now) { atomicExch(status, STATUS_MBAR_TIMEOUT); s_ok = 0; break; }
+                    now = seen;      // (another arrival, or the release: look again)
+                } else {
+                    now = ld_acquire_gpu_u32(bar);
+                }
+            }
         }
         fence_gpu();
     }
@@ -976,6 +985,10 @@ __device__ __forceinline__ void phase_finalize(const StepArgs& a, const CameHype
         const float bs = block_sum(v, sh.red);
         if (threadIdx.x == 0) blk[b] = bs;
     }
+    // The counters of the next phase.  They are back at zero after every phase that ran to its end; after one that some
+    // CTAs left at a barrier they are not.
+    if (!RES && w.tile == 0)
+        for (int i = threadIdx.x, nc = 1 + (s.tiles_r * s.tiles_c + PARTIAL_GROUP - 1) / PARTIAL_GROUP; i < nc; i += THREADS) s.counters[i] = 0;
     __syncthreads();      // (the shared arrays are free for the next item)
 }
 
@@ -1184,6 +1197,25 @@ GenericKernel pick_generic(int g, int p, int mode, int ctas) {
 }  // namespace
 
 int generic_tile_cols() { return G_CW; }
+
+// Self-test of the grid barrier: CTAs below `absent` leave without arriving, the others wait and record what they got.
+__global__ void k_selftest_grid_barrier(uint32_t* bar, int* status, int absent, uint32_t limit, int* observed) {
+    if ((int)blockIdx.x < absent) return;
+    const bool ok = grid_barrier(bar, status, limit);
+    if (threadIdx.x == 0) observed[blockIdx.x] = ok ? 1 : 0;
+}
+// One CTA of four stays away, then all four come: words = {status, barrier, observed[4], observed[4]}
+cudaError_t launch_selftest_grid_barrier(int* words, cudaStream_t st) {
+    for (int k = 0; k < 2; ++k) {
+        uint32_t* bar = reinterpret_cast<uint32_t*>(words + 1);
+        int *status = words, absent = k == 0, *observed = words + 2 + 4 * k;
+        uint32_t limit = k == 0 ? 4096u : G_POLL_LIMIT;
+        void* params[] = {&bar, &status, &absent, &limit, &observed};
+        const cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_selftest_grid_barrier), dim3(4), dim3(64), params, 0, st);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
 
 cudaError_t launch_generic(const KernelKey& key, const StepArgs& a, const CameHyper* host_hyp, int n_hyp, const GenericLists& l,
                            cudaStream_t st) {

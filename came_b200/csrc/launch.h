@@ -76,14 +76,15 @@ int persistent_grid_limit();
 constexpr int S_FIN_CHUNK = 2048;      // factor-vector entries one CTA of the clip finalize writes
 void fused_sq_geometry(int64_t cols, int elem_bytes, int* groups, int* ng, int* rb, int* slot_kb);
 bool fused_sq_eligible(int64_t cols, int elem_bytes);
-// whole-step kernel (generic.cu): its work lists and the two words of its grid barrier (zero before the first launch)
+// whole-step kernel (generic.cu): its work lists and the word of its grid barrier (zero before the first launch)
+constexpr int FLAT_GROUP = 8;
 struct GenericLists {
     const Work* tiles;      // matrix tiles
     const Work* vecs;       // blocks of 256 entries of the row, then the column vector
     const Work* flats;      // flat layout: blocks of 256 elements
     const Work* ones;       // 1-D tensors: blocks of 256 elements
-    int n_tiles, n_vecs, n_flats, n_ones;
-    int* bar;
+    int n_tiles, n_vecs, n_flats, n_ones;      // (n_flats: blocks, FLAT_GROUP per entry)
+    uint32_t* bar;
 };
 constexpr int GENERIC_MAX_HYP = 8;      // hyper-parameter records that travel as kernel arguments
 int generic_tile_cols();                 // columns of a warp's item
@@ -98,6 +99,7 @@ int nd_small_kb(int64_t rows, int64_t cols);
 // the same for 3 x 3 and 1 x 1 (nd_fixed.cu); key: element types, mode = 8-bit states | 3 x 3 << 1
 int nd_fixed_batch(int64_t rows, int64_t cols);
 cudaError_t launch_nd_fixed(int kernel, const KernelKey& key, const StepArgs& a, const Work* work, int n, cudaStream_t st);
+cudaError_t launch_selftest_grid_barrier(int* words, cudaStream_t st);
 cudaError_t launch_selftest_bounded_wait(int* status, int* observed, cudaStream_t st);
 
 cudaError_t launch_quantize_blockwise(const float* src, void* q, float* absmax, int64_t n, bool is_signed,

@@ -185,6 +185,15 @@ int came_b200_plan_status(came_plan_t* plan, came_stream_t stream, int* status);
  */
 int came_b200_selftest_bounded_wait(int* device_words, came_stream_t stream);
 
+/*
+ * Self-test of the whole-step kernel's grid barrier, without a step: enqueues two cooperative launches of four CTAs.  In
+ * the first one CTA never arrives and the others give up after 4096 polls; in the second all four arrive.  device_words:
+ * ten ints of device memory; after the stream has run they hold {1 (the status a timed-out wait records), 65536 (one
+ * generation, no arrival left over), -1, 0, 0, 0 (the first launch: the absent CTA, three that gave up), 1, 1, 1, 1}.
+ * No counterpart in the reference.
+ */
+int came_b200_selftest_grid_barrier(int* device_words, came_stream_t stream);
+
 /* Number of kernel launches the last came_b200_step on this plan enqueued. */
 int came_b200_plan_last_launches(const came_plan_t* plan);
 

@@ -98,3 +98,13 @@ def test_bounded_wait_runs_out_cleanly():
     opt.step()
     assert all(plan.status() == 0 for plan in opt._engine.plans.values())
     assert bool((p.data < 1.0).all())
+
+
+def test_grid_barrier_runs_out_cleanly():
+    """A CTA that never arrives ends the others' wait by its limit, and a later launch finds the barrier as new."""
+    from came_b200 import _lib
+    lib = _lib.load()
+    words = torch.full((10,), 7, device="cuda", dtype=torch.int32)
+    _lib.check(lib.came_b200_selftest_grid_barrier(words.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    assert words.tolist() == [1, 1 << 16, -1, 0, 0, 0, 1, 1, 1, 1]
