@@ -151,7 +151,9 @@ __device__ __forceinline__ bool last_warp(int* counter, int total, int lane) {
         if (before == total - 1) *counter = 0;
         fence_gpu();
     }
-    return __shfl_sync(0xffffffffu, before, 0) == total - 1;
+    before = __shfl_sync(0xffffffffu, before, 0);
+    __syncwarp();      // (a shuffle orders no memory: what lane 0 has acquired the other lanes may read from here on)
+    return before == total - 1;
 }
 // Sum of n partials, one per item, in index order: the last of every 64 items adds their partials (leave_partial); up to
 // 32 such groups the readers add themselves (read_sum: one load per lane, cheaper than one more chain of a fence, an atomic
