@@ -341,6 +341,7 @@ struct came_plan {
     bool has_fused_ma = false;
     std::vector<char> fused;       // per tensor: stepped by the fused momentum / apply kernel
     std::vector<char> pushable;    // ... or by the whole-step kernel, which serves the push mode too
+    std::vector<char> push_must;   // pushable whatever the size of the set: has to lie in the local buffer (else it is not pushed)
     bool needs_hyp = false;        // some kernel reads the hyper-parameters from the workspace
     int n_push = 0;                // push mode: peers that receive every parameter the fused kernel updates
     long long push_delta[MAX_PUSH_PEERS] = {};
@@ -622,8 +623,11 @@ int came_b200_plan_create(const CameTensorDesc* descs, int n_tensors, void* work
         }
     }
     plan->fused = fused;
-    plan->pushable = fused;
-    for (int i = 0; i < n_tensors; ++i) plan->pushable[i] = fused[i] || isgen(i);
+    plan->pushable = plan->push_must = fused;
+    for (int i = 0; i < n_tensors; ++i) {
+        plan->pushable[i] = fused[i] || isgen(i);
+        plan->push_must[i] = fused[i] || (isgen(i) && vf[i].wide && fused_ma_enabled() && D[i].g_dtype == D[i].p_dtype && D[i].mode != CAME_MODE_FP32);
+    }
     // The momentum pass, the residual finalize and the apply pass run wave by wave: a wave is a run of consecutive
     // tensors whose momentum state together stays below `wave_bytes`, so that the codes the momentum pass writes are
     // still in L2 when the apply pass reads them back (0: one wave, every pass covers all tensors).
@@ -701,7 +705,7 @@ int came_b200_plan_set_push(came_plan_t* plan, const void* local_base, size_t lo
     const uintptr_t buf_lo = reinterpret_cast<uintptr_t>(local_base), buf_hi = buf_lo + local_bytes;
     if (buf_lo % 16 != 0) return fail(CAME_E_INVALID, "plan_set_push: the local buffer is not 16-byte aligned");
     for (int i = 0; i < plan->n_tensors; ++i)
-        if (plan->pushable[i] && !param_in_range(buf_lo, buf_hi, plan->descs[i]))
+        if (plan->push_must[i] && !param_in_range(buf_lo, buf_hi, plan->descs[i]))
             return fail(CAME_E_INVALID, "plan_set_push: tensor %d does not lie inside the local buffer", i);
     long long delta[MAX_PUSH_PEERS];
     for (int k = 0; k < n_peers; ++k) {
@@ -719,7 +723,8 @@ int came_b200_plan_set_push(came_plan_t* plan, const void* local_base, size_t lo
 int came_b200_plan_pushed(const came_plan_t* plan, int* flags, int n_tensors) {
     if (!plan || !flags) return fail(CAME_E_INVALID, "plan_pushed: null argument");
     if (n_tensors != plan->n_tensors) return fail(CAME_E_INVALID, "plan_pushed: %d tensors given, plan has %d", n_tensors, plan->n_tensors);
-    for (int i = 0; i < n_tensors; ++i) flags[i] = plan->pushable[i] ? 1 : 0;
+    for (int i = 0; i < n_tensors; ++i)
+        flags[i] = plan->pushable[i] && (plan->n_push == 0 || pushed_param_in_range(*plan, plan->descs[i])) ? 1 : 0;
     return CAME_OK;
 }
 
@@ -736,7 +741,7 @@ int came_b200_plan_set_pointers(came_plan_t* plan, const void* const* g, void* c
         if (!next.g || !next.p) return fail(CAME_E_INVALID, "set_pointers: tensor %d: null pointer", i);
         if (!(vec_flags(next, fast) == plan->vflags[i]))
             return fail(CAME_E_INVALID, "set_pointers: tensor %d changes 16-byte alignment class; create a new plan", i);
-        if (plan->n_push > 0 && plan->pushable[i] && !pushed_param_in_range(*plan, next))
+        if (plan->n_push > 0 && plan->pushable[i] && pushed_param_in_range(*plan, plan->descs[i]) && !pushed_param_in_range(*plan, next))
             return fail(CAME_E_INVALID, "set_pointers: tensor %d leaves the buffer the push mode was set up for", i);
     }
     for (int i = 0; i < n_tensors; ++i) {
@@ -792,7 +797,7 @@ int came_b200_step(came_plan_t* plan, const CameHyper* hypers, int n_groups, cam
     StepArgs a{reinterpret_cast<const CameTensorDesc*>(plan->ws + plan->L.off_descs),
                reinterpret_cast<const Scratch*>(plan->ws + plan->L.off_scr),
                reinterpret_cast<const CameHyper*>(plan->ws + plan->L.off_hyp),
-               reinterpret_cast<int*>(plan->ws + plan->L.off_status), plan->n_push, 0, {}};
+               reinterpret_cast<int*>(plan->ws + plan->L.off_status), plan->n_push, 0, {}, plan->push_lo, plan->push_hi};
     for (int k = 0; k < plan->n_push; ++k) a.push_delta[k] = plan->push_delta[k];
     const Work* wbase = reinterpret_cast<const Work*>(plan->ws + plan->L.off_work);
     int* sync = reinterpret_cast<int*>(plan->ws + plan->L.off_sync);

@@ -653,6 +653,13 @@ __device__ __forceinline__ float g_apply_one(const Buf<TP>& b, float pv, float u
     return apply_step(pv, upd, h.lr, h.wd_lr, h.decay_mul, wd, [&](float x) { return b.round(x); });
 }
 
+// peers that receive a tensor's new values (push mode)
+__device__ __forceinline__ int peers_of(const StepArgs& a, const CameTensorDesc& d, int esz) {
+    if (a.n_push == 0) return 0;
+    const uintptr_t lo = reinterpret_cast<uintptr_t>(d.p);
+    return lo >= a.push_lo && lo + (uintptr_t)(d.rows * d.cols * esz) <= a.push_hi ? a.n_push : 0;
+}
+
 // p -= lr m R'_i C'_j with m read back from the state (came_kernels.cu:3332-3366, 2487-2511)
 template <typename TP, int MODE, int V>
 __device__ __forceinline__ void band_apply(const StepArgs& a, const CameHyper* hyp, const Item& it, const char* st, float& mean) {
@@ -685,7 +692,7 @@ __device__ __forceinline__ void band_apply(const StepArgs& a, const CameHyper* h
     const u64 k2 = splat(subtract ? -h.wd_lr : wd == 2 ? h.decay_mul : 1.0f), lr2 = splat(-h.lr);
     const Buf<TP> p(d.p, dt);
     const int64_t at = (int64_t)it.brow * it.C + it.col0 + Lane<V>::col(lane, 0);
-    const int live = it.R - it.brow, n_push = a.n_push;
+    const int live = it.R - it.brow, n_push = peers_of(a, d, esz);
 #pragma unroll
     for (int i = 0; i < NR; ++i) {
         const int r = Lane<V>::row(lane, i);
@@ -915,11 +922,12 @@ __device__ __forceinline__ void phase_apply_flat(const StepArgs& a, const CameHy
         const u64 t = fma2(lr2, pk(upd[e], upd[e + 1]), pk(pv[e], pv[e + 1]));
         pv[e] = t.x; pv[e + 1] = t.y;
     }
+    const int n_push = peers_of(a, d, size_of<TP>(d.p_dtype));
     if (V == 8) {
         if (cnt) {
             *reinterpret_cast<uint2*>(mq + i0) = make_uint2(lo, hi);
             p.put8(i0, pv);
-            for (int k = 0; k < a.n_push; ++k) p.put8(i0, pv, a.push_delta[k]);
+            for (int k = 0; k < n_push; ++k) p.put8(i0, pv, a.push_delta[k]);
         }
     } else {
 #pragma unroll
@@ -927,7 +935,7 @@ __device__ __forceinline__ void phase_apply_flat(const StepArgs& a, const CameHy
             if (e < cnt) {
                 mq[i0 + 32 * e] = (int8_t)((e < 4 ? lo : hi) >> (8 * (e & 3)));
                 p.put(i0 + 32 * e, pv[e]);
-                for (int k = 0; k < a.n_push; ++k) p.put(i0 + 32 * e, pv[e], a.push_delta[k]);
+                for (int k = 0; k < n_push; ++k) p.put(i0 + 32 * e, pv[e], a.push_delta[k]);
             }
     }
 }

@@ -323,6 +323,7 @@ class ShardedStepper:
             if o is None:
                 continue
             o.prime_for_cuda_graph()
+            o._engine.set_push(*self._push_args())      # (before asking: what is delivered depends on the local buffer)
             plans = list(o._engine.plans.values())
             flags = plans[0].pushed() if len(plans) == 1 and plans[0].n == len(idx) else [False] * len(idx)
             if not any(flags):

@@ -77,3 +77,36 @@ def test_bad_push_setups_are_refused():
     opt.step()                          # none of the refused calls left the plan in push mode
     torch.cuda.synchronize()
     assert plan.status() == 0 and not other.any()
+
+
+def test_odd_matrix_outside_the_local_buffer_is_left_out():
+    """A matrix that no staged path takes may lie elsewhere: the set-up is accepted, and it is not delivered."""
+    import came_b200
+    flat = torch.zeros(64 * 192, dtype=torch.bfloat16, device="cuda")
+    params = [torch.nn.Parameter(flat.view(64, 192)), torch.nn.Parameter(torch.zeros(33, 77, dtype=torch.bfloat16, device="cuda")),
+              torch.nn.Parameter(torch.zeros(40, 3, dtype=torch.bfloat16, device="cuda"))]
+    for p in params:
+        p.grad = torch.ones_like(p)
+    opt = came_b200.CAME8bit(params, lr=1e-3)
+    opt.prime_for_cuda_graph()
+    mirror = torch.zeros_like(flat)
+    opt._engine.set_push(flat.data_ptr(), 2 * flat.numel(), [mirror.data_ptr()])
+    (plan,) = opt._engine.plans.values()
+    assert plan.pushed() == [True, False, False]
+    params[1].grad = torch.ones_like(params[1])      # a new address: the plan is pointed at it
+    opt.step()
+    torch.cuda.synchronize()
+    assert plan.status() == 0 and torch.equal(mirror, flat) and bool((params[1].data != 0).all())
+    # inside the buffer it is delivered
+    both = torch.zeros(64 * 192 + 33 * 77 + 7, dtype=torch.bfloat16, device="cuda")
+    views = [both[:64 * 192].view(64, 192), both[64 * 192:64 * 192 + 33 * 77].view(33, 77)]
+    ps = [torch.nn.Parameter(v) for v in views]
+    for p in ps:
+        p.grad = torch.ones_like(p)
+    opt = came_b200.CAME8bit(ps, lr=1e-3)
+    opt.prime_for_cuda_graph()
+    mirror = torch.zeros(both.numel() + 7, dtype=torch.bfloat16, device="cuda")[:both.numel()]
+    opt._engine.set_push(both.data_ptr(), 2 * both.numel(), [mirror.data_ptr()])
+    opt.step()
+    torch.cuda.synchronize()
+    assert torch.equal(mirror, both) and bool((both[:64 * 192 + 33 * 77] != 0).all())
