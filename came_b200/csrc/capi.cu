@@ -943,8 +943,8 @@ int came_b200_plan_read_timing(came_plan_t* plan, float* ms, int* launches) {
 const char* came_b200_kernel_name(int kernel) {
     static const char* names[CAME_KERNEL_COUNT] = {
         "sq_partials", "sq_finalize", "sumsq", "s_finalize", "moment", "res_finalize",
-        "apply", "factors", "apply_flat", "nf_partial", "nf_apply", "nf_reduce", "nd_sq", "nd_mean", "nd_sumsq", "nd_s", "nd_res",
-        "nd_resmean", "nd_apply", "moment_apply", "generic"};
+        "apply", "generic", "apply_flat", "?", "?", "?", "nd_sq", "nd_mean", "nd_sumsq", "nd_s", "nd_res",
+        "nd_resmean", "nd_apply", "moment_apply"};
     return (kernel >= 0 && kernel < CAME_KERNEL_COUNT) ? names[kernel] : "?";
 }
 

@@ -40,12 +40,9 @@ enum KernelId {
     KID_MOMENT,
     KID_RES_FINALIZE,
     KID_APPLY,
-    KID_FACTORS,           // (part of KID_GENERIC)
+    KID_GENERIC,           // whole step of small sets, odd shapes and 1-D tensors (generic.cu)
     KID_APPLY_FLAT,
-    KID_NF_PARTIAL,        // (1-D tensors: part of KID_GENERIC; the numbers of the others stay)
-    KID_NF_APPLY,
-    KID_NF_REDUCE,
-    KID_ND_SQ,             // tensors of more than two dimensions (nd.cu)
+    KID_ND_SQ = 12,        // tensors of more than two dimensions (nd.cu); 9 to 11 are free, the numbers are part of the C interface
     KID_ND_MEAN,
     KID_ND_SUMSQ,
     KID_ND_S,
@@ -53,7 +50,6 @@ enum KernelId {
     KID_ND_RESMEAN,
     KID_ND_APPLY,
     KID_MOMENT_APPLY,      // momentum + residual finalize + apply of the tile layout as one kernel (fused_ma.cu)
-    KID_GENERIC,           // whole step of small sets, odd shapes and 1-D tensors (generic.cu)
     KID_COUNT
 };
 

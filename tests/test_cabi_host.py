@@ -32,6 +32,19 @@ def test_struct_layout_matches_header():
     assert C.sizeof(_lib.CameHyper) == 64
 
 
+def test_kernel_table_fits_callers_of_interface_version_1():
+    """read_timing fills arrays of the caller's CAME_KERNEL_COUNT: version 1 was published with 20."""
+    from came_b200 import _lib
+    lib = _lib.load()
+    header = open(os.path.join(ROOT, "include", "came_b200.h")).read()
+    assert lib.came_b200_version() == 1 and _lib.KERNEL_COUNT == 20
+    assert re.search(r"#define CAME_KERNEL_COUNT 20\b", header)
+    names = [lib.came_b200_kernel_name(k).decode() for k in range(20)]
+    assert {n: names.index(n) for n in ("sq_partials", "apply_flat", "nd_sq", "moment_apply")} == {
+        "sq_partials": 0, "apply_flat": 8, "nd_sq": 12, "moment_apply": 19}
+    assert "generic" in names and lib.came_b200_kernel_name(20) == b"?"
+
+
 def _desc(**kw):
     from came_b200 import _lib
     d = _lib.CameTensorDesc()
