@@ -87,7 +87,16 @@ VecFlags vec_flags(const CameTensorDesc& d, bool fast) {
 
 VecFlags vec_flags(const CameTensorDesc& d) { return vec_flags(d, !disable_fast()); }
 
-// Small sets: every matrix of a set with fewer elements than this on the staged path takes the whole-step kernel.
+// Small sets: every matrix of a set with fewer elements than this on the staged path takes the whole-step kernel; the flat
+// layout counts 4/3, as the whole-step kernel reads its gradients once more than the others'.  us a step, staged / whole-step
+// (p and g in bf16, fp32 for the last; one n x n matrix, or decoders of l layers of width h):
+//                            tile              flat              fp32
+//   n = 1024                  98 /  43         112 /  45         104 /  42
+//   n = 2048                 105 /  55         119 /  65         119 /  61
+//   n = 3072                 118 /  77         131 /  99         137 /  97
+//   n = 3840 (14 Mi)         125 / 105         138 / 138         151 / 132
+//   l = 4, h = 512 (13.5 Mi) 134 / 106         155 / 159         154 / 133
+//   l = 8, h = 512 (26.5 Mi) 161 / 184         193 / 304         230 / 255
 // CAME_B200_SMALL_SET_ELEMS overrides the line (0: none; read whenever a plan is sized or created).
 constexpr long long SMALL_SET_ELEMS = 16 << 20;
 
@@ -110,16 +119,28 @@ Context context(const CameTensorDesc* descs, int n) {
     const double line = e ? atof(e) : (double)SMALL_SET_ELEMS;
     double staged = 0.0;
     for (int i = 0; i < n; ++i)
-        if (vec_flags(descs[i]).wide) staged += (double)descs[i].rows * (double)descs[i].cols;
+        if (vec_flags(descs[i]).wide)
+            staged += (double)descs[i].rows * (double)descs[i].cols * (descs[i].mode == CAME_MODE_FLAT8 ? 4.0 / 3.0 : 1.0);
     Context c{staged < line, 16};
-    // As few bands per item as it takes to give every resident warp of the GPU (24 per SM) two items; more than 4, which
-    // only saves column partials and their summation, where every warp (16 per SM) still has eight to even the load out.
-    for (; c.bands > 1; c.bands /= 2) {
+    auto items = [&](int bands) {
         int64_t tiles = 0;
         for (int i = 0; i < n; ++i)
-            if (c.generic(descs[i])) tiles += generic_tiles(descs[i], c.bands);
-        if (tiles >= (c.bands > 4 ? 8 * 16 : 2 * 24) * 148) break;
-    }
+            if (c.generic(descs[i])) tiles += generic_tiles(descs[i], bands);
+        return tiles;
+    };
+    // Where it takes 8 bands or fewer: the fewest that leave no resident warp (16 per SM) a second item.  Fewer bands make
+    // more column partials, which the finalize phases add in one chain per column while the other CTAs wait at a barrier:
+    // one bf16 matrix of 3840 x 3840 takes 154 / 130 / 115 / 105 us at 1 / 2 / 4 / 8 bands, 16384 x 768 178 / 130 / 117 / 104,
+    // 1024 x 1024 43 / 48 / 58 / 67.
+    for (int b = 1; b <= 8; b *= 2)
+        if (items(b) <= 16 * 148) {
+            c.bands = b;
+            return c;
+        }
+    // Larger sets: as few bands per item as it takes to give every resident warp of the GPU (24 per SM) two items; more than 4, which
+    // only saves column partials and their summation, where every warp (16 per SM) still has eight to even the load out.
+    for (; c.bands > 1; c.bands /= 2)
+        if (items(c.bands) >= (c.bands > 4 ? 8 * 16 : 2 * 24) * 148) break;
     return c;
 }
 
