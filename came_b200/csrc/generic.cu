@@ -853,21 +853,22 @@ __device__ __forceinline__ void phase_apply_flat(const StepArgs& a, const CameHy
         }
     } else {
         float r[8], rr[8], c[8], rc[8];
-        if (C >= QBLOCK) {
-            // The block lies in at most two rows: their factors once, and every column factor's load independent of the
-            // others (bf16 set of width 1001: 1842 us with each load behind a test for a new row, 1758 us)
-            float ra, rra, rb, rrb;
+        if (C >= 32) {
+            // The block lies in at most nine rows: lane l forms the factors of the l-th of them, the elements get them by
+            // shuffles, and no column factor's load waits for a test for a new row.
             locate(b0, row, col);
-            row_factors(row, ra, rra);
-            row_factors(min(row + 1, (int)d.rows - 1), rb, rrb);
+            float fr, frr;
+            row_factors(row + min(lane, (int)d.rows - 1 - row), fr, frr);
+            uint32_t at = (uint32_t)col + (uint32_t)lane, k = at / (uint32_t)C;
+            at -= k * (uint32_t)C;
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-                const int at = col + j0 + 32 * e;
-                const bool next = at >= C;
-                c[e] = e < cnt ? s.vc[next ? at - C : at] : 0.0f;
-                rc[e] = e < cnt ? s.Rc[next ? at - C : at] : 0.0f;
-                r[e] = next ? rb : ra;
-                rr[e] = next ? rrb : rra;
+                r[e] = __shfl_sync(0xffffffffu, fr, k);
+                rr[e] = __shfl_sync(0xffffffffu, frr, k);
+                c[e] = e < cnt ? s.vc[at] : 0.0f;
+                rc[e] = e < cnt ? s.Rc[at] : 0.0f;
+                at += 32;
+                if (at >= (uint32_t)C) { at -= (uint32_t)C; ++k; }
             }
         } else {
             int have = -1;      // row the factors r, rr belong to
