@@ -36,6 +36,7 @@ using Owned = std::unique_ptr<PyObject, Unref>;
 
 struct Param {                    // (no reference to the parameter: swap_tensors() and the garbage collector count them)
     PyObject* obj;                // borrowed from the group's list: compared with what the list holds now
+    PyTypeObject* type;
     bool has_grad;
     at::ScalarType p_type, g_type;
     const void *p_ptr, *g_ptr;
@@ -112,7 +113,7 @@ bool build(StepTable* s, PyObject* groups, PyObject* plans, PyObject* states) {
         for (Py_ssize_t i = 0; ok && i < PyList_GET_SIZE(list); ++i) {
             PyObject* obj = PyList_GET_ITEM(list, i);
             if (!THPVariable_Check(obj)) { ok = false; break; }
-            Param e{obj, false, at::kFloat, at::kFloat, nullptr, nullptr, {}, -1, -1};
+            Param e{obj, Py_TYPE(obj), false, at::kFloat, at::kFloat, nullptr, nullptr, {}, -1, -1};
             const at::Tensor& t = THPVariable_Unpack(obj);
             const at::Tensor& g = t.grad();
             if (g.defined()) {
@@ -244,7 +245,7 @@ long step(StepTable* s, PyObject* groups) {
         if (!list || !PyList_Check(list) || (size_t)PyList_GET_SIZE(list) != ps.size()) return SLOW;
         for (size_t i = 0; i < ps.size(); ++i) {
             Param& e = ps[i];
-            if (PyList_GET_ITEM(list, (Py_ssize_t)i) != e.obj || !THPVariable_Check(e.obj)) return SLOW;
+            if (PyList_GET_ITEM(list, (Py_ssize_t)i) != e.obj || Py_TYPE(e.obj) != e.type) return SLOW;
             const at::Tensor& t = THPVariable_Unpack(e.obj);
             const at::Tensor& g = t.grad();
             if (g.defined() != e.has_grad) return SLOW;
@@ -260,16 +261,10 @@ long step(StepTable* s, PyObject* groups) {
             }
         }
     }
-    std::vector<Owned> states, counts;      // the states' new step counts: all of them are formed before the first is stored
+    // The states' step counts go up for all or for none: what does not simply add is left to the Python path.
     for (PyObject* d : *s->states) {
-        Py_INCREF(d);
-        states.emplace_back(d);
         PyObject* v = PyDict_GetItemWithError(d, s->k_step);
-        counts.emplace_back(v ? PyNumber_Add(v, s->one) : nullptr);
-        if (!counts.back()) {
-            PyErr_Clear();      // the Python path raises what there is to raise
-            return SLOW;
-        }
+        if (!v || !(PyLong_CheckExact(v) || PyFloat_CheckExact(v))) return SLOW;
     }
     CameHyper hyp[64];
     for (size_t gi = 0; gi < n_groups; ++gi)
@@ -291,8 +286,11 @@ long step(StepTable* s, PyObject* groups) {
             if (rc != CAME_OK) return FAILED + rc;
         }
     }
-    for (size_t i = 0; i < counts.size(); ++i)
-        if (PyDict_SetItem(states[i].get(), s->k_step, counts[i].get()) != 0) return SLOW;
+    for (PyObject* d : *s->states) {
+        PyObject* v = PyDict_GetItemWithError(d, s->k_step);
+        const Owned next(v ? PyNumber_Add(v, s->one) : nullptr);
+        if (!next || PyDict_SetItem(d, s->k_step, next.get()) != 0) return SLOW;
+    }
     long launches = 0;
     NoGil unlocked;
     for (const Target& t : targets) {
