@@ -234,23 +234,23 @@ template <int ESZ>
 __device__ __forceinline__ void stage_rows(char* dst, int pitch, const void* base, int esz, const Item& it, int lane) {
     const uintptr_t b = reinterpret_cast<uintptr_t>(base);
     const uintptr_t first = b + (uintptr_t)(((int64_t)it.brow * it.C + it.col0) * esz);
-    auto rows_on = [&](int r) { return (int64_t)r * it.C * esz; };      // (bytes; a row may be longer than 2^31)
     if constexpr (ESZ > 0) {
         constexpr int NCH = G_CW * ESZ / 16;
-        if (it.R - it.brow >= 16 && it.C - it.col0 >= G_CW) {
-            if (((first | (uintptr_t)rows_on(1)) & 15) == 0) {
+        if (it.R - it.brow >= 16 && it.C - it.col0 >= G_CW && it.C < (1 << 29)) {
+            const int pitch_g = it.C * ESZ;      // (below 2^31: one multiplication to 64 bits per address)
+            if (((first | (uintptr_t)pitch_g) & 15) == 0) {
                 const int r = lane / NCH, ch = lane % NCH;
-                const char* src = reinterpret_cast<const char*>(first) + rows_on(r) + 16 * ch;
+                const char* src = reinterpret_cast<const char*>(first) + (int64_t)r * pitch_g + 16 * ch;
                 char* to = dst + r * pitch + 16 * ch;
 #pragma unroll
-                for (int k = 0; k < NCH / 2; ++k, src += rows_on(32 / NCH), to += 32 / NCH * pitch) cp16(to, src, 16);
+                for (int k = 0; k < NCH / 2; ++k, src += (int64_t)(32 / NCH) * pitch_g, to += 32 / NCH * pitch) cp16(to, src, 16);
                 return;
             }
             if (it.R - it.brow > 16) {      // (a row follows: the last chunk stays inside the array)
 #pragma unroll
                 for (int k = 0; k < (16 * (NCH + 1) + 31) / 32; ++k) {
                     const int j = lane + 32 * k, r = j / (NCH + 1), ch = j - r * (NCH + 1);
-                    const uintptr_t src = ((first + (uintptr_t)rows_on(r)) & ~(uintptr_t)15) + 16 * ch;
+                    const uintptr_t src = ((first + (uintptr_t)((int64_t)r * pitch_g)) & ~(uintptr_t)15) + 16 * ch;
                     if (j < 16 * (NCH + 1)) cp16(dst + r * pitch + 16 * ch, reinterpret_cast<const void*>(src), 16);
                 }
                 return;
@@ -261,7 +261,7 @@ __device__ __forceinline__ void stage_rows(char* dst, int pitch, const void* bas
     const uintptr_t end = b + (uintptr_t)((int64_t)it.R * it.C * esz);
     for (int j = lane; j < 16 * nch; j += 32) {
         const int r = j / nch, ch = j - r * nch;
-        const uintptr_t row = first + (uintptr_t)rows_on(r), src = (row & ~(uintptr_t)15) + 16 * ch;
+        const uintptr_t row = first + (uintptr_t)((int64_t)r * it.C * esz), src = (row & ~(uintptr_t)15) + 16 * ch;
         const bool want = r < rows && src < row + width;
         cp16(dst + r * pitch + 16 * ch, reinterpret_cast<const void*>(want ? src : b & ~(uintptr_t)15),
              want ? (int)min((uintptr_t)16, end - src) : 0);
