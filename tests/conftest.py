@@ -12,6 +12,19 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (run with -m gpu on a B200)")
 
 
+@pytest.fixture(params=["staged", "whole-step"])
+def route(request, monkeypatch):
+    """The two routes of a matrix that the staged kernels take in large sets and the whole-step kernel in small ones: the
+    line between them is moved below or above every set of the test (a plan reads it when it is sized and created)."""
+    monkeypatch.setenv("CAME_B200_SMALL_SET_ELEMS", "0" if request.param == "staged" else "1e18")
+    return request.param
+
+
+@pytest.fixture
+def staged(monkeypatch):
+    monkeypatch.setenv("CAME_B200_SMALL_SET_ELEMS", "0")
+
+
 def pytest_collection_modifyitems(config, items):
     try:
         import torch

@@ -44,6 +44,19 @@ STATE_KEYS_F = ["exp_avg_absmax", "exp_avg_sq_row_absmax", "exp_avg_sq_col_absma
                 "exp_avg_res_row", "exp_avg_res_col", "exp_avg_sq"]
 
 
+def kernels_of(opt) -> set:
+    """Steps once more; the names of the kernels that were launched."""
+    plans = list(opt._engine.plans.values())
+    for plan in plans:
+        plan.set_timing(True)
+    opt.step()
+    names = set()
+    for plan in plans:
+        names |= set(plan.read_timing())
+        plan.set_timing(False)
+    return names
+
+
 def relerr(a: torch.Tensor, b: torch.Tensor) -> float:
     a, b = a.double(), b.double()
     return ((a - b).norm() / b.norm().clamp_min(1e-300)).item()

@@ -11,7 +11,7 @@ import pytest
 import torch
 
 from oracle import came_oracle as orc
-from tests.parity_util import run_pair
+from tests.parity_util import kernels_of, run_pair
 from tests.test_gpu_parity import H_DEFAULT, H_LLAMA, _check_8bit, _check_fp, _dt
 
 pytestmark = pytest.mark.gpu
@@ -29,7 +29,7 @@ def _status_ok(opt):
 @pytest.mark.parametrize("cls_name,preset2d,f16", [("CAME8bit", "TILE8", False), ("CAME8bit2D", "TILE8", False),
                                                    ("CAME8bitFull", "FLAT8", False), ("CAME8bitMemory", "FLAT8", True)])
 @pytest.mark.parametrize("dtype", ["bfloat16", "float16", "float32"])
-def test_8bit_classes_at_bench_columns(cls_name, preset2d, f16, dtype):
+def test_8bit_classes_at_bench_columns(cls_name, preset2d, f16, dtype, staged):
     import came_b200
     shapes = [s for s in BENCH_SHAPES if len(s) == 2 or cls_name != "CAME8bit2D"]
     preset = lambda dim: getattr(orc, preset2d) if dim == 2 else orc.FLAT8
@@ -40,7 +40,7 @@ def test_8bit_classes_at_bench_columns(cls_name, preset2d, f16, dtype):
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
-def test_camecuda_at_bench_columns(dtype):
+def test_camecuda_at_bench_columns(dtype, staged):
     import came_b200
     out, opt, _ = run_pair(came_b200.CAMECUDA, lambda dim: orc.CUDAFP, BENCH_SHAPES, _dt(dtype), 6, H_DEFAULT, seed=32,
                            per_tensor_scale=True)
@@ -49,7 +49,7 @@ def test_camecuda_at_bench_columns(dtype):
 
 
 @pytest.mark.parametrize("cls_name,preset2d", [("CAME8bit", "TILE8"), ("CAME8bitFull", "FLAT8")])
-def test_vocab_wide_rows(cls_name, preset2d):
+def test_vocab_wide_rows(cls_name, preset2d, route):
     """Rows too wide for the staged first pass take the two-pass kernels while the momentum / apply passes stay on
     the staged path (a [hidden, vocab]-shaped matrix)."""
     import came_b200
@@ -58,6 +58,7 @@ def test_vocab_wide_rows(cls_name, preset2d):
                            per_tensor_scale=True)
     _check_8bit(out, torch.bfloat16)
     _status_ok(opt)
+    assert ({"sq_partials", "sumsq", "moment_apply"} <= kernels_of(opt)) == (route == "staged")
 
 
 @pytest.mark.parametrize("shape,steps", [((4096, 11008), 2), ((32000, 4096), 1)])
@@ -70,7 +71,7 @@ def test_full_size_matrix(shape, steps):
     _status_ok(opt)
 
 
-def test_camecuda_zero_rows_and_columns_take_the_clamped_path():
+def test_camecuda_zero_rows_and_columns_take_the_clamped_path(route):
     """CAMECUDA clamps its factors at 1e-30 (came_kernels.cu:577, 591-592).  The staged first pass derives the clip sum
     from a closed form that holds while no clamp binds; rows and columns whose gradient is identically zero make one
     bind (v = (1 - beta2) * eps0 ~ 1e-33), and the step must then fall back to the explicit sum and still match."""
@@ -96,3 +97,4 @@ def test_camecuda_zero_rows_and_columns_take_the_clamped_path():
         assert relerr(p.data.cpu(), c) <= 1e-5
         for k in ("exp_avg", "exp_avg_sq_row", "exp_avg_sq_col", "exp_avg_res_row", "exp_avg_res_col"):
             assert relerr(opt.state[p][k].cpu(), st[k]) <= 1e-4, k
+    assert ({"sq_partials", "sumsq", "moment", "apply"} <= kernels_of(opt)) == (route == "staged")

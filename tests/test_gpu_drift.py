@@ -92,7 +92,7 @@ def drift_trajectory(cls_name, preset2d, update_f16, shapes, steps=STEPS, every=
     ("CAME8bitMemory", orc.FLAT8, True, SHAPES),
     ("CAME8bit2D", orc.TILE8, False, [s for s in SHAPES if len(s) == 2]),
 ])
-def test_200_step_drift_stays_bounded(cls_name, preset2d, f16, shapes):
+def test_200_step_drift_stays_bounded(cls_name, preset2d, f16, shapes, route):
     records = drift_trajectory(cls_name, preset2d, f16, shapes)
     assert len(records) == STEPS // EVERY
     for rec in records:

@@ -8,10 +8,10 @@ import pytest
 import torch
 
 from oracle import came_oracle as orc
-from tests.parity_util import run_pair, relerr
+from tests.parity_util import kernels_of, relerr, run_pair
 from tests.test_gpu_parity import H_DEFAULT, _check_fp, _dt
 
-pytestmark = pytest.mark.gpu
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("staged")]      # (as small sets they would take the whole-step kernel)
 
 SHAPES = [(130, 1088), (257, 2304), (64, 64), (7, 192), (1000, 1024), (300, 4096), (129, 3072)]
 
@@ -29,6 +29,8 @@ def _run(dtype, disable_fast, wd, steps=3):
             opt.step()
         for plan in opt._engine.plans.values():
             assert plan.status() == 0
+        names = kernels_of(opt)      # (a step more, on both sides)
+        assert names == {"generic"} if disable_fast else {"moment", "apply"} <= names and "generic" not in names
         return params, opt
     finally:
         os.environ.pop("CAME_B200_DISABLE_FAST", None)
@@ -62,3 +64,4 @@ def test_staged_against_oracle(dtype):
     _check_fp(out, _dt(dtype))
     for plan in opt._engine.plans.values():
         assert plan.status() == 0
+    assert {"moment", "apply"} <= kernels_of(opt)

@@ -4,6 +4,8 @@ gradients and a changing learning rate must leave exactly the bytes the eager st
 import pytest
 import torch
 
+from tests.parity_util import kernels_of
+
 pytestmark = pytest.mark.gpu
 
 SHAPES = [(256, 512), (384, 1024), (128, 192), (4096,), (300,)]
@@ -23,7 +25,7 @@ def _make(cls_name, dtype, **kw):
     ("CAME8bitMemory", torch.bfloat16, {}),
     ("CAMECUDA", torch.float32, {}),
 ])
-def test_captured_step_equals_eager(cls_name, dtype, kw):
+def test_captured_step_equals_eager(cls_name, dtype, kw, route):
     steps = 5
     gen = torch.Generator(device="cuda").manual_seed(9)
     grads = [[(torch.randn(s, device="cuda", generator=gen) * 1e-2).to(dtype) for s in SHAPES] for _ in range(steps)]
@@ -69,6 +71,7 @@ def test_captured_step_equals_eager(cls_name, dtype, kw):
                 assert torch.equal(va, sb[key]), key
     for plan in og._engine.plans.values():
         assert plan.status() == 0
+    assert ("sq_partials" in kernels_of(og)) == (route == "staged")
 
 
 def test_set_hyper_rejects_bad_records():

@@ -40,7 +40,7 @@ def _change(kind, step, ps, opt):
 
 
 @pytest.mark.parametrize("kind", ["same", "moved", "lr", "scale", "none", "strided", "unaligned"])
-def test_table_equals_full_path(kind):
+def test_table_equals_full_path(kind, route):
     (pa, oa), (pb, ob) = _make(), _make()
     keep = []
     for step in range(4):

@@ -12,7 +12,7 @@ import torch
 
 from oracle import came_oracle as orc
 from tests.golden.make_golden import codec_inputs
-from tests.parity_util import run_pair
+from tests.parity_util import kernels_of, run_pair
 
 pytestmark = pytest.mark.gpu
 
@@ -124,7 +124,7 @@ CASES_FP = [("CAME", orc.CAME), ("CAMECUDA", orc.CUDAFP)]
 @pytest.mark.parametrize("cls_name,preset", CASES_FP)
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16", "float16"])
 @pytest.mark.parametrize("shapes,hyper", [(EDGE_SHAPES, H_DEFAULT), (ALIGNED_SHAPES, H_LLAMA), (ALIGNED_SHAPES, H_NOWD)])
-def test_fp32_state_classes(cls_name, preset, dtype, shapes, hyper):
+def test_fp32_state_classes(cls_name, preset, dtype, shapes, hyper, route):
     import came_b200
     out, _, _ = run_pair(getattr(came_b200, cls_name), lambda dim: preset, shapes, _dt(dtype), 6, hyper, seed=11)
     _check_fp(out, _dt(dtype))
@@ -132,7 +132,7 @@ def test_fp32_state_classes(cls_name, preset, dtype, shapes, hyper):
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16", "float16"])
 @pytest.mark.parametrize("shapes,hyper", [(EDGE_SHAPES, H_DEFAULT), (ALIGNED_SHAPES, H_LLAMA), (ALIGNED_SHAPES, H_NOWD)])
-def test_came8bit(dtype, shapes, hyper):
+def test_came8bit(dtype, shapes, hyper, route):
     import came_b200
     preset = lambda dim: orc.TILE8 if dim == 2 else orc.FLAT8
     out, opt, gp = run_pair(came_b200.CAME8bit, preset, shapes, _dt(dtype), 6, hyper, seed=12)
@@ -142,7 +142,7 @@ def test_came8bit(dtype, shapes, hyper):
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
-def test_came8bit2d(dtype):
+def test_came8bit2d(dtype, route):
     import came_b200
     shapes = [s for s in EDGE_SHAPES + ALIGNED_SHAPES if len(s) == 2]
     out, _, _ = run_pair(came_b200.CAME8bit2D, lambda dim: orc.TILE8, shapes, _dt(dtype), 6, H_LLAMA, seed=13)
@@ -152,7 +152,7 @@ def test_came8bit2d(dtype):
 @pytest.mark.parametrize("cls_name,f16", [("CAME8bitFull", False), ("CAME8bitMemory", True)])
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16", "float16"])
 @pytest.mark.parametrize("shapes,hyper", [(EDGE_SHAPES, H_DEFAULT), (ALIGNED_SHAPES, H_LLAMA)])
-def test_flat_classes(cls_name, f16, dtype, shapes, hyper):
+def test_flat_classes(cls_name, f16, dtype, shapes, hyper, route):
     import came_b200
     out, opt, gp = run_pair(getattr(came_b200, cls_name), lambda dim: orc.FLAT8, shapes, _dt(dtype), 6, hyper, seed=14,
                             oracle_kw=dict(update_f16=f16))
@@ -169,13 +169,14 @@ MANY_ITEM_SHAPES = [(38400, 64), (12800, 256), (6400, 1280), (4096,)]
 
 @pytest.mark.parametrize("cls_name,preset2d", [("CAME8bit", "TILE8"), ("CAME8bitFull", "FLAT8")])
 @pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
-def test_many_items_per_cta(cls_name, preset2d, dtype):
+def test_many_items_per_cta(cls_name, preset2d, dtype, route):
     import came_b200
     preset = lambda dim: getattr(orc, preset2d) if dim == 2 else orc.FLAT8
     out, opt, gp = run_pair(getattr(came_b200, cls_name), preset, MANY_ITEM_SHAPES, _dt(dtype), 2, H_LLAMA, seed=21)
     _check_8bit(out, _dt(dtype))
     for plan in opt._engine.plans.values():
         assert plan.status() == 0
+    assert ("moment_apply" in kernels_of(opt)) == (route == "staged")
 
 
 def test_mixed_grad_dtype_takes_flat_layout():
@@ -190,7 +191,7 @@ def test_mixed_grad_dtype_takes_flat_layout():
     assert opt.state[p]["_mode"] == "full8bit"
 
 
-def test_bit_reproducible():
+def test_bit_reproducible(route):
     """Two optimizers fed the same inputs end with identical bytes (fixed-order reductions, no float atomics)."""
     import came_b200
     from tests.parity_util import make_inputs
@@ -326,7 +327,7 @@ def test_sharded_stepper_checkpoint_round_trip():
         st2.load_state_dict(bad)
 
 
-def test_grad_scale_is_applied_on_load():
+def test_grad_scale_is_applied_on_load(route):
     """`grad_scale` of a param_group multiplies every gradient as the kernels read it.  A power of two commutes with
     every rounding, so stepping 1024 * g with grad_scale = 1 / 1024 must leave exactly the bytes of stepping g; a
     general scale is compared with the oracle fed the scaled gradients."""

@@ -5,6 +5,8 @@ GPUs: tests/test_gpu_peer_gather.py.)  No counterpart in the reference, which is
 import pytest
 import torch
 
+from tests.parity_util import kernels_of
+
 pytestmark = pytest.mark.gpu
 
 SHAPES = [(256, 1024), (4096,), (130, 2304), (64, 192), (300,), (129, 1088)]
@@ -31,7 +33,7 @@ def _setup(cls_name, dtype):
 
 @pytest.mark.parametrize("cls_name,dtype", [("CAME8bit", torch.bfloat16), ("CAME8bit", torch.float32),
                                             ("CAME8bitFull", torch.bfloat16)])
-def test_mirror_receives_exactly_the_pushed_tensors(cls_name, dtype):
+def test_mirror_receives_exactly_the_pushed_tensors(cls_name, dtype, route):
     flat, params, opt = _setup(cls_name, dtype)
     mirrors = [torch.zeros_like(flat) for _ in range(2)]
     nbytes = flat.numel() * flat.element_size()
@@ -59,9 +61,10 @@ def test_mirror_receives_exactly_the_pushed_tensors(cls_name, dtype):
     torch.cuda.synchronize()
     for m, b in zip(mirrors, before):
         assert torch.equal(m, b)
+    assert ("moment_apply" in kernels_of(opt)) == (route == "staged")
 
 
-def test_bad_push_setups_are_refused():
+def test_bad_push_setups_are_refused(route):
     flat, params, opt = _setup("CAME8bit", torch.bfloat16)
     (plan,) = opt._engine.plans.values()
     nbytes = flat.numel() * flat.element_size()

@@ -2,7 +2,9 @@
 import pytest
 import torch
 
-from tests.parity_util import make_inputs
+from oracle import came_oracle as orc
+from tests.parity_util import make_inputs, run_pair
+from tests.test_gpu_parity import _check_8bit, _check_fp
 
 pytestmark = pytest.mark.gpu
 
@@ -49,3 +51,87 @@ def test_vector_whose_clip_divisor_is_infinite(cls_name, n):
     for _ in range(2):
         opt.step()
     assert torch.equal(p.data, before)
+
+
+PRESETS = [("CAME8bit", lambda dim: orc.TILE8 if dim == 2 else orc.FLAT8), ("CAME8bitFull", lambda dim: orc.FLAT8),
+           ("CAMECUDA", lambda dim: orc.CUDAFP)]
+MATRICES = [(256, 512), (130, 1088), (33, 77), (16, 8), (300,)]
+
+
+@pytest.mark.parametrize("cls_name,preset", PRESETS)
+def test_gradients_that_are_all_zero(cls_name, preset, route):
+    import came_b200
+    out, _, _ = run_pair(getattr(came_b200, cls_name), preset, MATRICES, torch.float32, 3, H, seed=6, grad_scale=0.0)
+    (_check_fp if cls_name == "CAMECUDA" else _check_8bit)(out, torch.float32)
+
+
+@pytest.mark.parametrize("cls_name", ["CAME8bit", "CAME8bitFull", "CAMECUDA"])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_a_poisoned_gradient_stays_in_its_tensor(cls_name, value, route):
+    """Every wait ends, and the other tensors get the bytes they get without it."""
+    import came_b200
+    shapes = MATRICES + [(6, 3, 3), (5, 2, 40, 24)]
+    params0, grads = make_inputs(shapes, torch.bfloat16, 2, seed=7)
+    results = []
+    for bad in range(-1, len(shapes)):
+        ps = [torch.nn.Parameter(p.cuda()) for p in params0]
+        opt = getattr(came_b200, cls_name)(ps, **H)
+        for gs in grads:
+            for i, (p, g) in enumerate(zip(ps, gs)):
+                p.grad = g.cuda()
+                if i == bad:
+                    p.grad.view(-1)[p.numel() // 2] = value
+            opt.step()
+        assert all(plan.status() == 0 for plan in opt._engine.plans.values())
+        results.append([p.data for p in ps])
+        for i, (a, b) in enumerate(zip(results[0], results[-1])):
+            assert bool(b.isfinite().all()) == (i != bad), (i, bad)
+            assert i == bad or torch.equal(a, b), (i, bad)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_flat_layout_off_the_16_byte_boundary(dtype):
+    """Parameters and gradients at odd elements of larger buffers: the same bytes as on the boundary (odd widths: the same
+    arithmetic), and nothing is written beside them."""
+    import came_b200
+    shapes = [(37, 201), (64, 777), (100, 21), (9, 31), (257, 5)]
+    params0, grads = make_inputs(shapes, dtype, 3, seed=8)
+    finals = []
+    for shift in (0, 1, 3):
+        def place(t):
+            big = torch.full((t.numel() + 8,), 7.0, dtype=dtype, device="cuda")
+            view = big[shift:shift + t.numel()].view(t.shape)
+            view.copy_(t)
+            return big, view
+        placed = [place(p) for p in params0]
+        ps = [torch.nn.Parameter(v) for _, v in placed]
+        opt = came_b200.CAME8bitFull(ps, **H)
+        for gs in grads:
+            for p, g in zip(ps, gs):
+                p.grad = place(g)[1]
+            opt.step()
+        for (big, v) in placed:
+            assert bool((big[:shift] == 7.0).all()) and bool((big[shift + v.numel():] == 7.0).all())
+        finals.append([p.data.clone() for p in ps] + [v.clone() for p in ps for _, v in sorted(opt.state[p].items()) if torch.is_tensor(v)])
+    for other in finals[1:]:
+        for a, b in zip(finals[0], other):
+            assert torch.equal(a, b)
+
+
+def test_more_param_groups_than_the_launch_carries():
+    """Up to four groups travel as kernel arguments, more are read from the workspace: the same bytes."""
+    import came_b200
+    shapes = [(33, 77), (64, 48), (300,), (40, 24), (17, 16), (5,)]
+    params0, grads = make_inputs(shapes, torch.bfloat16, 3, seed=9)
+    finals = []
+    for groups in (1, 4, 5, 6):
+        ps = [torch.nn.Parameter(p.cuda()) for p in params0]
+        opt = came_b200.CAME8bit([dict(params=ps[k:k + 1] if k < groups - 1 else ps[k:]) for k in range(groups)], **H)
+        for gs in grads:
+            for p, g in zip(ps, gs):
+                p.grad = g.cuda()
+            opt.step()
+        finals.append([p.data for p in ps])
+    for other in finals[1:]:
+        for a, b in zip(finals[0], other):
+            assert torch.equal(a, b)
