@@ -263,8 +263,8 @@ class ShardedStepper:
     bucket b travels over NVLink while bucket b+1 is being stepped.  `gather_mode`: "nccl" (in-place
     all_gather_into_tensor per bucket), "peer" (copy-engine pulls over CUDA IPC mappings, see PeerGather) or "push":
     the kernel that applies a tensor's update stores the new weights into every peer's buffer as it goes (plain stores
-    over NVLink into the same IPC mappings), so there is no separate exchange pass for those tensors; what the fused
-    kernel does not step (1-D tensors, odd shapes) is still pulled, and one small all-reduce after the step orders
+    over NVLink into the same IPC mappings), so there is no separate exchange pass for those tensors; what no
+    kernel delivers (1-D and N-D tensors, the fp32 layout of large sets) is still pulled, and one small all-reduce after the step orders
     every rank's stores before anybody reads the weights."""
 
     def __init__(self, sharded: ShardedParams, params_by_index: dict, make_optimizer, gather_mode: str = "nccl",
@@ -310,7 +310,7 @@ class ShardedStepper:
     def reset_push(self) -> None:
         """Push mode: forget which tensors the kernels deliver.  The next `step()` works it out again (a collective:
         call this on every rank) -- needed when the tensors of an optimizer, their dtypes or their alignment changed
-        after the first step, since a tensor that leaves the fused kernel must be pulled from then on."""
+        after the first step, since a tensor that no kernel delivers any more must be pulled."""
         self._push_ranges = None
 
     def _setup_push(self) -> None:
