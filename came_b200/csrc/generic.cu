@@ -762,9 +762,9 @@ __device__ __forceinline__ void issue_flat(const StepArgs& a, const Work& w, cha
     if (lane == 0) cp4(slot + S::OFF_X, d.m_absmax + w.tile);
 }
 struct FlatTensor {      // what a warp's blocks of one tensor share: formed once, not per block of 8 elements per lane
-    int tensor = -1;
+    int tensor = -1, n_push;
     float inv_clip, mean, inv;
-    __device__ __forceinline__ void use(const StepArgs& a, const CameHyper* hyp, int t, int lane) {
+    __device__ __forceinline__ void use(const StepArgs& a, const CameHyper* hyp, int t, int p_size, int lane) {
         if (t == tensor) return;
         tensor = t;
         const CameTensorDesc& d = a.descs[t];
@@ -772,6 +772,7 @@ struct FlatTensor {      // what a warp's blocks of one tensor share: formed onc
         inv_clip = read_inv_clip(s, hyp[d.group], d.rows * d.cols, lane);
         mean = read_mean(s.rowblk2, s.nbR, (int)d.rows, d.flags & CAME_F_RESROW_FIX, d.flags & CAME_F_RESROW_CLAMP, lane);
         inv = 1.0f / mean;
+        n_push = peers_of(a, d, p_size);
     }
 };
 template <typename TG, typename TP, typename S, int V>
@@ -923,12 +924,11 @@ __device__ __forceinline__ void phase_apply_flat(const StepArgs& a, const CameHy
         const u64 t = fma2(lr2, pk(upd[e], upd[e + 1]), pk(pv[e], pv[e + 1]));
         pv[e] = t.x; pv[e + 1] = t.y;
     }
-    const int n_push = peers_of(a, d, size_of<TP>(d.p_dtype));
     if (V == 8) {
         if (cnt) {
             *reinterpret_cast<uint2*>(mq + i0) = make_uint2(lo, hi);
             p.put8(i0, pv);
-            for (int k = 0; k < n_push; ++k) p.put8(i0, pv, a.push_delta[k]);
+            for (int k = 0; k < ft.n_push; ++k) p.put8(i0, pv, a.push_delta[k]);
         }
     } else {
 #pragma unroll
@@ -936,7 +936,7 @@ __device__ __forceinline__ void phase_apply_flat(const StepArgs& a, const CameHy
             if (e < cnt) {
                 mq[i0 + 32 * e] = (int8_t)((e < 4 ? lo : hi) >> (8 * (e & 3)));
                 p.put(i0 + 32 * e, pv[e]);
-                for (int k = 0; k < n_push; ++k) p.put(i0 + 32 * e, pv[e], a.push_delta[k]);
+                for (int k = 0; k < ft.n_push; ++k) p.put(i0 + 32 * e, pv[e], a.push_delta[k]);
             }
     }
 }
@@ -1156,7 +1156,7 @@ __global__ void __launch_bounds__(THREADS, CTAS) k_step_generic(const __grid_con
             }
             cp_commit();
             const Work w = ahead[0];
-            ft.use(a, hyp, w.tensor, lane);
+            ft.use(a, hyp, w.tensor, size_of<TP>(a.descs[w.tensor].p_dtype), lane);
             cp_wait<F::COUNT - 1>();
             __syncwarp();
             if (a.scr[w.tensor].g_v == 8) phase_apply_flat<TG, TP, F, 8>(a, hyp, w, ft, stages + slot * F::BYTES);
