@@ -20,7 +20,7 @@ constexpr int MAX_GROUPS = 64;
 constexpr size_t ALIGN = 256;
 
 thread_local char g_err[512] = "";
-// CAME_B200_DISABLE_FAST=1 in the environment routes every tensor through the generic kernels (used by the
+// CAME_B200_DISABLE_FAST=1 in the environment routes every matrix through the whole-step kernel (used by the
 // tests to compare the two implementations of a pass against each other).  Read whenever a plan is sized or created,
 // so that it must not change between came_b200_workspace_bytes and came_b200_plan_create of one plan.
 inline bool disable_fast() { const char* e = getenv("CAME_B200_DISABLE_FAST"); return e && e[0] == '1'; }

@@ -75,8 +75,7 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(flo
 template <typename T> __device__ __forceinline__ float round_to(float x) { return to_f32(from_f32<T>(x)); }
 
 // ------------------------------------------------------------------------------------------
-// N contiguous elements -> fp32 registers.  VEC: 16-byte loads (caller guarantees alignment and
-// that all N elements are in range).  !VEC: scalar loads, elements at col+e >= ncols read as 0.
+// N contiguous elements -> fp32 registers and back, by 16-byte accesses (the caller guarantees the alignment)
 // ------------------------------------------------------------------------------------------
 __device__ __forceinline__ void unpack_bf16x8(const uint4& r, float* v) {
     const uint32_t w[4] = {r.x, r.y, r.z, r.w};
@@ -96,94 +95,54 @@ __device__ __forceinline__ void unpack_f16x8(const uint4& r, float* v) {
     }
 }
 
-template <int N, bool VEC>
-__device__ __forceinline__ void load_run(const float* p, int64_t off, int col, int ncols, float* v) {
-    if (VEC) {
+template <int N>
+__device__ __forceinline__ void load_run(const float* p, float* v) {
 #pragma unroll
-        for (int i = 0; i < N / 4; ++i) {
-            const float4 f = reinterpret_cast<const float4*>(p + off)[i];
-            v[4 * i] = f.x; v[4 * i + 1] = f.y; v[4 * i + 2] = f.z; v[4 * i + 3] = f.w;
-        }
-    } else {
-#pragma unroll
-        for (int e = 0; e < N; ++e) v[e] = (col + e < ncols) ? p[off + e] : 0.0f;
+    for (int i = 0; i < N / 4; ++i) {
+        const float4 f = reinterpret_cast<const float4*>(p)[i];
+        v[4 * i] = f.x; v[4 * i + 1] = f.y; v[4 * i + 2] = f.z; v[4 * i + 3] = f.w;
     }
 }
-template <int N, bool VEC>
-__device__ __forceinline__ void load_run(const __nv_bfloat16* p, int64_t off, int col, int ncols, float* v) {
-    if (VEC) {
+template <int N>
+__device__ __forceinline__ void load_run(const __nv_bfloat16* p, float* v) {
 #pragma unroll
-        for (int i = 0; i < N / 8; ++i) {
-            const uint4 r = reinterpret_cast<const uint4*>(p + off)[i];
-            unpack_bf16x8(r, v + 8 * i);
-        }
-    } else {
-#pragma unroll
-        for (int e = 0; e < N; ++e) v[e] = (col + e < ncols) ? __bfloat162float(p[off + e]) : 0.0f;
-    }
+    for (int i = 0; i < N / 8; ++i) unpack_bf16x8(reinterpret_cast<const uint4*>(p)[i], v + 8 * i);
 }
-template <int N, bool VEC>
-__device__ __forceinline__ void load_run(const __half* p, int64_t off, int col, int ncols, float* v) {
-    if (VEC) {
+template <int N>
+__device__ __forceinline__ void load_run(const __half* p, float* v) {
 #pragma unroll
-        for (int i = 0; i < N / 8; ++i) {
-            const uint4 r = reinterpret_cast<const uint4*>(p + off)[i];
-            unpack_f16x8(r, v + 8 * i);
-        }
-    } else {
-#pragma unroll
-        for (int e = 0; e < N; ++e) v[e] = (col + e < ncols) ? __half2float(p[off + e]) : 0.0f;
-    }
+    for (int i = 0; i < N / 8; ++i) unpack_f16x8(reinterpret_cast<const uint4*>(p)[i], v + 8 * i);
 }
 
-template <int N, bool VEC>
-__device__ __forceinline__ void store_run(float* p, int64_t off, int col, int ncols, const float* v) {
-    if (VEC) {
+template <int N>
+__device__ __forceinline__ void store_run(float* p, const float* v) {
 #pragma unroll
-        for (int i = 0; i < N / 4; ++i)
-            reinterpret_cast<float4*>(p + off)[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-    } else {
+    for (int i = 0; i < N / 4; ++i) reinterpret_cast<float4*>(p)[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+}
+template <int N>
+__device__ __forceinline__ void store_run(__nv_bfloat16* p, const float* v) {
 #pragma unroll
-        for (int e = 0; e < N; ++e)
-            if (col + e < ncols) p[off + e] = v[e];
+    for (int i = 0; i < N / 8; ++i) {
+        uint32_t w[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(v[8 * i + 2 * k], v[8 * i + 2 * k + 1]);
+            w[k] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        reinterpret_cast<uint4*>(p)[i] = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
-template <int N, bool VEC>
-__device__ __forceinline__ void store_run(__nv_bfloat16* p, int64_t off, int col, int ncols, const float* v) {
-    if (VEC) {
+template <int N>
+__device__ __forceinline__ void store_run(__half* p, const float* v) {
 #pragma unroll
-        for (int i = 0; i < N / 8; ++i) {
-            uint32_t w[4];
+    for (int i = 0; i < N / 8; ++i) {
+        uint32_t w[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const __nv_bfloat162 h = __floats2bfloat162_rn(v[8 * i + 2 * k], v[8 * i + 2 * k + 1]);
-                w[k] = *reinterpret_cast<const uint32_t*>(&h);
-            }
-            reinterpret_cast<uint4*>(p + off)[i] = make_uint4(w[0], w[1], w[2], w[3]);
+        for (int k = 0; k < 4; ++k) {
+            const __half2 h = __floats2half2_rn(v[8 * i + 2 * k], v[8 * i + 2 * k + 1]);
+            w[k] = *reinterpret_cast<const uint32_t*>(&h);
         }
-    } else {
-#pragma unroll
-        for (int e = 0; e < N; ++e)
-            if (col + e < ncols) p[off + e] = __float2bfloat16_rn(v[e]);
-    }
-}
-template <int N, bool VEC>
-__device__ __forceinline__ void store_run(__half* p, int64_t off, int col, int ncols, const float* v) {
-    if (VEC) {
-#pragma unroll
-        for (int i = 0; i < N / 8; ++i) {
-            uint32_t w[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const __half2 h = __floats2half2_rn(v[8 * i + 2 * k], v[8 * i + 2 * k + 1]);
-                w[k] = *reinterpret_cast<const uint32_t*>(&h);
-            }
-            reinterpret_cast<uint4*>(p + off)[i] = make_uint4(w[0], w[1], w[2], w[3]);
-        }
-    } else {
-#pragma unroll
-        for (int e = 0; e < N; ++e)
-            if (col + e < ncols) p[off + e] = __float2half_rn(v[e]);
+        reinterpret_cast<uint4*>(p)[i] = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
 
@@ -327,9 +286,10 @@ __device__ __forceinline__ float col_factor(float v, bool clamp) {
     return 1.0f / sqrtf(v);
 }
 
-// 1 / sqrt(x) by one Newton step y (3 - x y^2) / 2 from the hardware's approximation: within one unit in the last place, like
-// a rounded division of a rounded square root, in a fifth of the instructions.  Outside the range in which no term
-// under- or overflows: those two.
+// 1 / sqrt(x) by one Newton step y (3 - x y^2) / 2 from the hardware's approximation, in a fifth of the instructions of a
+// rounded division of a rounded square root.  Against 64 bits, every mantissa of two binades: at most 1.00 units in the last
+// place off, 0.33 in the mean square, 13 % of the values not the nearest (division of a root: 1.49, 0.43, 26 %).  Outside
+// the range in which no term under- or overflows: division and root.
 static __device__ __noinline__ float inv_sqrt_plain(float x) { return 1.0f / sqrtf(x); }      // (out of line: rare, and long)
 __device__ __forceinline__ float inv_sqrt(float x) {
     if (!(x > 1e-30f && x < 1e30f)) return inv_sqrt_plain(x);

@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(THREADS) k_sq_partials(StepArgs a, const Work*
             const int col = col0 + h * 256 + lane * 8;
             if (col < C) {
                 float v[8];
-                load_run<8, true>(g, (int64_t)row * C + col, col, C, v);
+                load_run<8>(g + (int64_t)row * C + col, v);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
                     v[e] *= gscale;
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(THREADS) k_sumsq(StepArgs a, const Work* __res
             const int col = col0 + hh * 256 + lane * 8;
             if (col < C) {
                 float v[8];
-                load_run<8, true>(g, (int64_t)row * C + col, col, C, v);
+                load_run<8>(g + (int64_t)row * C + col, v);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
                     const float u = ((v[e] * gscale) * r) * cf[hh * 8 + e];   // masked elements: v = 0, cf = 0

@@ -12,7 +12,7 @@
 // consecutive columns (lane & 7) of 4 rows (lane >> 3, +4, +8, +12): column sums stay in 8 registers across
 // the bands, row sums need a 3-step shuffle, a 16x16 tile is shared by 8 lanes.
 //
-// Results equal those of k_moment / k_apply in factored.cu up to the order of a few fp32 roundings.
+// Results equal those of the whole-step kernel (generic.cu) up to the order of a few fp32 roundings.
 #include "wide.cuh"
 
 namespace came {

@@ -6,7 +6,7 @@
 // is 8 rows (a row of 1024 fp32 values is 4 KB), a lane owns 8 consecutive columns (lane & 7) of 2 rows (lane >> 3,
 // +4), a warp 64 columns.  The new momentum goes from registers to global memory (32 bytes per lane and row).
 //
-// Results equal those of k_moment / k_apply in factored.cu up to the order of a few fp32 roundings.
+// Results equal those of the whole-step kernel (generic.cu) up to the order of a few fp32 roundings.
 // Reference: kCameFactoredExpAvgRes (came_kernels.cu:2307-2342), kCameFactoredParamUpdate (came_kernels.cu:2487-2511).
 #include "wide.cuh"
 

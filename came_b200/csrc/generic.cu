@@ -43,13 +43,13 @@ template <typename T> struct Buf {
     T* p;
     __device__ __forceinline__ Buf(const void* q, int) : p(reinterpret_cast<T*>(const_cast<void*>(q))) {}
     __device__ __forceinline__ float get(int64_t i) const { return to_f32(p[i]); }
-    __device__ __forceinline__ void get8(int64_t i, float* v) const { load_run<8, true>(p, i, 0, 8, v); }
+    __device__ __forceinline__ void get8(int64_t i, float* v) const { load_run<8>(p + i, v); }
     __device__ __forceinline__ float round(float x) const { return round_to<T>(x); }
     __device__ __forceinline__ void put(int64_t i, float x, int64_t delta = 0) const {
         *reinterpret_cast<T*>(reinterpret_cast<char*>(p + i) + delta) = from_f32<T>(x);
     }
     __device__ __forceinline__ void put8(int64_t i, const float* v, int64_t delta = 0) const {
-        store_run<8, true>(reinterpret_cast<T*>(reinterpret_cast<char*>(p) + delta), i, 0, 8, v);
+        store_run<8>(reinterpret_cast<T*>(reinterpret_cast<char*>(p + i) + delta), v);
     }
 };
 struct Any {};
@@ -201,14 +201,6 @@ template <typename T, int MODE> struct Stage {
     static constexpr int COUNT = 2 * G_WARPS * BYTES <= 72 * 1024 ? 2 : 1;
 };
 
-__device__ __forceinline__ void cp16(void* dst, const void* src, int bytes) {      // bytes < 16: the rest becomes zero
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp4(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 struct Item {
     int tensor, tile, R, C, tr, tc, brow, col0, k, nb;      // brow: first row of band k of nb
@@ -399,7 +391,7 @@ __device__ __forceinline__ void tile_col_sums(const Item& it, float* colpart, co
             acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], 8);
             acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], 16);
         }
-        if (lane < 8 && it.col0 + 8 * lane < it.C) store_run<8, true>(dst, 8 * lane, 0, 8, acc);
+        if (lane < 8 && it.col0 + 8 * lane < it.C) store_run<8>(dst + 8 * lane, acc);
     } else {
 #pragma unroll
         for (int e = 0; e < 2; ++e)
@@ -615,7 +607,9 @@ __device__ __forceinline__ void band_moment(const StepArgs& a, const CameHyper* 
         for (int i = 0; i < NR; ++i) {
             const int r = Lane<V>::row(lane, i);
             int8_t* dst = reinterpret_cast<int8_t*>(m_base) + at + (int64_t)r * it.C + Lane<V>::col(lane, 0);
-            uint32_t y[E];      // the low byte of m * (127 / A) + 1.5 * 2^23 is the code (see fast_tile8.cu)
+            // The low byte of m * (127 / A) + 1.5 * 2^23 is the code (see fast_tile8.cu).  Of 26 M random values 20 do not get
+            // the code nearest to the 64-bit quotient (rounded quotient times 127: 38).
+            uint32_t y[E];
 #pragma unroll
             for (int e = 0; e < E; e += 2) {
                 const u64 t = fma2(pk(m[i][e], m[i][e + 1]), pk(q127[0], q127[V == 8 ? 0 : 1]), splat(ROUND_MAGIC));
@@ -636,7 +630,7 @@ __device__ __forceinline__ void band_moment(const StepArgs& a, const CameHyper* 
             const int r = Lane<V>::row(lane, i);
             float* dst = reinterpret_cast<float*>(m_base) + at + (int64_t)r * it.C + Lane<V>::col(lane, 0);
             if constexpr (V == 8) {
-                if (r < live && in[0]) store_run<8, true>(dst, 0, 0, 8, m[i]);
+                if (r < live && in[0]) store_run<8>(dst, m[i]);
             } else {
                 if (r < live && in[0]) dst[0] = m[i][0];
                 if (r < live && in[1]) dst[32] = m[i][1];
@@ -847,8 +841,8 @@ __device__ __forceinline__ void phase_apply_flat(const StepArgs& a, const CameHy
             float r, rr, c[8], rc[8];
             locate(i0, row, col);
             row_factors(row, r, rr);
-            load_run<8, true>(s.vc, col, 0, 8, c);
-            load_run<8, true>(s.Rc, col, 0, 8, rc);
+            load_run<8>(s.vc + col, c);
+            load_run<8>(s.Rc + col, rc);
 #pragma unroll
             for (int e = 0; e < 8; e += 2) pair(e, splat(r), splat(rr), pk(c[e], c[e + 1]), pk(rc[e], rc[e + 1]));
         }

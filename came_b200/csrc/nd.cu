@@ -73,7 +73,7 @@ __device__ __forceinline__ void nd_load4(const void* base, int dtype, int64_t i,
     }
 }
 __device__ __forceinline__ void nd_store4(void* base, int dtype, int64_t i, const float* v) {
-    if (dtype == CAME_DT_F32) store_run<4, true>(reinterpret_cast<float*>(base), i, 0, 4, v);
+    if (dtype == CAME_DT_F32) store_run<4>(reinterpret_cast<float*>(base) + i, v);
     else {
         uint32_t w[2];
 #pragma unroll

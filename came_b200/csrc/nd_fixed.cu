@@ -29,12 +29,6 @@ constexpr int F3_MATS = 256;                 // matrices of a 3 x 3 chunk, one p
 constexpr int F3_ROWS = 3 * F3_MATS;         // entries of a vector of the chunk
 constexpr int F1_MATS = 8 * QBLOCK;          // elements of a 1 x 1 chunk, a block per warp
 
-__device__ __forceinline__ void cp16(void* dst, const void* src, int bytes) {      // bytes < 16: the rest becomes zero
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp4(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
 
 // `bytes` consecutive bytes global -> shared.  A base on a 16-byte boundary: asynchronous 16-byte copies, of the last one
 // only the array's bytes; any other: byte by byte.
@@ -224,15 +218,15 @@ __global__ void __launch_bounds__(THREADS, 3) k_nd33(StepArgs a, const Work* __r
     if (i >= n) return;
     Chunk3 next(a, work[i]);
     issue3<QUANT, STEP>(a, next, L, f3_smem, gsz, psz);
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    cp_commit();
     for (; i < n; i += stride, buf ^= 1) {
         const Chunk3 k = next;
         if (i + stride < n) {
             next = Chunk3(a, work[i + stride]);
             issue3<QUANT, STEP>(a, next, L, f3_smem + (buf ^ 1) * L.bytes, gsz, psz);
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        cp_commit();
+        cp_wait<1>();
         __syncthreads();
         char* const st = f3_smem + buf * L.bytes;
         if (QUANT) {
@@ -340,7 +334,7 @@ __global__ void __launch_bounds__(THREADS, 3) k_nd33(StepArgs a, const Work* __r
             __syncthreads();      // the stage is free again
         }
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    cp_wait<0>();
 }
 
 // ---- 1 x 1 ------------------------------------------------------------------------------------------------------
@@ -348,7 +342,7 @@ __global__ void __launch_bounds__(THREADS, 3) k_nd33(StepArgs a, const Work* __r
 __device__ __forceinline__ void load8(const void* base, int dt, int64_t i, int64_t n, float scale, float (&v)[8]) {
     with_type(dt, [&](auto tag) {
         const auto* p = reinterpret_cast<const decltype(tag)*>(base);
-        if (i + 8 <= n && (reinterpret_cast<uintptr_t>(base) & 15) == 0) load_run<8, true>(p, i, 0, 8, v);
+        if (i + 8 <= n && (reinterpret_cast<uintptr_t>(base) & 15) == 0) load_run<8>(p + i, v);
         else
 #pragma unroll
             for (int e = 0; e < 8; ++e) v[e] = i + e < n ? to_f32(p[i + e]) : 0.0f;
@@ -360,7 +354,7 @@ __device__ __forceinline__ void store8(void* base, int dt, int64_t i, int64_t n,
     with_type(dt, [&](auto tag) {
         using T = decltype(tag);
         T* p = reinterpret_cast<T*>(base);
-        if (i + 8 <= n && (reinterpret_cast<uintptr_t>(base) & 15) == 0) store_run<8, true>(p, i, 0, 8, v);
+        if (i + 8 <= n && (reinterpret_cast<uintptr_t>(base) & 15) == 0) store_run<8>(p + i, v);
         else
 #pragma unroll
             for (int e = 0; e < 8; ++e)

@@ -55,6 +55,16 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
                  : "memory");
 }
 
+// per-thread asynchronous copies global -> shared, and the groups they complete in
+__device__ __forceinline__ void cp16(void* dst, const void* src, int bytes) {      // bytes < 16: the rest becomes zero
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp4(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
 // L2 eviction-priority policies for streams (read once: evict first) and for data another pass reads back soon
 // (evict last), and the copy / store forms that carry them
 __device__ __forceinline__ uint64_t l2_policy_evict_first() {
