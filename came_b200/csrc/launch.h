@@ -75,13 +75,12 @@ constexpr int S_FIN_CHUNK = 2048;      // factor-vector entries one CTA of the c
 void fused_sq_geometry(int64_t cols, int elem_bytes, int* groups, int* ng, int* rb, int* slot_kb);
 bool fused_sq_eligible(int64_t cols, int elem_bytes);
 // whole-step kernel (generic.cu): its work lists and the word of its grid barrier (zero before the first launch)
-constexpr int FLAT_GROUP = 8;
 struct GenericLists {
     const Work* tiles;      // matrix tiles
     const Work* vecs;       // blocks of 256 entries of the row, then the column vector
     const Work* flats;      // flat layout: blocks of 256 elements
     const Work* ones;       // 1-D tensors: blocks of 256 elements
-    int n_tiles, n_vecs, n_flats, n_ones;      // (n_flats: blocks, FLAT_GROUP per entry)
+    int n_tiles, n_vecs, n_flats, n_ones;
     uint32_t* bar;
 };
 constexpr int GENERIC_MAX_HYP = 8;      // hyper-parameter records that travel as kernel arguments
